@@ -25,24 +25,6 @@ __device__ __forceinline__ double pick3(int ax, double x, double y, double z) {
   return ax == 0 ? x : (ax == 1 ? y : z);
 }
 
-// Rule for one root r of an N-point rule (phase A lanes each need one root).
-// (table staged in shared memory at s)
-template <int N>
-__device__ __forceinline__ void rys_rule_one(double T, int r, const double* s, double* t2, double* w) {
-  constexpr int NI = rys_nint(N);
-  if (T >= double(NI)) {
-    const int base = (N * (N - 1)) / 2;
-    *t2 = __ldg(kRysAsymRoot + base + r) / T;
-    *w = __ldg(kRysAsymWeight + base + r) / sqrt(T);
-    return;
-  }
-  const int k = int(T);
-  const double x2 = 2.0 * (2.0 * (T - double(k)) - 1.0);
-  const double* c = s + k * rys_tab_stride<N>();
-  *t2 = cheb_clenshaw_s(c + r * (RYS_TAB_DEG + 1), x2);
-  *w = cheb_clenshaw_s(c + (N + r) * (RYS_TAB_DEG + 1), x2);
-}
-
 // Shared-memory footprint (doubles) of one warp of the J/K team kernel
 template <int LA, int LB, int LC, int LD>
 struct TeamJK {
@@ -123,7 +105,7 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
   using C = Cls<LA, LB, LC, LD>;
   using TM = TeamJK<LA, LB, LC, LD>;
   constexpr int NR = C::NR, TSZ = TM::TSP, CPL = TM::CPL;  // table stride
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   double* rtab = smem;
   rys_stage_table<NR>(rtab);
   __syncthreads();
@@ -307,22 +289,6 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
 // The Rys coefficients are read through L1 (the 3*NR lanes of a warp read one
 // T interval), so no table is staged per block, and the warps per block are
 // chosen so that the per-warp tables fit.
-template <int N>
-__device__ __forceinline__ void rys_rule_one_g(double T, int r, double* t2, double* w) {
-  constexpr int NI = rys_nint(N);
-  if (T >= double(NI)) {
-    const int base = (N * (N - 1)) / 2;
-    *t2 = __ldg(kRysAsymRoot + base + r) / T;
-    *w = __ldg(kRysAsymWeight + base + r) / sqrt(T);
-    return;
-  }
-  const int k = int(T);
-  const double x2 = 2.0 * (2.0 * (T - double(k)) - 1.0);
-  const double* c = kRysCheb + kRysOffset[N] + k * (2 * N * (RYS_TAB_DEG + 1));
-  *t2 = cheb_clenshaw(c + r * (RYS_TAB_DEG + 1), x2);
-  *w = cheb_clenshaw(c + (N + r) * (RYS_TAB_DEG + 1), x2);
-}
-
 // Warps per block for a per-warp shared footprint of `per_warp` doubles: the
 // choice of 4, 2, 1 with the most warps resident per SM (228 KB shared memory,
 // 1 KB reserved per block; at most 16 counted, beyond which registers limit
@@ -538,7 +504,7 @@ grad_team2_kernel(GradArgs args) {
               const double rs = rsqrt(pb.p + pl.p);
               const double T = pb.p * pl.p * (rs * rs) * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
               double t2, wr;
-              rys_rule_one_g<NR>(T, r, &t2, &wr);
+              rys_rule_one<NR, true>(T, r, nullptr, &t2, &wr);
               rts_all[2 * lane] = t2;
               rts_all[2 * lane + 1] = wr;
             }
@@ -553,7 +519,7 @@ grad_team2_kernel(GradArgs args) {
           if (lane < NR) {  // the Rys rule, one root per lane
             const double T = p * q * inv_s * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
             double t2, wr;
-            rys_rule_one_g<NR>(T, lane, &t2, &wr);
+            rys_rule_one<NR, true>(T, lane, nullptr, &t2, &wr);
             rts_all[2 * lane] = t2;
             rts_all[2 * lane + 1] = wr;
           }

@@ -166,6 +166,41 @@ __device__ __forceinline__ PrimPair load_pp(const PrimPair* __restrict__ p) {
   return r;
 }
 
+// The primitive quartets (i, j) of a contracted quartet with nb x nk primitive
+// pairs, in ket-major order (i fastest), starting at item `first` and stepping
+// by `stride`.  The division is done once per quartet: per step it would cost
+// as many instructions as the pair data of an (ss|ss) primitive quartet.
+struct PrimItems {
+  int i, j, nb, nk, di, dj, jl;
+  __device__ __forceinline__ PrimItems(int nb_, int nk_, int first, int stride) : nb(nb_), nk(nk_), jl(-1) {
+    if (stride == 1 && first == 0) {
+      i = j = 0;
+      di = nb > 1 ? 1 : 0;
+      dj = nb > 1 ? 0 : 1;
+    } else {
+      const int n1 = nb > 0 ? nb : 1;
+      j = first / n1;
+      i = first - j * n1;
+      dj = stride / n1;
+      di = stride - dj * n1;
+    }
+  }
+  __device__ __forceinline__ bool more() const { return j < nk && nb > 0; }
+  __device__ __forceinline__ bool new_ket() {
+    const bool n = j != jl;
+    jl = j;
+    return n;
+  }
+  __device__ __forceinline__ void next() {
+    i += di;
+    j += dj;
+    if (i >= nb) {
+      i -= nb;
+      ++j;
+    }
+  }
+};
+
 // Contracted (radially normalised) quartet (ab|cd) into acc[NCOMP].
 // Primitive quartets are visited as items it = i * np_ket + j, starting at
 // `first` with step `stride`, so that `stride` lanes can share one quartet.
@@ -186,16 +221,10 @@ __device__ __forceinline__ void quartet(const ShellPair& bp, const ShellPair& kp
   // ket-major order: the bra primitive is the same on every lane of the warp
   // (one broadcast line per load); each lane's own ket primitive, scattered
   // across lanes, is loaded once per j
-  const int nitems = bp.np * kp.np;
-  int jl = -1;
   PrimPair k;
-  for (int it = first; it < nitems; it += stride) {
-    const int j = it / bp.np, i = it - j * bp.np;
-    if (j != jl) {
-      k = load_pp(pp + kp.pstart + j);
-      jl = j;
-    }
-    const PrimPair b = load_pp(pp + bp.pstart + i);
+  for (PrimItems it(bp.np, kp.np, first, stride); it.more(); it.next()) {
+    if (it.new_ket()) k = load_pp(pp + kp.pstart + it.j);
+    const PrimPair b = load_pp(pp + bp.pstart + it.i);
     if (b.K * k.K < thr) continue;
     const double p = b.p, q = k.p, s = p + q;
     const double PQ[3] = {b.P[0] - k.P[0], b.P[1] - k.P[1], b.P[2] - k.P[2]};
@@ -275,7 +304,7 @@ template <typename R, int LA, int LB, int LC, int LD, int G, bool DO_K>
 __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr int NG = 32 / G;
-  extern __shared__ double rtab[];
+  extern __shared__ __align__(16) double rtab[];
   rys_stage_table<C::NR>(rtab);
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -511,7 +540,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
   // second block beside the staged Rys table: those kernels read the table
   // through L1 instead
   constexpr bool STAGE = grad_stages_rys<LA, LB, LC, LD, WSH>();
-  extern __shared__ double rtab[];
+  extern __shared__ __align__(16) double rtab[];
   if constexpr (STAGE) rys_stage_table<NR>(rtab);
   constexpr int TABD = STAGE ? rys_tab_doubles<NR>() : 0;
   // weights of this thread's quartet: Wsh[c * 128] (WSH), as R
@@ -590,17 +619,10 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
               else W[o] = wt;
             }
       const double CD[3] = {kp.A[0] - kp.B[0], kp.A[1] - kp.B[1], kp.A[2] - kp.B[2]};
-      const int nitems = bp.np * kp.np;
-      int jl = -1;
       PrimPair k;
-      for (int it = sub; it < nitems; it += G) {
-        // ket-major order (see quartet)
-        const int pj = it / bp.np, pi = it - pj * bp.np;
-        if (pj != jl) {
-          k = load_pp(args.pp + kp.pstart + pj);
-          jl = pj;
-        }
-        const PrimPair b = load_pp(args.pp + bp.pstart + pi);
+      for (PrimItems it(bp.np, kp.np, sub, G); it.more(); it.next()) {  // ket-major order (see quartet)
+        if (it.new_ket()) k = load_pp(args.pp + kp.pstart + it.j);
+        const PrimPair b = load_pp(args.pp + bp.pstart + it.i);
         if (b.K * k.K < args.prim_thr) continue;
         const double p = b.p, q = k.p, s = p + q;
         const double PQ[3] = {b.P[0] - k.P[0], b.P[1] - k.P[1], b.P[2] - k.P[2]};

@@ -8,8 +8,16 @@
 //     recurrence coefficients (Gautschi, "Orthogonal Polynomials", 2.1.7),
 //   * eigenvalues of the Jacobi matrix by Sturm-sequence bisection,
 //   * Christoffel numbers w_i = 1 / sum_j p_j(x_i)^2 (orthonormal p_j).
-// Roots and weights are then fitted piecewise on T in [0, Tasym(n)) with
-// Chebyshev series of fixed degree on unit-width intervals.  Beyond Tasym(n)
+// Roots and weights are then fitted piecewise on T in [0, Tasym(n)): Chebyshev
+// interpolation in binary128 on intervals of fixed width, converted to powers
+// of x = 2 (T - T0) / width - 1 in [-1, 1] before rounding to double, so that
+// the device evaluates them with one FMA per coefficient (Horner).  Their
+// coefficients fall by more than a factor of four per order, so the power form
+// loses nothing: worst relative error of Horner in double 2.0e-16 (n = 1) to
+// 2.9e-16 (n = 5), against 2.8e-16 to 3.6e-16 for the Chebyshev form by Clenshaw's
+// recurrence, which needs an add and an FMA per coefficient.  Orders 1 and 2 take half-width intervals and degree 9 (ten
+// coefficients; 12 and 28 KB), the others unit intervals and degree 11, whose
+// half-width tables (48 KB and more) would cost resident blocks.  Beyond Tasym(n)
 // the rule is the large-T limit: roots y_i / T and weights W_i / sqrt(T), with
 // (y_i, W_i) the Gauss rule for the weight y^{-1/2} e^{-y} / 2 on [0, inf).
 // Tasym(n) is the first integer T from which that limit agrees with the exact
@@ -26,8 +34,10 @@
 typedef __float128 q;
 
 static const int kMaxN = 7;
-static const int kDeg = 11;          // Chebyshev degree per interval
-static const double kWidth = 1.0;    // interval width in T
+// polynomial degree per interval (odd: an even number of coefficients, read in
+// 16-byte pairs) and intervals per unit of T
+static int deg_of(int n) { return n <= 2 ? 9 : 11; }
+static int per_unit(int n) { return n <= 2 ? 2 : 1; }
 
 // F_k(T) = int_0^1 t^{2k} e^{-T t^2} dt, k = 0..m, by the series of F_m and
 // downward recurrence (all terms positive, no cancellation).
@@ -119,14 +129,25 @@ static void asym_base(int n, q* y, q* W) {
   gauss_from_moments(n, mu, y, W);
 }
 
-static double cheb_eval(const double* c, double xx) {
-  double b1 = 0, b2 = 0;
-  for (int j = kDeg; j >= 1; --j) {
-    double t = c[j] + 2 * xx * b1 - b2;
-    b2 = b1;
-    b1 = t;
+static double horner(const double* c, int deg, double x) {
+  double v = c[deg];
+  for (int j = deg - 1; j >= 0; --j) v = std::fma(v, x, c[j]);
+  return v;
+}
+
+// powers of x from Chebyshev coefficients c_0..c_deg
+static std::vector<q> to_powers(const std::vector<q>& c) {
+  const size_t n = c.size();
+  std::vector<q> out(n, 0), t0(n, 0), t1(n, 0), t2(n, 0);
+  t0[0] = 1;
+  t1[1] = 1;
+  for (size_t k = 0; k < n; ++k) {
+    for (size_t i = 0; i < n; ++i) out[i] += c[k] * t0[i];
+    for (size_t i = 0; i < n; ++i) t2[i] = (i ? 2 * t1[i - 1] : 0) - t0[i];
+    t0 = t1;
+    t1 = t2;
   }
-  return c[0] + xx * b1 - b2;
+  return out;
 }
 
 int main(int argc, char** argv) {
@@ -155,55 +176,60 @@ int main(int argc, char** argv) {
       if (!ok) { Ta = T0 + 1; break; }
     }
     tasym[n] = Ta;
-    const int nint = int(std::ceil(Ta / kWidth));
+    const int deg = deg_of(n), np = deg + 1, nint = Ta * per_unit(n);
+    const double width = 1.0 / per_unit(n);
     offset[n] = int(coef.size());
     for (int k = 0; k < nint; ++k) {
-      const double t0 = k * kWidth;
+      const double t0 = k * width;
       // Chebyshev interpolation at deg+1 Chebyshev points of the 1st kind
-      const int np = kDeg + 1;
       std::vector<q> vals(size_t(np) * 2 * n);
       for (int j = 0; j < np; ++j) {
         q th = M_PIq * (j + 0.5Q) / np;
         q xx = cosq(th);
-        q T = t0 + (xx + 1) * 0.5Q * kWidth;
+        q T = t0 + (xx + 1) * 0.5Q * width;
         exact_rule(n, T, x, w);
         for (int i = 0; i < n; ++i) {
           vals[size_t(j) * 2 * n + i] = x[i];
           vals[size_t(j) * 2 * n + n + i] = w[i];
         }
       }
-      for (int f = 0; f < 2 * n; ++f)
-        for (int m = 0; m <= kDeg; ++m) {
+      for (int f = 0; f < 2 * n; ++f) {
+        std::vector<q> c(np);
+        for (int m = 0; m <= deg; ++m) {
           q s = 0;
           for (int j = 0; j < np; ++j)
             s += vals[size_t(j) * 2 * n + f] * cosq(m * M_PIq * (j + 0.5Q) / np);
-          s *= (m == 0 ? 1.0Q : 2.0Q) / np;
-          coef.push_back((double)s);
+          c[m] = s * (m == 0 ? 1.0Q : 2.0Q) / np;
         }
+        for (q v : to_powers(c)) coef.push_back((double)v);
+      }
     }
     // accuracy report on a dense grid
     double worst = 0;
     for (int k = 0; k < nint; ++k)
       for (int s = 0; s < 23; ++s) {
-        const double T = k * kWidth + (s + 0.37) / 23.0 * kWidth;
+        const double T = k * width + (s + 0.37) / 23.0 * width;
         exact_rule(n, T, x, w);
-        const double* c = &coef[offset[n] + size_t(k) * 2 * n * (kDeg + 1)];
-        const double xx = 2 * (T - k * kWidth) / kWidth - 1;
+        const double* c = &coef[offset[n] + size_t(k) * 2 * n * np];
+        const double xx = 2 * (T - k * width) / width - 1;
         for (int f = 0; f < 2 * n; ++f) {
-          const double v = cheb_eval(c + f * (kDeg + 1), xx);
-          const double ex = (double)(f < n ? x[f] : w[f - n]);
-          worst = std::fmax(worst, std::fabs(v - ex) / std::fabs(ex));
+          const q ex = f < n ? x[f] : w[f - n];
+          worst = std::fmax(worst, (double)fabsq((horner(c + f * np, deg, xx) - ex) / ex));
         }
       }
-    fprintf(stderr, "n=%d Tasym=%d intervals=%d worst rel err %.3e\n", n, Ta, nint, worst);
+    fprintf(stderr, "n=%d Tasym=%d intervals=%d degree=%d worst rel err %.3e\n", n, Ta, nint, deg, worst);
   }
   offset[kMaxN + 1] = int(coef.size());
   FILE* f = fopen(argv[1], "w");
-  fprintf(f, "// Generated by gen_rys_tables.cpp (binary128 Rys rules, Chebyshev fits). Do not edit.\n");
-  fprintf(f, "#define RYS_TAB_MAXN %d\n#define RYS_TAB_DEG %d\n#define RYS_TAB_WIDTH %.1f\n", kMaxN, kDeg, kWidth);
-  fprintf(f, "#ifndef RYS_TAB_QUAL\n#define RYS_TAB_QUAL static const\n#endif\n");
-  fprintf(f, "#define RYS_TAB_NINT {0");
+  fprintf(f, "// Generated by gen_rys_tables.cpp (binary128 Rys rules, piecewise polynomials). Do not edit.\n");
+  fprintf(f, "#define RYS_TAB_MAXN %d\n", kMaxN);
+  fprintf(f, "#ifndef RYS_TAB_QUAL\n#define RYS_TAB_QUAL static const\n#endif\n#ifndef RYS_TAB_ALIGN\n#define RYS_TAB_ALIGN\n#endif\n");
+  fprintf(f, "#define RYS_TAB_TASYM {0");
   for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", tasym[n]);
+  fprintf(f, "}\n#define RYS_TAB_NCOEF {0");
+  for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", deg_of(n) + 1);
+  fprintf(f, "}\n#define RYS_TAB_PER_UNIT {0");
+  for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", per_unit(n));
   fprintf(f, "}\n");
   fprintf(f, "RYS_TAB_QUAL int kRysTasym[%d] = {0", kMaxN + 1);
   for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", tasym[n]);
@@ -214,8 +240,8 @@ int main(int argc, char** argv) {
   for (double v : asy_y) fprintf(f, "  %.17e,\n", v);
   fprintf(f, "};\nRYS_TAB_QUAL double kRysAsymWeight[%zu] = {\n", asy_w.size());
   for (double v : asy_w) fprintf(f, "  %.17e,\n", v);
-  fprintf(f, "};\n// [n][interval][root 0..n-1, weight 0..n-1][Chebyshev coefficient 0..DEG]\n");
-  fprintf(f, "RYS_TAB_QUAL double kRysCheb[%zu] = {\n", coef.size());
+  fprintf(f, "};\n// [n][interval][root 0..n-1, weight 0..n-1][power of x, 0..NCOEF-1]\n");
+  fprintf(f, "RYS_TAB_ALIGN RYS_TAB_QUAL double kRysPoly[%zu] = {\n", coef.size());
   for (size_t i = 0; i < coef.size(); ++i) fprintf(f, "%.17e,%s", coef[i], (i % 4 == 3) ? "\n" : " ");
   fprintf(f, "};\n");
   fclose(f);

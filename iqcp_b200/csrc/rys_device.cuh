@@ -5,8 +5,9 @@
 // computes them per call from moments with Schmidt orthogonalisation and a
 // companion-matrix QR (rys/mod.rs:468-790).  On the device a per-call
 // eigen-solve diverges across lanes, so the rule is read from tables instead:
-// degree-11 Chebyshev series on unit intervals of T up to Tasym(n), and the
-// large-T Hermite limit (roots y_i/T, weights W_i/sqrt(T)) beyond it.  The
+// polynomials on intervals of T up to Tasym(n) (degree 9 on half-unit intervals
+// for n <= 2, 11 on unit intervals above), and the large-T Hermite limit
+// (roots y_i/T, weights W_i/sqrt(T)) beyond it.  The
 // tables (rys_tables.inc, made by gen_rys_tables.cpp in binary128) are exact
 // to ~3e-16 relative, i.e. closer to the true rule than the reference's own
 // FP64 moment method.
@@ -18,56 +19,86 @@
 #include <cuda_runtime.h>
 
 #define RYS_TAB_QUAL __device__ const
+#define RYS_TAB_ALIGN __align__(16)
 #include "rys_tables.inc"
 #undef RYS_TAB_QUAL
+#undef RYS_TAB_ALIGN
 
 namespace iqcp {
 
-// unit intervals below Tasym(n)
-__host__ __device__ constexpr int rys_nint(int n) {
-  constexpr int t[RYS_TAB_MAXN + 1] = RYS_TAB_NINT;
+// Tasym(n), polynomial coefficients per function, intervals per unit of T
+__host__ __device__ constexpr int rys_tasym(int n) {
+  constexpr int t[RYS_TAB_MAXN + 1] = RYS_TAB_TASYM;
+  return t[n];
+}
+__host__ __device__ constexpr int rys_ncoef(int n) {
+  constexpr int t[RYS_TAB_MAXN + 1] = RYS_TAB_NCOEF;
+  return t[n];
+}
+__host__ __device__ constexpr int rys_per_unit(int n) {
+  constexpr int t[RYS_TAB_MAXN + 1] = RYS_TAB_PER_UNIT;
   return t[n];
 }
 // Shared-memory copy of the order-N table: [interval][root 0..N-1, weight
-// 0..N-1][coefficient], interval stride padded to an odd number of doubles so
-// that lanes reading different intervals fall on different bank pairs.
+// 0..N-1][coefficient].  Coefficients are read in 16-byte pairs; the interval
+// stride is padded to an odd number of pairs so that lanes reading different
+// intervals fall on different banks.
 template <int N>
-__host__ __device__ constexpr int rys_tab_stride() { return 2 * N * (RYS_TAB_DEG + 1) + 1; }
+__host__ __device__ constexpr int rys_tab_width() { return 2 * N * rys_ncoef(N); }
 template <int N>
-__host__ __device__ constexpr int rys_tab_doubles() { return rys_nint(N) * rys_tab_stride<N>(); }
+__host__ __device__ constexpr int rys_tab_stride() { return rys_tab_width<N>() + 2; }
+template <int N>
+__host__ __device__ constexpr int rys_nint() { return rys_tasym(N) * rys_per_unit(N); }
+template <int N>
+__host__ __device__ constexpr int rys_tab_doubles() { return rys_nint<N>() * rys_tab_stride<N>(); }
 
 // Copy the order-N table into shared memory (all threads of the block).  Each
 // lane reads the interval of its own T, so table reads are scattered: from
 // shared memory they cost a few bank wavefronts, from L1 one cache line per lane.
 template <int N>
 __device__ __forceinline__ void rys_stage_table(double* __restrict__ s) {
-  constexpr int W = 2 * N * (RYS_TAB_DEG + 1);
-  const double* g = kRysCheb + kRysOffset[N];
-  for (int i = threadIdx.x; i < rys_nint(N) * W; i += blockDim.x) {
+  constexpr int W = rys_tab_width<N>() / 2;
+  const double2* g = reinterpret_cast<const double2*>(kRysPoly + kRysOffset[N]);
+  double2* d = reinterpret_cast<double2*>(s);
+  for (int i = threadIdx.x; i < rys_nint<N>() * W; i += blockDim.x) {
     const int k = i / W;
-    s[k * rys_tab_stride<N>() + (i - k * W)] = __ldg(g + i);
+    d[k * (rys_tab_stride<N>() / 2) + (i - k * W)] = __ldg(g + i);
   }
 }
 
-__device__ __forceinline__ double cheb_clenshaw_s(const double* c, double x2) {
-  double b1 = 0.0, b2 = 0.0;
+// Polynomial of NC coefficients (16-byte aligned) at x in [-1, 1]; LDG: through
+// the read-only path instead of shared memory.
+template <int NC, bool LDG>
+__device__ __forceinline__ double rys_poly(const double* __restrict__ c, double x) {
+  const double2* p = reinterpret_cast<const double2*>(c);
+  double v = 0.0;
 #pragma unroll
-  for (int j = RYS_TAB_DEG; j >= 1; --j) {
-    const double t = fma(x2, b1, c[j] - b2);
-    b2 = b1;
-    b1 = t;
+  for (int j = NC / 2 - 1; j >= 0; --j) {
+    const double2 u = LDG ? __ldg(p + j) : p[j];
+    v = j == NC / 2 - 1 ? u.y : fma(v, x, u.y);
+    v = fma(v, x, u.x);
   }
-  return fma(0.5 * x2, b1, c[0] - b2);
+  return v;
 }
 
-// rys_rule with the order-N table staged in shared memory at `s`
+// Interval of T < Tasym(N) and the position x in [-1, 1] inside it.
 template <int N>
+__device__ __forceinline__ int rys_interval(double T, double* x) {
+  const double t = T * rys_per_unit(N);
+  const int k = int(t);
+  *x = 2.0 * (t - double(k)) - 1.0;
+  return k;
+}
+
+// The n-point rule at T.  s: the order-N table staged in shared memory, or
+// null to read it through L1.  The large-T limit takes 1/sqrt(T) and 1/T from
+// one reciprocal square root.
+template <int N, bool LDG = false>
 __device__ __forceinline__ void rys_rule_tab(double T, const double* s, double* __restrict__ r,
                                              double* __restrict__ w) {
-  constexpr int NI = rys_nint(N);
-  if (T >= double(NI)) {
-    const double it = 1.0 / T;
-    const double is = 1.0 / sqrt(T);
+  static_assert(N >= 1 && N <= RYS_TAB_MAXN, "unsupported Rys order");
+  if (T >= double(rys_tasym(N))) {
+    const double is = rsqrt(T), it = is * is;
     const int base = (N * (N - 1)) / 2;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -76,50 +107,38 @@ __device__ __forceinline__ void rys_rule_tab(double T, const double* s, double* 
     }
     return;
   }
-  const int k = int(T);
-  const double x2 = 2.0 * (2.0 * (T - double(k)) - 1.0);
-  const double* c = s + k * rys_tab_stride<N>();
+  constexpr int NC = rys_ncoef(N);
+  double x;
+  const int k = rys_interval<N>(T, &x);
+  const double* c = LDG ? kRysPoly + kRysOffset[N] + k * rys_tab_width<N>() : s + k * rys_tab_stride<N>();
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    r[i] = cheb_clenshaw_s(c + i * (RYS_TAB_DEG + 1), x2);
-    w[i] = cheb_clenshaw_s(c + (N + i) * (RYS_TAB_DEG + 1), x2);
+    r[i] = rys_poly<NC, LDG>(c + i * NC, x);
+    w[i] = rys_poly<NC, LDG>(c + (N + i) * NC, x);
   }
-}
-
-__device__ __forceinline__ double cheb_clenshaw(const double* __restrict__ c, double x2) {
-  // x2 = 2x; sum_j c_j T_j(x)
-  double b1 = 0.0, b2 = 0.0;
-#pragma unroll
-  for (int j = RYS_TAB_DEG; j >= 1; --j) {
-    const double t = fma(x2, b1, __ldg(c + j) - b2);
-    b2 = b1;
-    b1 = t;
-  }
-  return fma(0.5 * x2, b1, __ldg(c) - b2);
 }
 
 template <int N>
 __device__ __forceinline__ void rys_rule(double T, double* __restrict__ r, double* __restrict__ w) {
-  static_assert(N >= 1 && N <= RYS_TAB_MAXN, "unsupported Rys order");
-  if (T >= double(kRysTasym[N])) {
-    const double it = 1.0 / T;
-    const double is = 1.0 / sqrt(T);
+  rys_rule_tab<N, true>(T, nullptr, r, w);
+}
+
+// Root and weight r of the N-point rule alone (kernels whose lanes each take one root)
+template <int N, bool LDG = false>
+__device__ __forceinline__ void rys_rule_one(double T, int r, const double* s, double* t2, double* w) {
+  if (T >= double(rys_tasym(N))) {
+    const double is = rsqrt(T);
     const int base = (N * (N - 1)) / 2;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      r[i] = __ldg(kRysAsymRoot + base + i) * it;
-      w[i] = __ldg(kRysAsymWeight + base + i) * is;
-    }
+    *t2 = __ldg(kRysAsymRoot + base + r) * (is * is);
+    *w = __ldg(kRysAsymWeight + base + r) * is;
     return;
   }
-  const int k = int(T);  // unit-width intervals
-  const double x2 = 2.0 * (2.0 * (T - double(k)) - 1.0);
-  const double* c = kRysCheb + kRysOffset[N] + k * (2 * N * (RYS_TAB_DEG + 1));
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    r[i] = cheb_clenshaw(c + i * (RYS_TAB_DEG + 1), x2);
-    w[i] = cheb_clenshaw(c + (N + i) * (RYS_TAB_DEG + 1), x2);
-  }
+  constexpr int NC = rys_ncoef(N);
+  double x;
+  const int k = rys_interval<N>(T, &x);
+  const double* c = LDG ? kRysPoly + kRysOffset[N] + k * rys_tab_width<N>() : s + k * rys_tab_stride<N>();
+  *t2 = rys_poly<NC, LDG>(c + r * NC, x);
+  *w = rys_poly<NC, LDG>(c + (N + r) * NC, x);
 }
 
 // Runtime-order dispatch (tests / batch entry point)
