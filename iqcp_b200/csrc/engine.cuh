@@ -187,13 +187,18 @@ struct GradArgs {
   const int* mol_n;           // per molecule: nbf
 };
 
+// One launch covers the shell pairs of consecutive molecules (atoms atom0 ..
+// atom1 - 1 of the context).
 struct OneEArgs {
-  int n_shells, n_atoms, nbf;
-  const int* l;
-  const int* nprim;
-  const int* pstart;
-  const int* off;
-  const double* center;
+  const ShellPair* pairs;
+  const int* list;                   // the launch's pairs, sorted by class
+  int first[kNumPairClasses + 1];    // class c: list[first[c]] .. list[first[c + 1] - 1]
+  int n_mol, atom0, atom1;
+  const int* mol_atom0;              // per molecule: first atom (n_mol + 1)
+  const int* mol_n;                  // per molecule: nbf
+  const long long* mol_base;         // per molecule: offset of its block in the packed matrices
+  const int* nprim;                  // per shell
+  const int* pstart;                 // per shell: first primitive
   const double* exps;
   const double* coefs;
   const double* atom_xyz;
@@ -202,11 +207,10 @@ struct OneEArgs {
   double* T;  // may be null
   double* V;  // may be null
   // nuclear gradient of the one-electron energy (one_electron_grad_kernel)
-  const int* atom;     // per shell: atom index
-  const double* D;     // density, nbf x nbf
-  const double* W;     // energy-weighted density (factor 2 convention), nbf x nbf
-  double* grad;        // n_atoms x 3, added to
-  int gsmem;           // accumulate per block in shared memory (3 * n_atoms doubles)
+  const double* D;     // density, packed
+  const double* W;     // energy-weighted density (factor 2 convention), packed
+  double* grad;        // atoms of the context x 3, added to
+  int gsmem;           // accumulate per block in shared memory (3 doubles per atom of the launch)
 };
 
 // Host launchers (eri_aux.cu, onee.cu)

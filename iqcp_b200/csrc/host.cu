@@ -52,6 +52,7 @@ struct iqcp_ctx {
   long long* d_mol_base = nullptr;
   int* d_mol_n = nullptr;
   int* d_mol_bf0 = nullptr;
+  int* d_mol_atom0 = nullptr;
   Packing pack{};
   std::vector<int> shell_l, shell_off, shell_atom;
   // device tables
@@ -83,6 +84,12 @@ struct iqcp_ctx {
   int* d_bint = nullptr;          // l | nprim | pstart | off | z | atom (per shell, molecule-local)
   double* d_bdbl = nullptr;       // center | exps | coefs | atom_xyz
   int n_prims = 0;
+  // one-electron launches: runs of molecules with at most kOneEAtoms atoms
+  // together (or one larger molecule), their pairs sorted by class
+  static constexpr int kOneEAtoms = 2048;
+  struct OneEChunk { int list0, atom0, atom1, first[kNumPairClasses + 1]; };
+  std::vector<OneEChunk> onee;
+  int* d_cls_list = nullptr;
   // host copies
   std::vector<ShellPair> pairs;
   std::vector<int> list_offset;   // per class, into d_ket_list
@@ -655,6 +662,8 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   CK(cudaMemcpy(ctx->d_mol_base, ctx->mol_base.data(), sizeof(long long) * (nmol + 1), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_mol_n, ctx->mol_nbf.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_mol_bf0, ctx->mol_bf0.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&ctx->d_mol_atom0, sizeof(int) * (nmol + 1)));
+  CK(cudaMemcpy(ctx->d_mol_atom0, ctx->mol_atom0.data(), sizeof(int) * (nmol + 1), cudaMemcpyHostToDevice));
   ctx->pack = Packing{ctx->d_mol_base, ctx->d_mol_n, ctx->d_mol_bf0, nmol, ctx->packed};
 
   if (pps.empty()) pps.push_back(PrimPair());
@@ -664,24 +673,40 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   CK(cudaMemcpy(ctx->d_pairs, ctx->pairs.data(), sizeof(ShellPair) * npairs, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ctx->d_pp, pps.data(), sizeof(PrimPair) * pps.size(), cudaMemcpyHostToDevice));
 
-  // Schwarz bounds on the device, one launch per pair class
+  // class-sorted pair lists of the one-electron launches; the Schwarz bounds on
+  // the device take them too, one launch per class and run of molecules
   {
-    std::vector<std::vector<int>> by_cls(kNumPairClasses);
-    for (int i = 0; i < npairs; ++i) {
-      const ShellPair& p = ctx->pairs[i];
-      by_cls[pair_class(ctx->shell_l[p.sa], ctx->shell_l[p.sb])].push_back(i);
+    std::vector<int> list;
+    list.reserve(npairs);
+    int p0 = 0;
+    for (int m = 0; m < nmol;) {
+      iqcp_ctx::OneEChunk ch{};
+      ch.list0 = (int)list.size();
+      ch.atom0 = ctx->mol_atom0[m];
+      int m1 = m + 1;
+      while (m1 < nmol && ctx->mol_atom0[m1 + 1] - ch.atom0 <= iqcp_ctx::kOneEAtoms) ++m1;
+      ch.atom1 = ctx->mol_atom0[m1];
+      std::vector<int> by_cls[kNumPairClasses];
+      for (; p0 < npairs && ctx->pairs[p0].mol < m1; ++p0) {
+        const ShellPair& p = ctx->pairs[p0];
+        by_cls[pair_class(ctx->shell_l[p.sa], ctx->shell_l[p.sb])].push_back(p0);
+      }
+      for (int c = 0; c < kNumPairClasses; ++c) {
+        ch.first[c] = (int)list.size() - ch.list0;
+        list.insert(list.end(), by_cls[c].begin(), by_cls[c].end());
+      }
+      ch.first[kNumPairClasses] = (int)list.size() - ch.list0;
+      ctx->onee.push_back(ch);
+      m = m1;
     }
-    int* d_list = nullptr;
-    CK(cudaMalloc(&d_list, sizeof(int) * npairs));
-    int pos = 0;
-    for (int c = 0; c < kNumPairClasses; ++c) {
-      if (by_cls[c].empty()) continue;
-      CK(cudaMemcpy(d_list + pos, by_cls[c].data(), sizeof(int) * by_cls[c].size(), cudaMemcpyHostToDevice));
-      CK(launch_schwarz(c, ctx->d_pairs, ctx->d_pp, d_list + pos, (int)by_cls[c].size(), kthr, ctx->stream));
-      pos += (int)by_cls[c].size();
-    }
+    CK(cudaMalloc(&ctx->d_cls_list, sizeof(int) * npairs));
+    CK(cudaMemcpy(ctx->d_cls_list, list.data(), sizeof(int) * npairs, cudaMemcpyHostToDevice));
+    for (const auto& ch : ctx->onee)
+      for (int c = 0; c < kNumPairClasses; ++c)
+        if (ch.first[c + 1] > ch.first[c])
+          CK(launch_schwarz(c, ctx->d_pairs, ctx->d_pp, ctx->d_cls_list + ch.list0 + ch.first[c],
+                            ch.first[c + 1] - ch.first[c], kthr, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaFree(d_list));
     CK(cudaMemcpy(ctx->pairs.data(), ctx->d_pairs, sizeof(ShellPair) * npairs, cudaMemcpyDeviceToHost));
   }
   std::vector<int> ket_list;
@@ -768,6 +793,8 @@ void iqcp_destroy(iqcp_ctx* ctx) {
   cudaFree(ctx->d_mol_base);
   cudaFree(ctx->d_mol_n);
   cudaFree(ctx->d_mol_bf0);
+  cudaFree(ctx->d_mol_atom0);
+  cudaFree(ctx->d_cls_list);
   cudaFree(ctx->d_counters);
   cudaFree(ctx->d_fp32);
   cudaFree(ctx->d_multi);
@@ -1212,24 +1239,25 @@ int iqcp_eri_compressed(iqcp_ctx* ctx, double* out, long long out_len) {
   return IQCP_OK;
 }
 
-static OneEArgs one_e_args(const iqcp_ctx* ctx, int m) {
+static OneEArgs one_e_args(const iqcp_ctx* ctx, const iqcp_ctx::OneEChunk& ch) {
   const int ns = ctx->n_shells;
-  const int s0 = ctx->mol_shell0[m], a0 = ctx->mol_atom0[m];
   OneEArgs a;
   std::memset(&a, 0, sizeof(a));
-  a.n_shells = ctx->mol_shell0[m + 1] - s0;
-  a.n_atoms = ctx->mol_atom0[m + 1] - a0;
-  a.nbf = ctx->mol_nbf[m];
-  a.l = ctx->d_bint + s0;
-  a.nprim = ctx->d_bint + ns + s0;
-  a.pstart = ctx->d_bint + 2 * ns + s0;
-  a.off = ctx->d_bint + 3 * ns + s0;
-  a.z = ctx->d_bint + 4 * ns + a0;
-  a.atom = ctx->d_bint + 4 * ns + ctx->n_atoms + s0;
-  a.center = ctx->d_bdbl + 3 * s0;
+  a.pairs = ctx->d_pairs;
+  a.list = ctx->d_cls_list + ch.list0;
+  std::copy(ch.first, ch.first + kNumPairClasses + 1, a.first);
+  a.n_mol = ctx->n_mol;
+  a.atom0 = ch.atom0;
+  a.atom1 = ch.atom1;
+  a.mol_atom0 = ctx->d_mol_atom0;
+  a.mol_n = ctx->d_mol_n;
+  a.mol_base = ctx->d_mol_base;
+  a.nprim = ctx->d_bint + ns;
+  a.pstart = ctx->d_bint + 2 * ns;
+  a.z = ctx->d_bint + 4 * ns;
   a.exps = ctx->d_bdbl + 3 * ns;
   a.coefs = a.exps + ctx->n_prims;
-  a.atom_xyz = a.coefs + ctx->n_prims + 3 * a0;
+  a.atom_xyz = a.coefs + ctx->n_prims;
   return a;
 }
 
@@ -1238,13 +1266,11 @@ int iqcp_one_electron(iqcp_ctx* ctx, double* S, double* T, double* V) {
   int rc = ensure_device(ctx);
   if (rc) return rc;
   const size_t bytes = sizeof(double) * (size_t)ctx->packed;
-  // one launch per molecule block of the packed matrices
-  for (int m = 0; m < ctx->n_mol; ++m) {
-    const long long mb = ctx->mol_base[m];
-    OneEArgs a = one_e_args(ctx, m);
-    a.S = S ? ctx->d_io[0] + mb : nullptr;
-    a.T = T ? ctx->d_io[1] + mb : nullptr;
-    a.V = V ? ctx->d_io[2] + mb : nullptr;
+  for (const auto& ch : ctx->onee) {
+    OneEArgs a = one_e_args(ctx, ch);
+    a.S = S ? ctx->d_io[0] : nullptr;
+    a.T = T ? ctx->d_io[1] : nullptr;
+    a.V = V ? ctx->d_io[2] : nullptr;
     CK(launch_one_electron(a, ctx->stream));
   }
   if (S) CK(cudaMemcpyAsync(S, ctx->d_io[0], bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1258,13 +1284,12 @@ int iqcp_one_electron_grad_device(iqcp_ctx* ctx, const double* dD, const double*
   if (!ctx || !dD || !dW || !dgrad) return IQCP_ERR_ARG;
   int rc = ensure_device(ctx);
   if (rc) return rc;
-  for (int m = 0; m < ctx->n_mol; ++m) {
-    const long long mb = ctx->mol_base[m];
-    OneEArgs a = one_e_args(ctx, m);
-    a.D = dD + mb;
-    a.W = dW + mb;
-    a.grad = dgrad + 3 * ctx->mol_atom0[m];
-    a.gsmem = a.n_atoms <= 2048 ? 1 : 0;
+  for (const auto& ch : ctx->onee) {
+    OneEArgs a = one_e_args(ctx, ch);
+    a.D = dD;
+    a.W = dW;
+    a.grad = dgrad;
+    a.gsmem = ch.atom1 - ch.atom0 <= iqcp_ctx::kOneEAtoms ? 1 : 0;
     CK(launch_one_electron_grad(a, ctx->stream));
   }
   return IQCP_OK;

@@ -2,51 +2,34 @@
 // attraction V over the same normalised Cartesian primitives as the ERIs.
 // They stand in for overlap_matrix (integrals/overlap.rs:647), the kinetic
 // and nuclear builders behind hcore_matrix (integrals/hcore.rs:103,
-// nuclear.rs:68-305): H = T + V.  Evaluated with McMurchie-Davidson Hermite
-// expansions, one thread per (shell a, shell b) block, all component pairs.
-// one_electron_grad_kernel contracts their nuclear derivatives with D and W.
+// nuclear.rs:68-305): H = T + V.  one_electron_grad_kernel contracts their
+// nuclear derivatives with D and W.
+//
+// One warp per shell pair, all molecules of the context and all angular
+// classes in one launch.  The warp stages up to 32 primitive pairs in shared
+// memory (one per lane), then its lanes share the (primitive pair, atom) items
+// of the nuclear attraction; S and T take one primitive pair per lane.  The
+// 1D integrals come from the ERI engine's recurrences (axis_table): with
+// t^2 = 0 they are the Gaussian moments of S and T, and a point charge is the
+// q -> infinity limit of the ket (c00 = PA - t^2 PC, b10 = (1 - t^2) / 2p), whose
+// Rys rule has la + lb roots' worth of degree, at most three roots.  Tables and
+// sums stay in registers.  What bounds it is latency at small sizes and the FP64
+// pipe at large ones; both were far off with a thread per shell pair, Hermite
+// arrays in local memory and primitives and atoms in series: the RHF gradient of
+// a 30-atom cc-pVDZ molecule 77.6 -> 45.9 ms (this part 29 ms -> under 1 ms), a
+// batched SCF of six small molecules 120 -> 79 ms.
 #include <cuda_runtime.h>
 
-#include "engine.cuh"
-#include "rys_device.cuh"
+#include "eri_templates.cuh"
 
 namespace iqcp {
 
 namespace {
 
-constexpr int kE = 5;        // powers up to l + 2 (kinetic) with l <= 2
-constexpr int kT = 2 * kE;   // Hermite index range
-
-// E[i][j][t] for one direction, i <= ia_max < NI, j <= jb_max
-template <int NI>
-__device__ void hermite_e(double a, double b, double X, int imax, int jmax, double E[NI][kE][kT]) {
-  const double p = a + b, mu = a * b / p;
-  const double XPA = -b / p * X, XPB = a / p * X, o2p = 0.5 / p;
-  for (int i = 0; i <= imax; ++i)
-    for (int j = 0; j <= jmax; ++j)
-      for (int t = 0; t < kT; ++t) E[i][j][t] = 0.0;
-  E[0][0][0] = exp(-mu * X * X);
-  for (int i = 0; i <= imax; ++i)
-    for (int j = 0; j <= jmax; ++j) {
-      if (i == 0 && j == 0) continue;
-      for (int t = 0; t <= i + j; ++t) {
-        double v;
-        if (i > 0) {
-          v = XPA * E[i - 1][j][t];
-          if (t > 0) v += o2p * E[i - 1][j][t - 1];
-          if (t + 1 <= i + j - 1) v += double(t + 1) * E[i - 1][j][t + 1];
-        } else {
-          v = XPB * E[i][j - 1][t];
-          if (t > 0) v += o2p * E[i][j - 1][t - 1];
-          if (t + 1 <= i + j - 1) v += double(t + 1) * E[i][j - 1][t + 1];
-        }
-        E[i][j][t] = v;
-      }
-    }
-}
+constexpr double kPi = 3.14159265358979323846;
 
 __device__ __forceinline__ double rad_norm_dev(double a, int l) {
-  const double tap = 2.0 * a / 3.14159265358979323846;
+  const double tap = 2.0 * a / kPi;
   double v = sqrt(sqrt(tap * tap * tap));
   const double fa = 4.0 * a;
   if (l == 1) v *= sqrt(fa);
@@ -54,109 +37,193 @@ __device__ __forceinline__ double rad_norm_dev(double a, int l) {
   return v;
 }
 
-__device__ __forceinline__ double ang_dev(int l, int c) {
-  return (l == 2 && (c == 0 || c == 3 || c == 5)) ? 0.57735026918962576451 : 1.0;
+// One primitive pair; ea is the exponent on A
+struct Prim1 {
+  double p, inv_p, P[3], c, ea, eb;
+};
+
+// Shell pair seen from one side: A is the shell that is differentiated
+struct Side {
+  double A[3], B[3];
+  int sa, sb, oa, ob, atom_a, mol;
+};
+
+__device__ __forceinline__ Side side_of(const ShellPair& s, bool swap) {
+  Side r;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    r.A[d] = swap ? s.B[d] : s.A[d];
+    r.B[d] = swap ? s.A[d] : s.B[d];
+  }
+  r.sa = swap ? s.sb : s.sa;
+  r.sb = swap ? s.sa : s.sb;
+  r.oa = swap ? s.ob : s.oa;
+  r.ob = swap ? s.oa : s.ob;
+  r.atom_a = swap ? s.atom_b : s.atom_a;
+  r.mol = s.mol;
+  return r;
+}
+
+// Primitive pair `k` (ip = k / npb, jp = k % npb) of a shell pair
+__device__ __forceinline__ Prim1 prim_pair(const OneEArgs& a, const Side& s, int la, int lb, int npb, int k) {
+  const int ip = k / npb, jp = k - ip * npb;
+  const int pa = a.pstart[s.sa] + ip, pb = a.pstart[s.sb] + jp;
+  Prim1 q;
+  q.ea = a.exps[pa];
+  q.eb = a.exps[pb];
+  q.p = q.ea + q.eb;
+  q.inv_p = 1.0 / q.p;
+  double r2 = 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    q.P[d] = (q.ea * s.A[d] + q.eb * s.B[d]) * q.inv_p;
+    r2 += (s.A[d] - s.B[d]) * (s.A[d] - s.B[d]);
+  }
+  q.c = a.coefs[pa] * rad_norm_dev(q.ea, la) * a.coefs[pb] * rad_norm_dev(q.eb, lb) *
+        exp(-q.ea * q.eb * q.inv_p * r2);
+  return q;
+}
+
+// The warp's staged primitive pairs, one array per field
+constexpr int kStage = 32;
+struct Stage {
+  double f[7][kStage];  // p, 1/p, P, c, ea
+};
+
+__device__ __forceinline__ void stage_store(Stage& st, int lane, const Prim1& q) {
+  st.f[0][lane] = q.p;
+  st.f[1][lane] = q.inv_p;
+  st.f[2][lane] = q.P[0];
+  st.f[3][lane] = q.P[1];
+  st.f[4][lane] = q.P[2];
+  st.f[5][lane] = q.c;
+  st.f[6][lane] = q.ea;
+}
+
+// kinetic 1D integral from overlaps I(i, j) with row length LBX: -1/2 d^2/dx^2 on j
+template <int LBX>
+__device__ __forceinline__ double kinetic_1d(const double* I, int i, int j, double eb) {
+  double k = -2.0 * eb * double(2 * j + 1) * I[i * LBX + j] + 4.0 * eb * eb * I[i * LBX + j + 2];
+  if (j >= 2) k += double(j * (j - 1)) * I[i * LBX + (j >= 2 ? j - 2 : 0)];
+  return -0.5 * k;
+}
+
+// ---------------------------------------------------------------------------
+template <int LA, int LB>
+__device__ __forceinline__ void pair_integrals(const OneEArgs& a, const ShellPair& sp, Stage& st, int lane) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NC = NA * NB, NR = (LA + LB) / 2 + 1;
+  const Side s = side_of(sp, false);
+  const int npb = a.nprim[s.sb], np = a.nprim[s.sa] * npb, n = a.mol_n[s.mol];
+  const long long mb = a.mol_base[s.mol];
+  const double AB[3] = {s.A[0] - s.B[0], s.A[1] - s.B[1], s.A[2] - s.B[2]};
+  auto put = [&](double* M, const double* v) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const double x = warp_sum(v[c]) * ang_factor(LA, c / NB) * ang_factor(LB, c % NB);
+      if (lane == (c & 31)) {
+        const long long i = s.oa + c / NB, j = s.ob + c % NB;
+        M[mb + i * n + j] = x;
+        if (s.sa != s.sb) M[mb + j * n + i] = x;
+      }
+    }
+  };
+  if (a.V) {
+    const int a0 = a.mol_atom0[s.mol], na = a.mol_atom0[s.mol + 1] - a0;
+    double v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = 0.0;
+    for (int k0 = 0; k0 < np; k0 += kStage) {
+      const int nk = np - k0 < kStage ? np - k0 : kStage;
+      __syncwarp();
+      if (lane < nk) stage_store(st, lane, prim_pair(a, s, LA, LB, npb, k0 + lane));
+      __syncwarp();
+      for (int it = lane; it < nk * na; it += 32) {
+        const int k = it / na, c = a0 + it - k * na;
+        const double p = st.f[0][k], inv_p = st.f[1][k];
+        double PA[3], PC[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          PA[d] = st.f[2 + d][k] - s.A[d];
+          PC[d] = st.f[2 + d][k] - a.atom_xyz[3 * c + d];
+        }
+        double rt[NR], wt[NR];
+        rys_rule<NR>(p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), rt, wt);
+        const double pre = -double(a.z[c]) * 2.0 * kPi * inv_p * st.f[5][k];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const double b10 = (0.5 - 0.5 * rt[r]) * inv_p;
+          double I[3][(LA + 1) * (LB + 1)];
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            axis_table<double, LA + LB, 0, LA, LB, 0, 0>(PA[d] - rt[r] * PC[d], 0.0, 0.0, b10, 0.0, AB[d], 0.0,
+                                                         d == 2 ? wt[r] * pre : 1.0, I[d]);
+#pragma unroll
+          for (int q = 0; q < NC; ++q) {
+            const int i = q / NB, j = q % NB;
+            v[q] = fma(I[0][cart_pow(LA, i, 0) * (LB + 1) + cart_pow(LB, j, 0)] *
+                           I[1][cart_pow(LA, i, 1) * (LB + 1) + cart_pow(LB, j, 1)],
+                       I[2][cart_pow(LA, i, 2) * (LB + 1) + cart_pow(LB, j, 2)], v[q]);
+          }
+        }
+      }
+    }
+    put(a.V, v);
+  }
+  if (a.S || a.T) {
+    double sv[NC], tv[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) sv[c] = tv[c] = 0.0;
+    for (int k = lane; k < np; k += 32) {
+      const Prim1 q = prim_pair(a, s, LA, LB, npb, k);
+      const double sp1 = sqrt(kPi * q.inv_p), cc = q.c * sp1 * sp1 * sp1;
+      double I[3][(LA + 1) * (LB + 3)];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        axis_table<double, LA + LB + 2, 0, LA, LB + 2, 0, 0>(q.P[d] - s.A[d], 0.0, 0.0, 0.5 * q.inv_p, 0.0, AB[d],
+                                                             0.0, 1.0, I[d]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        double s1[3], t1[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int i = cart_pow(LA, c / NB, d), j = cart_pow(LB, c % NB, d);
+          s1[d] = I[d][i * (LB + 3) + j];
+          t1[d] = kinetic_1d<LB + 3>(I[d], i, j, q.eb);
+        }
+        sv[c] = fma(cc * s1[0], s1[1] * s1[2], sv[c]);
+        tv[c] = fma(cc, t1[0] * s1[1] * s1[2] + s1[0] * t1[1] * s1[2] + s1[0] * s1[1] * t1[2], tv[c]);
+      }
+    }
+    if (a.S) put(a.S, sv);
+    if (a.T) put(a.T, tv);
+  }
+}
+
+constexpr int kWarps = 4;
+
+// Class of position i of the class-sorted pair list
+__device__ __forceinline__ int class_of(const OneEArgs& a, int i) {
+  int c = 0;
+  while (i >= a.first[c + 1]) ++c;
+  return c;
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) one_electron_kernel(OneEArgs a) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= a.n_shells * a.n_shells) return;
-  const int sa = idx / a.n_shells, sb = idx % a.n_shells;
-  const int la = a.l[sa], lb = a.l[sb];
-  const int na = ncart(la), nb = ncart(lb);
-  const double A[3] = {a.center[3 * sa], a.center[3 * sa + 1], a.center[3 * sa + 2]};
-  const double B[3] = {a.center[3 * sb], a.center[3 * sb + 1], a.center[3 * sb + 2]};
-  double s[36], t[36], v[36];
-  for (int i = 0; i < 36; ++i) s[i] = t[i] = v[i] = 0.0;
-  double E[3][3][kE][kT];
-  for (int ip = 0; ip < a.nprim[sa]; ++ip) {
-    const double ea = a.exps[a.pstart[sa] + ip];
-    const double ca = a.coefs[a.pstart[sa] + ip] * rad_norm_dev(ea, la);
-    for (int jp = 0; jp < a.nprim[sb]; ++jp) {
-      const double eb = a.exps[a.pstart[sb] + jp];
-      const double cb = a.coefs[a.pstart[sb] + jp] * rad_norm_dev(eb, lb);
-      const double p = ea + eb;
-      for (int d = 0; d < 3; ++d) hermite_e<3>(ea, eb, A[d] - B[d], la, lb + 2, E[d]);
-      const double sp = sqrt(3.14159265358979323846 / p);
-      const double cc = ca * cb;
-      double P[3];
-      for (int d = 0; d < 3; ++d) P[d] = (ea * A[d] + eb * B[d]) / p;
-      // overlap and kinetic
-      for (int ia = 0; ia < na; ++ia)
-        for (int ib = 0; ib < nb; ++ib) {
-          double s1[3], t1[3];
-          for (int d = 0; d < 3; ++d) {
-            const int i = cart_pow(la, ia, d), j = cart_pow(lb, ib, d);
-            s1[d] = E[d][i][j][0] * sp;
-            double k = -2.0 * eb * double(2 * j + 1) * E[d][i][j][0] + 4.0 * eb * eb * E[d][i][j + 2][0];
-            if (j >= 2) k += double(j * (j - 1)) * E[d][i][j - 2][0];
-            t1[d] = -0.5 * k * sp;
-          }
-          s[ia * nb + ib] += cc * s1[0] * s1[1] * s1[2];
-          t[ia * nb + ib] += cc * (t1[0] * s1[1] * s1[2] + s1[0] * t1[1] * s1[2] + s1[0] * s1[1] * t1[2]);
-        }
-      if (!a.V) continue;
-      // nuclear attraction: R_tuv via Boys F_n(p |PC|^2), n <= la + lb <= 4
-      const int N = la + lb;
-      for (int c = 0; c < a.n_atoms; ++c) {
-        const double PC[3] = {P[0] - a.atom_xyz[3 * c], P[1] - a.atom_xyz[3 * c + 1],
-                              P[2] - a.atom_xyz[3 * c + 2]};
-        double F[8];
-        boys_all_dev(N, p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), F);
-        // R^n_{tuv}, t+u+v <= N - n, stored for n = 0 only at the end
-        double R[5][5][5][5];
-        double fac = 1.0;
-        for (int n = 0; n <= N; ++n) {
-          R[n][0][0][0] = fac * F[n];
-          fac *= -2.0 * p;
-        }
-        for (int n = N - 1; n >= 0; --n) {
-          const int lim = N - n;
-          for (int tt = 0; tt <= lim; ++tt)
-            for (int uu = 0; uu <= lim - tt; ++uu)
-              for (int vv = 0; vv <= lim - tt - uu; ++vv) {
-                if (tt + uu + vv == 0) continue;
-                double val;
-                if (tt > 0) {
-                  val = PC[0] * R[n + 1][tt - 1][uu][vv];
-                  if (tt > 1) val += double(tt - 1) * R[n + 1][tt - 2][uu][vv];
-                } else if (uu > 0) {
-                  val = PC[1] * R[n + 1][tt][uu - 1][vv];
-                  if (uu > 1) val += double(uu - 1) * R[n + 1][tt][uu - 2][vv];
-                } else {
-                  val = PC[2] * R[n + 1][tt][uu][vv - 1];
-                  if (vv > 1) val += double(vv - 1) * R[n + 1][tt][uu][vv - 2];
-                }
-                R[n][tt][uu][vv] = val;
-              }
-        }
-        const double pre = -double(a.z[c]) * 2.0 * 3.14159265358979323846 / p * cc;
-        for (int ia = 0; ia < na; ++ia)
-          for (int ib = 0; ib < nb; ++ib) {
-            const int ix = cart_pow(la, ia, 0), jx = cart_pow(lb, ib, 0);
-            const int iy = cart_pow(la, ia, 1), jy = cart_pow(lb, ib, 1);
-            const int iz = cart_pow(la, ia, 2), jz = cart_pow(lb, ib, 2);
-            double acc = 0.0;
-            for (int tt = 0; tt <= ix + jx; ++tt)
-              for (int uu = 0; uu <= iy + jy; ++uu)
-                for (int vv = 0; vv <= iz + jz; ++vv)
-                  acc += E[0][ix][jx][tt] * E[1][iy][jy][uu] * E[2][iz][jz][vv] * R[0][tt][uu][vv];
-            v[ia * nb + ib] += pre * acc;
-          }
-      }
+__global__ void __launch_bounds__(32 * kWarps) one_electron_kernel(OneEArgs a) {
+  __shared__ Stage stage[kWarps];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = blockIdx.x * kWarps + wib; i < a.first[kNumPairClasses]; i += gridDim.x * kWarps) {
+    const ShellPair sp = a.pairs[a.list[i]];
+    switch (class_of(a, i)) {
+      case 0: pair_integrals<0, 0>(a, sp, stage[wib], lane); break;
+      case 1: pair_integrals<1, 0>(a, sp, stage[wib], lane); break;
+      case 2: pair_integrals<1, 1>(a, sp, stage[wib], lane); break;
+      case 3: pair_integrals<2, 0>(a, sp, stage[wib], lane); break;
+      case 4: pair_integrals<2, 1>(a, sp, stage[wib], lane); break;
+      default: pair_integrals<2, 2>(a, sp, stage[wib], lane); break;
     }
   }
-  const int oa = a.off[sa], ob = a.off[sb];
-  for (int ia = 0; ia < na; ++ia)
-    for (int ib = 0; ib < nb; ++ib) {
-      const double g = ang_dev(la, ia) * ang_dev(lb, ib);
-      const long long o = (long long)(oa + ia) * a.nbf + ob + ib;
-      if (a.S) a.S[o] = g * s[ia * nb + ib];
-      if (a.T) a.T[o] = g * t[ia * nb + ib];
-      if (a.V) a.V[o] = g * v[ia * nb + ib];
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -165,197 +232,235 @@ __global__ void __launch_bounds__(128) one_electron_kernel(OneEArgs a) {
 // overlap_derivative_matrix / hcore_derivative_matrix, gradient.rs:188,355):
 //   g_A += 2 sum_{mu on A, nu} [D_mn d(T+V)_mn/dA - W_mn dS_mn/dA]   (bra derivative;
 //          the ket term is equal by symmetry of D and W)
-//   g_C += sum_mn D_mn dV^C_mn/dC                                      (operator term)
+//   g_C += sum_mn D_mn dV^C_mn/dC = -sum_mn (D_mn + D_nm) dV^C_mn/dA   (operator
+//          term: V^C depends on differences of A, B and C only)
 //   g_A -= sum_{B != A} Z_A Z_B (A - B) / |A - B|^3
 // The derivative of a Cartesian Gaussian w.r.t. its centre raises and lowers
 // the power: d/dA_x x^i e^{-a x^2} = 2a x^{i+1} e^{..} - i x^{i-1} e^{..}.
-// One thread per (shell a, shell b) block; per-block gradient in shared memory.
-__global__ void __launch_bounds__(128) one_electron_grad_kernel(OneEArgs a) {
-  extern __shared__ double gacc[];
-  if (a.gsmem) {
-    for (int i = threadIdx.x; i < 3 * a.n_atoms; i += blockDim.x) gacc[i] = 0.0;
-    __syncthreads();
+// One warp per ordered shell pair; in the nuclear part a group of lanes keeps
+// one atom, so that the operator term is one shared-memory atomic per lane and
+// pair.  Per-block gradient in shared memory.
+namespace {
+
+// weights of the warp's block in shared memory: 2 D_ab, D_ab + D_ba, 2 W_ab with angular factors
+struct GradWeights {
+  double d2[36], ds[36], w2[36];
+};
+
+template <int LA, int LB>
+__device__ __forceinline__ void pair_gradient(const OneEArgs& a, const Side& s, Stage& st, GradWeights& w, int lane,
+                                              double* gout) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NC = NA * NB, NR = (LA + LB + 1) / 2 + 1;
+  const int npb = a.nprim[s.sb], np = a.nprim[s.sa] * npb, n = a.mol_n[s.mol];
+  const long long mb = a.mol_base[s.mol];
+  const int a0 = a.mol_atom0[s.mol], na = a.mol_atom0[s.mol + 1] - a0;
+  const double AB[3] = {s.A[0] - s.B[0], s.A[1] - s.B[1], s.A[2] - s.B[2]};
+  __syncwarp();
+  for (int c = lane; c < NC; c += 32) {
+    const long long i = s.oa + c / NB, j = s.ob + c % NB;
+    const double g = ang_factor(LA, c / NB) * ang_factor(LB, c % NB);
+    const double dij = a.D[mb + i * n + j], dji = a.D[mb + j * n + i];
+    w.d2[c] = 2.0 * g * dij;
+    w.ds[c] = g * (dij + dji);
+    w.w2[c] = 2.0 * g * a.W[mb + i * n + j];
   }
-  double* gout = a.gsmem ? gacc : a.grad;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  // nuclear repulsion: threads 0 .. n_atoms-1 of block 0 (n_atoms <= 128 per
-  // thread pass; larger molecules loop)
-  if (blockIdx.x == 0) {
-    for (int i = threadIdx.x; i < a.n_atoms; i += blockDim.x) {
-      double g[3] = {0, 0, 0};
-      for (int j = 0; j < a.n_atoms; ++j) {
-        if (j == i) continue;
-        double r[3], r2 = 0.0;
+  double gA[3] = {0, 0, 0};
+  // lanes per atom
+  int lpa = 1;
+  while (2 * lpa * na <= 32) lpa *= 2;
+  for (int k0 = 0; k0 < np; k0 += kStage) {
+    const int nk = np - k0 < kStage ? np - k0 : kStage;
+    __syncwarp();
+    if (lane < nk) {
+      const Prim1 q = prim_pair(a, s, LA, LB, npb, k0 + lane);
+      stage_store(st, lane, q);
+      // S and T: this lane's primitive pair
+      const double sp1 = sqrt(kPi * q.inv_p), cc = q.c * sp1 * sp1 * sp1;
+      double I[3][(LA + 2) * (LB + 3)];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        axis_table<double, LA + LB + 3, 0, LA + 1, LB + 2, 0, 0>(q.P[d] - s.A[d], 0.0, 0.0, 0.5 * q.inv_p, 0.0,
+                                                                 AB[d], 0.0, 1.0, I[d]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const double dmn = cc * w.d2[c], wmn = cc * w.w2[c];
+        double s1[3], t1[3], ds[3], dt[3];
+#pragma unroll
         for (int d = 0; d < 3; ++d) {
-          r[d] = a.atom_xyz[3 * i + d] - a.atom_xyz[3 * j + d];
-          r2 += r[d] * r[d];
+          const int i = cart_pow(LA, c / NB, d), j = cart_pow(LB, c % NB, d);
+          s1[d] = I[d][i * (LB + 3) + j];
+          t1[d] = kinetic_1d<LB + 3>(I[d], i, j, q.eb);
+          ds[d] = 2.0 * q.ea * I[d][(i + 1) * (LB + 3) + j];
+          dt[d] = 2.0 * q.ea * kinetic_1d<LB + 3>(I[d], i + 1, j, q.eb);
+          if (i > 0) {
+            ds[d] -= double(i) * I[d][(i > 0 ? i - 1 : 0) * (LB + 3) + j];
+            dt[d] -= double(i) * kinetic_1d<LB + 3>(I[d], i > 0 ? i - 1 : 0, j, q.eb);
+          }
         }
-        const double rr = sqrt(r2);
-        const double f = double(a.z[i] * a.z[j]) / (rr * rr * rr);
-        for (int d = 0; d < 3; ++d) g[d] -= f * r[d];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int e1 = (d + 1) % 3, e2 = (d + 2) % 3;
+          const double dS = ds[d] * s1[e1] * s1[e2];
+          const double dT = dt[d] * s1[e1] * s1[e2] + ds[d] * (t1[e1] * s1[e2] + s1[e1] * t1[e2]);
+          gA[d] += dmn * dT - wmn * dS;
+        }
       }
-      for (int d = 0; d < 3; ++d) atomicAdd(gout + 3 * i + d, g[d]);
     }
-  }
-  if (idx < a.n_shells * a.n_shells) {
-    const int sa = idx / a.n_shells, sb = idx % a.n_shells;
-    const int la = a.l[sa], lb = a.l[sb];
-    const int na = ncart(la), nb = ncart(lb);
-    const int oa = a.off[sa], ob = a.off[sb];
-    const double A[3] = {a.center[3 * sa], a.center[3 * sa + 1], a.center[3 * sa + 2]};
-    const double B[3] = {a.center[3 * sb], a.center[3 * sb + 1], a.center[3 * sb + 2]};
-    // D and W of the block with the angular factors of both components
-    double dm[36], wm[36];
-    for (int ia = 0; ia < na; ++ia)
-      for (int ib = 0; ib < nb; ++ib) {
-        const double g = ang_dev(la, ia) * ang_dev(lb, ib);
-        const long long o = (long long)(oa + ia) * a.nbf + ob + ib;
-        dm[ia * nb + ib] = g * a.D[o];
-        wm[ia * nb + ib] = g * a.W[o];
-      }
-    double gA[3] = {0, 0, 0};
-    double E[3][4][kE][kT];  // bra powers up to la + 1
-    const int N = la + lb + 1;
-    for (int ip = 0; ip < a.nprim[sa]; ++ip) {
-      const double ea = a.exps[a.pstart[sa] + ip];
-      const double ca = a.coefs[a.pstart[sa] + ip] * rad_norm_dev(ea, la);
-      for (int jp = 0; jp < a.nprim[sb]; ++jp) {
-        const double eb = a.exps[a.pstart[sb] + jp];
-        const double cb = a.coefs[a.pstart[sb] + jp] * rad_norm_dev(eb, lb);
-        const double p = ea + eb;
-        for (int d = 0; d < 3; ++d) hermite_e<4>(ea, eb, A[d] - B[d], la + 1, lb + 2, E[d]);
-        const double sp = sqrt(3.14159265358979323846 / p);
-        const double cc = ca * cb;
-        // 1D overlap / kinetic factors s(i, j), t(i, j) per direction
-        auto s1 = [&](int d, int i, int j) { return E[d][i][j][0] * sp; };
-        auto t1 = [&](int d, int i, int j) {
-          double k = -2.0 * eb * double(2 * j + 1) * E[d][i][j][0] + 4.0 * eb * eb * E[d][i][j + 2][0];
-          if (j >= 2) k += double(j * (j - 1)) * E[d][i][j - 2][0];
-          return -0.5 * k * sp;
-        };
-        for (int ia = 0; ia < na; ++ia)
-          for (int ib = 0; ib < nb; ++ib) {
-            const double dmn = dm[ia * nb + ib], wmn = wm[ia * nb + ib];
-            int pi[3], pj[3];
-            for (int d = 0; d < 3; ++d) {
-              pi[d] = cart_pow(la, ia, d);
-              pj[d] = cart_pow(lb, ib, d);
-            }
-            double s[3], t[3], ds[3], dt[3];
-            for (int d = 0; d < 3; ++d) {
-              s[d] = s1(d, pi[d], pj[d]);
-              t[d] = t1(d, pi[d], pj[d]);
-              ds[d] = 2.0 * ea * s1(d, pi[d] + 1, pj[d]) - (pi[d] > 0 ? pi[d] * s1(d, pi[d] - 1, pj[d]) : 0.0);
-              dt[d] = 2.0 * ea * t1(d, pi[d] + 1, pj[d]) - (pi[d] > 0 ? pi[d] * t1(d, pi[d] - 1, pj[d]) : 0.0);
-            }
-            for (int d = 0; d < 3; ++d) {
-              const int e1 = (d + 1) % 3, e2 = (d + 2) % 3;
-              const double dS = ds[d] * s[e1] * s[e2];
-              const double dT = dt[d] * s[e1] * s[e2] + ds[d] * (t[e1] * s[e2] + s[e1] * t[e2]);
-              gA[d] += 2.0 * cc * (dmn * dT - wmn * dS);
-            }
-          }
-        double P[3];
-        for (int d = 0; d < 3; ++d) P[d] = (ea * A[d] + eb * B[d]) / p;
-        for (int c = 0; c < a.n_atoms; ++c) {
-          const double PC[3] = {P[0] - a.atom_xyz[3 * c], P[1] - a.atom_xyz[3 * c + 1],
-                                P[2] - a.atom_xyz[3 * c + 2]};
-          double F[8];
-          boys_all_dev(N, p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), F);
-          // R^0_{tuv}, t+u+v <= N <= 5, by the downward recurrence in n with
-          // two levels kept (Rn: level n + 1, R: level n)
-          double R[6][6][6], Rn[6][6][6];
-          double fac = 1.0;
-          for (int n = 0; n < N; ++n) fac *= -2.0 * p;
-          Rn[0][0][0] = fac * F[N];
-          for (int n = N - 1; n >= 0; --n) {
-            fac /= -2.0 * p;
-            const int lim = N - n;
-            for (int tt = 0; tt <= lim; ++tt)
-              for (int uu = 0; uu <= lim - tt; ++uu)
-                for (int vv = 0; vv <= lim - tt - uu; ++vv) {
-                  double val;
-                  if (tt + uu + vv == 0) {
-                    val = fac * F[n];
-                  } else if (tt > 0) {
-                    val = PC[0] * Rn[tt - 1][uu][vv];
-                    if (tt > 1) val += double(tt - 1) * Rn[tt - 2][uu][vv];
-                  } else if (uu > 0) {
-                    val = PC[1] * Rn[tt][uu - 1][vv];
-                    if (uu > 1) val += double(uu - 1) * Rn[tt][uu - 2][vv];
-                  } else {
-                    val = PC[2] * Rn[tt][uu][vv - 1];
-                    if (vv > 1) val += double(vv - 1) * Rn[tt][uu][vv - 2];
-                  }
-                  R[tt][uu][vv] = val;
-                }
-            for (int tt = 0; tt <= lim; ++tt)
-              for (int uu = 0; uu <= lim - tt; ++uu)
-                for (int vv = 0; vv <= lim - tt - uu; ++vv) Rn[tt][uu][vv] = R[tt][uu][vv];
-          }
-          const double zc = double(a.z[c]) * 2.0 * 3.14159265358979323846 / p * cc;
-          double gC[3] = {0, 0, 0};
-          for (int ia = 0; ia < na; ++ia)
-            for (int ib = 0; ib < nb; ++ib) {
-              const double dmn = dm[ia * nb + ib];
-              int pi[3], pj[3];
-              for (int d = 0; d < 3; ++d) {
-                pi[d] = cart_pow(la, ia, d);
-                pj[d] = cart_pow(lb, ib, d);
-              }
-              // Hermite sum with the bra power of direction dd shifted by sh,
-              // and one more R index in direction hf (operator term; -1: none)
-              auto hsum = [&](int dd, int sh, int hf) {
-                int q[3] = {pi[0], pi[1], pi[2]};
-                if (dd >= 0) q[dd] += sh;
-                double acc = 0.0;
-                for (int tt = 0; tt <= q[0] + pj[0]; ++tt)
-                  for (int uu = 0; uu <= q[1] + pj[1]; ++uu)
-                    for (int vv = 0; vv <= q[2] + pj[2]; ++vv)
-                      acc += E[0][q[0]][pj[0]][tt] * E[1][q[1]][pj[1]][uu] * E[2][q[2]][pj[2]][vv] *
-                             R[tt + (hf == 0)][uu + (hf == 1)][vv + (hf == 2)];
-                return acc;
-              };
-              for (int d = 0; d < 3; ++d) {
-                // basis-function derivative of V^c (bra): V = -Z 2pi/p sum E R
-                double dv = 2.0 * ea * hsum(d, 1, -1);
-                if (pi[d] > 0) dv -= double(pi[d]) * hsum(d, -1, -1);
-                gA[d] += 2.0 * dmn * (-zc) * dv;
-                // operator derivative: dV^c/dC_d = +Z 2pi/p sum E R_{+1 in d}
-                gC[d] += dmn * zc * hsum(-1, 0, d);
-              }
-            }
+    __syncwarp();
+    for (int c = lane / lpa; c < na; c += 32 / lpa) {
+      const double C[3] = {a.atom_xyz[3 * (a0 + c)], a.atom_xyz[3 * (a0 + c) + 1], a.atom_xyz[3 * (a0 + c) + 2]};
+      const double zc = -double(a.z[a0 + c]) * 2.0 * kPi;
+      double gC[3] = {0, 0, 0};
+      for (int k = lane % lpa; k < nk; k += lpa) {
+        const double p = st.f[0][k], inv_p = st.f[1][k], e2 = 2.0 * st.f[6][k];
+        double PA[3], PC[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          PA[d] = st.f[2 + d][k] - s.A[d];
+          PC[d] = st.f[2 + d][k] - C[d];
+        }
+        double rt[NR], wt[NR];
+        rys_rule<NR>(p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]), rt, wt);
+        const double pre = zc * inv_p * st.f[5][k];
+#pragma unroll 1
+        for (int r = 0; r < NR; ++r) {
+          // the rule's entries by selection: an indexed access would put them in local memory
+          const double t2 = r == 0 ? rt[0] : (r == 1 ? rt[NR > 1 ? 1 : 0] : rt[NR - 1]);
+          const double wr = r == 0 ? wt[0] : (r == 1 ? wt[NR > 1 ? 1 : 0] : wt[NR - 1]);
+          const double b10 = (0.5 - 0.5 * t2) * inv_p;
+          double I[3][(LA + 2) * (LB + 1)];
+#pragma unroll
           for (int d = 0; d < 3; ++d)
-            if (gC[d] != 0.0) atomicAdd(gout + 3 * c + d, gC[d]);
+            axis_table<double, LA + LB + 1, 0, LA + 1, LB, 0, 0>(PA[d] - t2 * PC[d], 0.0, 0.0, b10, 0.0, AB[d], 0.0,
+                                                                 d == 2 ? wr * pre : 1.0, I[d]);
+#pragma unroll
+          for (int q = 0; q < NC; ++q) {
+            double v[3], dv[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const int i = cart_pow(LA, q / NB, d), j = cart_pow(LB, q % NB, d);
+              v[d] = I[d][i * (LB + 1) + j];
+              dv[d] = e2 * I[d][(i + 1) * (LB + 1) + j];
+              if (i > 0) dv[d] -= double(i) * I[d][(i > 0 ? i - 1 : 0) * (LB + 1) + j];
+            }
+            const double x = dv[0] * (v[1] * v[2]), y = dv[1] * (v[0] * v[2]), z = dv[2] * (v[0] * v[1]);
+            const double d2 = w.d2[q], ds = w.ds[q];
+            gA[0] = fma(d2, x, gA[0]);
+            gA[1] = fma(d2, y, gA[1]);
+            gA[2] = fma(d2, z, gA[2]);
+            gC[0] = fma(ds, x, gC[0]);
+            gC[1] = fma(ds, y, gC[1]);
+            gC[2] = fma(ds, z, gC[2]);
+          }
         }
       }
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (gC[d] != 0.0) atomicAdd(gout + 3 * (a0 + c - a.atom0) + d, -gC[d]);
     }
-    const int at = a.atom[sa];
-    for (int d = 0; d < 3; ++d) atomicAdd(gout + 3 * at + d, gA[d]);
   }
-  if (a.gsmem) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 3 * a.n_atoms; i += blockDim.x)
-      if (gacc[i] != 0.0) atomicAdd(a.grad + i, gacc[i]);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double g = warp_sum(gA[d]);
+    if (lane == 0) atomicAdd(gout + 3 * (s.atom_a - a.atom0) + d, g);
   }
 }
 
+// Nuclear repulsion gradient of atom i (its molecule's atoms a0 .. a1)
+__device__ __forceinline__ void repulsion_gradient(const OneEArgs& a, int i, int a0, int a1, double* gout) {
+  double g[3] = {0, 0, 0};
+  for (int j = a0; j < a1; ++j) {
+    if (j == i) continue;
+    double r[3], r2 = 0.0;
+    for (int d = 0; d < 3; ++d) {
+      r[d] = a.atom_xyz[3 * i + d] - a.atom_xyz[3 * j + d];
+      r2 += r[d] * r[d];
+    }
+    const double rr = sqrt(r2);
+    const double f = double(a.z[i]) * double(a.z[j]) / (rr * rr * rr);
+    for (int d = 0; d < 3; ++d) g[d] -= f * r[d];
+  }
+  for (int d = 0; d < 3; ++d) atomicAdd(gout + 3 * (i - a.atom0) + d, g[d]);
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(32 * kWarps) one_electron_grad_kernel(OneEArgs a) {
+  __shared__ Stage stage[kWarps];
+  __shared__ GradWeights weights[kWarps];
+  extern __shared__ double gacc[];
+  const int nacc = a.gsmem ? 3 * (a.atom1 - a.atom0) : 0;
+  for (int i = threadIdx.x; i < nacc; i += blockDim.x) gacc[i] = 0.0;
+  __syncthreads();
+  double* gout = a.gsmem ? gacc : a.grad + 3 * a.atom0;  // row 0: atom a.atom0
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // nuclear repulsion: one thread per atom over the grid
+  for (int i = a.atom0 + blockIdx.x * blockDim.x + threadIdx.x; i < a.atom1; i += gridDim.x * blockDim.x) {
+    int lo = 0, hi = a.n_mol - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (a.mol_atom0[mid] <= i) lo = mid; else hi = mid - 1;
+    }
+    repulsion_gradient(a, i, a.mol_atom0[lo], a.mol_atom0[lo + 1], gout);
+  }
+  const int npairs = a.first[kNumPairClasses];
+  for (int u = blockIdx.x * kWarps + wib; u < 2 * npairs; u += gridDim.x * kWarps) {
+    const int i = u >> 1;
+    const bool swap = u & 1;
+    const ShellPair sp = a.pairs[a.list[i]];
+    if (swap && sp.sa == sp.sb) continue;
+    const Side s = side_of(sp, swap);
+    Stage& st = stage[wib];
+    GradWeights& w = weights[wib];
+    switch (2 * class_of(a, i) + (swap ? 1 : 0)) {
+      case 0: case 1: pair_gradient<0, 0>(a, s, st, w, lane, gout); break;
+      case 2: pair_gradient<1, 0>(a, s, st, w, lane, gout); break;
+      case 3: pair_gradient<0, 1>(a, s, st, w, lane, gout); break;
+      case 4: case 5: pair_gradient<1, 1>(a, s, st, w, lane, gout); break;
+      case 6: pair_gradient<2, 0>(a, s, st, w, lane, gout); break;
+      case 7: pair_gradient<0, 2>(a, s, st, w, lane, gout); break;
+      case 8: pair_gradient<2, 1>(a, s, st, w, lane, gout); break;
+      case 9: pair_gradient<1, 2>(a, s, st, w, lane, gout); break;
+      default: pair_gradient<2, 2>(a, s, st, w, lane, gout); break;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nacc; i += blockDim.x)
+    if (gacc[i] != 0.0) atomicAdd(a.grad + 3 * a.atom0 + i, gacc[i]);
+}
+
+// One resident wave of blocks, fewer for small molecules
+static cudaError_t one_e_blocks(const void* kernel, size_t smem, int units, int* blocks) {
+  int per_sm = 0, dev = 0, sms = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kWarps, smem);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int need = (units + kWarps - 1) / kWarps, cap = (per_sm > 0 ? per_sm : 1) * sms;
+  *blocks = need < cap ? (need > 0 ? need : 1) : cap;
+  return cudaSuccess;
+}
+
 cudaError_t launch_one_electron_grad(const OneEArgs& a, cudaStream_t st) {
-  const int n = a.n_shells * a.n_shells;
-  const int blocks = (n + 127) / 128 > 0 ? (n + 127) / 128 : 1;
-  const size_t smem = a.gsmem ? sizeof(double) * 3 * a.n_atoms : 0;
-  if (smem > 48 * 1024) {
+  const size_t smem = a.gsmem ? sizeof(double) * 3 * (a.atom1 - a.atom0) : 0;
+  // beside the static arrays: dynamic shared memory beyond the default limit has to be asked for
+  if (smem > 32 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(one_electron_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem);
     if (e != cudaSuccess) return e;
   }
-  one_electron_grad_kernel<<<blocks, 128, smem, st>>>(a);
+  int blocks = 0;
+  const cudaError_t e = one_e_blocks((const void*)one_electron_grad_kernel, smem, 2 * a.first[kNumPairClasses], &blocks);
+  if (e != cudaSuccess) return e;
+  one_electron_grad_kernel<<<blocks, 32 * kWarps, smem, st>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_one_electron(const OneEArgs& a, cudaStream_t st) {
-  const int n = a.n_shells * a.n_shells;
-  one_electron_kernel<<<(n + 127) / 128, 128, 0, st>>>(a);
+  int blocks = 0;
+  const cudaError_t e = one_e_blocks((const void*)one_electron_kernel, 0, a.first[kNumPairClasses], &blocks);
+  if (e != cudaSuccess) return e;
+  one_electron_kernel<<<blocks, 32 * kWarps, 0, st>>>(a);
   return cudaGetLastError();
 }
 
