@@ -9,10 +9,12 @@
 // classes in one launch.  The warp stages up to 32 primitive pairs in shared
 // memory (one per lane), then its lanes share the (primitive pair, atom) items
 // of the nuclear attraction; S and T take one primitive pair per lane.  The
-// 1D integrals come from the ERI engine's recurrences (axis_table): with
-// t^2 = 0 they are the Gaussian moments of S and T, and a point charge is the
-// q -> infinity limit of the ket (c00 = PA - t^2 PC, b10 = (1 - t^2) / 2p), whose
-// Rys rule has la + lb roots' worth of degree, at most three roots.  Tables and
+// 1D integrals follow one two-centre recurrence (pair_table): with (PA, PB, 1/2p)
+// they are the Gaussian moments of S and T, and a point charge is the q ->
+// infinity limit of a Rys ket, (PA - t^2 PC, PB - t^2 PC, (1 - t^2) / 2p), with at
+// most three roots.  The second index is not taken by horizontal transfer: for
+// a tight shell on B that forms moments of order 1/p as differences of AB^2,
+// which the kinetic energy then multiplies by 4 b^2.  Tables and
 // sums stay in registers.  What bounds it is latency at small sizes and the FP64
 // pipe at large ones; both were far off with a thread per shell pair, Hermite
 // arrays in local memory and primitives and atoms in series: the RHF gradient of
@@ -100,6 +102,29 @@ __device__ __forceinline__ void stage_store(Stage& st, int lane, const Prim1& q)
   st.f[6][lane] = q.ea;
 }
 
+// 1D integrals I(i, j), i <= IA, j <= IB, at I[i (IB+1) + j]:
+// I(i, j+1) = cb I(i, j) + b [i I(i-1, j) + j I(i, j-1)], likewise i + 1 with ca
+template <int IA, int IB>
+__device__ __forceinline__ void pair_table(double ca, double cb, double b, double g00, double* I) {
+  constexpr int W = IB + 1;
+  I[0] = g00;
+#pragma unroll
+  for (int j = 0; j < IB; ++j) {
+    double v = cb * I[j];
+    if (j > 0) v = fma(double(j) * b, I[j > 0 ? j - 1 : 0], v);
+    I[j + 1] = v;
+  }
+#pragma unroll
+  for (int i = 0; i < IA; ++i)
+#pragma unroll
+    for (int j = 0; j <= IB; ++j) {
+      double v = ca * I[i * W + j];
+      if (i > 0) v = fma(double(i) * b, I[(i > 0 ? i - 1 : 0) * W + j], v);
+      if (j > 0) v = fma(double(j) * b, I[i * W + (j > 0 ? j - 1 : 0)], v);
+      I[(i + 1) * W + j] = v;
+    }
+}
+
 // kinetic 1D integral from overlaps I(i, j) with row length LBX: -1/2 d^2/dx^2 on j
 template <int LBX>
 __device__ __forceinline__ double kinetic_1d(const double* I, int i, int j, double eb) {
@@ -115,7 +140,6 @@ __device__ __forceinline__ void pair_integrals(const OneEArgs& a, const ShellPai
   const Side s = side_of(sp, false);
   const int npb = a.nprim[s.sb], np = a.nprim[s.sa] * npb, n = a.mol_n[s.mol];
   const long long mb = a.mol_base[s.mol];
-  const double AB[3] = {s.A[0] - s.B[0], s.A[1] - s.B[1], s.A[2] - s.B[2]};
   auto put = [&](double* M, const double* v) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -140,10 +164,11 @@ __device__ __forceinline__ void pair_integrals(const OneEArgs& a, const ShellPai
       for (int it = lane; it < nk * na; it += 32) {
         const int k = it / na, c = a0 + it - k * na;
         const double p = st.f[0][k], inv_p = st.f[1][k];
-        double PA[3], PC[3];
+        double PA[3], PB[3], PC[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           PA[d] = st.f[2 + d][k] - s.A[d];
+          PB[d] = st.f[2 + d][k] - s.B[d];
           PC[d] = st.f[2 + d][k] - a.atom_xyz[3 * c + d];
         }
         double rt[NR], wt[NR];
@@ -155,8 +180,7 @@ __device__ __forceinline__ void pair_integrals(const OneEArgs& a, const ShellPai
           double I[3][(LA + 1) * (LB + 1)];
 #pragma unroll
           for (int d = 0; d < 3; ++d)
-            axis_table<double, LA + LB, 0, LA, LB, 0, 0>(PA[d] - rt[r] * PC[d], 0.0, 0.0, b10, 0.0, AB[d], 0.0,
-                                                         d == 2 ? wt[r] * pre : 1.0, I[d]);
+            pair_table<LA, LB>(PA[d] - rt[r] * PC[d], PB[d] - rt[r] * PC[d], b10, d == 2 ? wt[r] * pre : 1.0, I[d]);
 #pragma unroll
           for (int q = 0; q < NC; ++q) {
             const int i = q / NB, j = q % NB;
@@ -179,8 +203,7 @@ __device__ __forceinline__ void pair_integrals(const OneEArgs& a, const ShellPai
       double I[3][(LA + 1) * (LB + 3)];
 #pragma unroll
       for (int d = 0; d < 3; ++d)
-        axis_table<double, LA + LB + 2, 0, LA, LB + 2, 0, 0>(q.P[d] - s.A[d], 0.0, 0.0, 0.5 * q.inv_p, 0.0, AB[d],
-                                                             0.0, 1.0, I[d]);
+        pair_table<LA, LB + 2>(q.P[d] - s.A[d], q.P[d] - s.B[d], 0.5 * q.inv_p, 1.0, I[d]);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         double s1[3], t1[3];
@@ -254,7 +277,6 @@ __device__ __forceinline__ void pair_gradient(const OneEArgs& a, const Side& s, 
   const int npb = a.nprim[s.sb], np = a.nprim[s.sa] * npb, n = a.mol_n[s.mol];
   const long long mb = a.mol_base[s.mol];
   const int a0 = a.mol_atom0[s.mol], na = a.mol_atom0[s.mol + 1] - a0;
-  const double AB[3] = {s.A[0] - s.B[0], s.A[1] - s.B[1], s.A[2] - s.B[2]};
   __syncwarp();
   for (int c = lane; c < NC; c += 32) {
     const long long i = s.oa + c / NB, j = s.ob + c % NB;
@@ -279,8 +301,7 @@ __device__ __forceinline__ void pair_gradient(const OneEArgs& a, const Side& s, 
       double I[3][(LA + 2) * (LB + 3)];
 #pragma unroll
       for (int d = 0; d < 3; ++d)
-        axis_table<double, LA + LB + 3, 0, LA + 1, LB + 2, 0, 0>(q.P[d] - s.A[d], 0.0, 0.0, 0.5 * q.inv_p, 0.0,
-                                                                 AB[d], 0.0, 1.0, I[d]);
+        pair_table<LA + 1, LB + 2>(q.P[d] - s.A[d], q.P[d] - s.B[d], 0.5 * q.inv_p, 1.0, I[d]);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const double dmn = cc * w.d2[c], wmn = cc * w.w2[c];
@@ -313,10 +334,11 @@ __device__ __forceinline__ void pair_gradient(const OneEArgs& a, const Side& s, 
       double gC[3] = {0, 0, 0};
       for (int k = lane % lpa; k < nk; k += lpa) {
         const double p = st.f[0][k], inv_p = st.f[1][k], e2 = 2.0 * st.f[6][k];
-        double PA[3], PC[3];
+        double PA[3], PB[3], PC[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           PA[d] = st.f[2 + d][k] - s.A[d];
+          PB[d] = st.f[2 + d][k] - s.B[d];
           PC[d] = st.f[2 + d][k] - C[d];
         }
         double rt[NR], wt[NR];
@@ -331,8 +353,7 @@ __device__ __forceinline__ void pair_gradient(const OneEArgs& a, const Side& s, 
           double I[3][(LA + 2) * (LB + 1)];
 #pragma unroll
           for (int d = 0; d < 3; ++d)
-            axis_table<double, LA + LB + 1, 0, LA + 1, LB, 0, 0>(PA[d] - t2 * PC[d], 0.0, 0.0, b10, 0.0, AB[d], 0.0,
-                                                                 d == 2 ? wr * pre : 1.0, I[d]);
+            pair_table<LA + 1, LB>(PA[d] - t2 * PC[d], PB[d] - t2 * PC[d], b10, d == 2 ? wr * pre : 1.0, I[d]);
 #pragma unroll
           for (int q = 0; q < NC; ++q) {
             double v[3], dv[3];
