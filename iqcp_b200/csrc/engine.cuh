@@ -75,7 +75,7 @@ struct QuartetTask {
   int nket;       // 1..32
   int diag;       // 1 when bra and ket lists are the same class (position ket0+i == bra_pos => pair with itself)
   int bra_pos;    // position of the bra in its class list
-  int flags;      // reserved (0)
+  int lg;         // thread kernels: 2^lg lanes share each ket's primitive quartets (nket <= 32 >> lg)
 };
 
 // Dynamic task distribution of the persistent quartet kernels: lane 0 of a
@@ -139,7 +139,7 @@ struct JKArgs {
   double* J;         // unsymmetrised accumulators (nbf x nbf)
   double* K;         // may be null
   double prim_thr;
-  int mode;          // kernel variant: 0 thread per quartet, 1 warp-cooperative, 2/3: 8/32 lanes per quartet
+  int mode;          // kernel variant: 1 warp-cooperative, else a group of lanes per quartet
   Mixed mx;
   int* next_task;             // work counter (zeroed before the launch)
   int ket_split = 1;          // team kernels: warps per task, each taking a slice of its kets
@@ -177,7 +177,7 @@ struct GradArgs {
   double* grad;      // natoms x 3
   double prim_thr;
   double schwarz_thr;
-  int mode;          // kernel variant: 0 thread per quartet, 1 warp-cooperative, 2/3: 8/32 lanes per quartet
+  int mode;          // kernel variant: 0 group of lanes per quartet, 1 warp-cooperative, 2 / 3 see eri_launch.cuh
   int natoms;        // gradient rows; accumulated per block in shared memory when gsmem
   int gsmem;
   Mixed mx;

@@ -58,7 +58,8 @@ __global__ void __launch_bounds__(128) grad_group_kernel(GradArgs args) {
   using GG = GroupGrad<R, LA, LB, LC, LD, G>;
   constexpr int EA = LA + 1, EB = LB, EC = LC + 1, ED = LD;
   constexpr int ESZ = (EA + 1) * (EB + 1) * (EC + 1) * (ED + 1);
-  constexpr int NR = GG::NR, NG = GG::NG;
+  constexpr int NR = GG::NR, NG = GG::NG, LG = G == 32 ? 5 : 3;
+  static_assert((1 << LG) == G, "8 or 32 lanes per quartet");
   auto eidx = [](int a, int b, int c, int d) { return ((a * (EB + 1) + b) * (EC + 1) + c) * (ED + 1) + d; };
   extern __shared__ __align__(16) double smem[];
   double* rtab = smem;
@@ -178,8 +179,8 @@ __global__ void __launch_bounds__(128) grad_group_kernel(GradArgs args) {
     // ket atoms differ per group: segmented reduction, lane 0 of the group adds
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      const double c = group_sum<G>(gC[x]);
-      const double dsum = group_sum<G>(gAq[x] + gBq[x] + gC[x]);
+      const double c = group_sum(gC[x], LG);
+      const double dsum = group_sum(gAq[x] + gBq[x] + gC[x], LG);
       if (active && sub == 0) {
         atomicAdd(gout + 3 * kp.atom_a + x, c);
         atomicAdd(gout + 3 * kp.atom_b + x, -dsum);  // translational invariance

@@ -62,12 +62,9 @@ inline int team_ket_split(K kernel, size_t smem, int ntasks, int threads) {
              ST>>>(ARGS);                                                                                \
   } while (0)
 
-// mode: 0 one quartet per thread, 1 warp-cooperative (eri_team.cuh),
-// 2 / 3 eight / thirty-two lanes share one quartet's primitive quartets
-// (J/K: small classes only; gradient: see launch_grad_variant; requests a
-// class has no kernel for fall back to mode 0).  The FP32 share
-// of a mixed call (pass 2) has modes 0 (up to 324 components), 1, and 2 for
-// the small classes; other requests map onto those.
+// J/K variants: 1 warp-cooperative (eri_team.cuh), every other mode a group of
+// lanes per quartet, as wide as the task says (build_tasks).  Above 324
+// components the FP32 share of a mixed call (pass 2) has the team kernel only.
 template <typename R, int LA, int LB, int LC, int LD>
 cudaError_t launch_jk_variant(const JKArgs& a, cudaStream_t st) {
   using C = Cls<LA, LB, LC, LD>;
@@ -79,19 +76,9 @@ cudaError_t launch_jk_variant(const JKArgs& a, cudaStream_t st) {
     JKArgs b = a;
     if (a.K) IQCP_LAUNCH_TEAM((jk_team_kernel<R, LA, LB, LC, LD, true>), 128, bytes, b, st);
     else IQCP_LAUNCH_TEAM((jk_team_kernel<R, LA, LB, LC, LD, false>), 128, bytes, b, st);
-  } else if (C::NCOMP <= 27 && (a.mode == 2 || a.mode == 3)) {
-    if constexpr (C::NCOMP <= 27) {
-      if (a.mode == 2 || F32) {
-        if (a.K) IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 8, true>), tb, a, st);
-        else IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 8, false>), tb, a, st);
-      } else {
-        if (a.K) IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 32, true>), tb, a, st);
-        else IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 32, false>), tb, a, st);
-      }
-    }
   } else if constexpr (!F32 || C::NCOMP <= 324) {
-    if (a.K) IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 1, true>), tb, a, st);
-    else IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, 1, false>), tb, a, st);
+    if (a.K) IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, true>), tb, a, st);
+    else IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, false>), tb, a, st);
   }
   return cudaGetLastError();
 }
@@ -109,7 +96,8 @@ inline size_t max_smem_optin() {
   return (size_t)v;
 }
 
-// Gradient variants: mode 2 is one quartet per thread with the D x D weights
+// Gradient variants: mode 0 a group of lanes per quartet (build_tasks), mode 1
+// warp-cooperative, mode 2 as mode 0 with the D x D weights
 // in shared memory (classes of kWshMinComp..kWshMaxComp components; others map
 // to mode 0), mode 3 the grouped kernel of eri_group.cuh (up to
 // kGroupGradMaxComp components, 32 lanes per quartet; the FP32 share uses 8).
@@ -142,14 +130,14 @@ cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
   if (team) {
     IQCP_LAUNCH_TEAM((grad_team2_kernel<R, LA, LB, LC, LD>), 32 * TG::WPB, bytes, a, st);
   } else if (wsh) {
-    if constexpr (WSH_OK) IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, 1, true>), bytes, a, st);
+    if constexpr (WSH_OK) IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, true>), bytes, a, st);
   } else if (group) {
     if constexpr (C::NCOMP <= kGroupGradMaxComp) {
       if (F32) IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 8>), bytes, a, st);
       else IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 32>), bytes, a, st);
     }
   } else if constexpr (!F32 || C::NCOMP <= 324) {
-    IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, 1>), bytes, a, st);
+    IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD>), bytes, a, st);
   }
   return cudaGetLastError();
 }

@@ -289,21 +289,24 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Quartet kernel with G lanes per contracted quartet (G = 1, 8 or 32): the 32/G
-// groups of a warp take consecutive kets of the task; the G lanes of a group
-// split the quartet's primitive quartets and combine their partial blocks with
-// a segmented shuffle reduction; lane 0 of each group digests the block.
-template <int G>
-__device__ __forceinline__ double group_sum(double v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// Sum over the 2^lg consecutive lanes of a group, on every lane of it.
+__device__ __forceinline__ double group_sum(double v, int lg) {
+  for (int o = (1 << lg) >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-template <typename R, int LA, int LB, int LC, int LD, int G, bool DO_K>
+// Components up to which a quartet's primitive quartets can be shared by a
+// group of lanes (a task's `lg`); above, each lane takes a whole quartet
+// whatever the task says (the group's sum would cost more than it spreads).
+constexpr int kMaxGroupComp = 108;
+
+// J/K, one contracted quartet per group of 2^task.lg lanes: the groups of a warp
+// take consecutive kets of the task, the lanes of a group split the quartet's
+// primitive quartets and add their partial blocks by shuffles, and the first
+// lane of each group digests the block.
+template <typename R, int LA, int LB, int LC, int LD, bool DO_K>
 __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
   using C = Cls<LA, LB, LC, LD>;
-  constexpr int NG = 32 / G;
   extern __shared__ __align__(16) double rtab[];
   rys_stage_table<C::NR>(rtab);
   __syncthreads();
@@ -312,7 +315,8 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
   const QuartetTask task = args.tasks[warp];
   const ShellPair bp = args.pairs[task.bra];
   if (task_inactive(args.mol_active, bp.mol)) continue;
-  const int grp = lane / G, sub = lane - grp * G;
+  const int lg = C::NCOMP <= kMaxGroupComp ? task.lg : 0;
+  const int NG = 32 >> lg, grp = lane >> lg, sub = lane & ((1 << lg) - 1);
   // this task's molecule block (bra and ket pairs always share a molecule)
   const int n = args.mol_n[bp.mol];
   const long long mb = args.mol_base[bp.mol];
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
     if (active) {
       const int kpos = task.ket0 + (args.mx.pass ? nth_set_bit(sel, kk) : kk);
       kp = args.pairs[__ldg(args.ket_list + kpos)];
-      quartet<R, LA, LB, LC, LD>(bp, kp, args.pp, args.prim_thr, acc, sub, G, rtab);
+      quartet<R, LA, LB, LC, LD>(bp, kp, args.pp, args.prim_thr, acc, sub, 1 << lg, rtab);
       f = 1.0;
       if (bp.sa == bp.sb) f *= 0.5;
       if (kp.sa == kp.sb) f *= 0.5;
@@ -339,9 +343,11 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
 #pragma unroll
       for (int i = 0; i < C::NCOMP; ++i) acc[i] = 0.0;
     }
-    if (G > 1) {
+    if constexpr (C::NCOMP <= kMaxGroupComp) {
+      for (int o = (1 << lg) >> 1; o > 0; o >>= 1) {
 #pragma unroll
-      for (int i = 0; i < C::NCOMP; ++i) acc[i] = group_sum<G>(acc[i]);
+        for (int i = 0; i < C::NCOMP; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+      }
     }
     const bool digest = active && sub == 0;
     // every density of the call (nset > 1: response densities) is digested
@@ -510,7 +516,8 @@ __global__ void __launch_bounds__(128) store_kernel(StoreArgs args) {
 // WSH: the D x D weights of each lane's quartet live in shared memory (one
 // column of NCOMP per thread, read back one component at a time) instead of
 // NCOMP registers, which leaves the registers to the extended tables of the
-// mid-size classes (G = 1 only).
+// mid-size classes.  A group of 2^task.lg lanes shares a quartet's primitive
+// quartets as in jk_kernel; each lane then holds the quartet's weights.
 template <int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int grad_wsh_doubles() {
   return 128 * ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD);
@@ -523,7 +530,7 @@ __host__ __device__ constexpr bool grad_stages_rys() {
 // Resident blocks asked of the compiler: 4 for L <= 1 (for (ps|ss) the
 // 128-register cap spills 76 bytes per thread, and is still faster than 3
 // blocks without spill: 4.2 against 4.4 ms on the 40-atom step); 1 above.
-template <typename R, int LA, int LB, int LC, int LD, int G, bool WSH = false>
+template <typename R, int LA, int LB, int LC, int LD, bool WSH = false>
 __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_kernel(GradArgs args) {
   using C = Cls<LA, LB, LC, LD>;
   // tables extended by one on A and C; the B derivative takes I(a, b+1) from
@@ -533,9 +540,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
   constexpr int ESZ = (EA + 1) * (EB + 1) * (EC + 1) * (ED + 1);
   auto eidx = [](int a, int b, int c, int d) { return ((a * (EB + 1) + b) * (EC + 1) + c) * (ED + 1) + d; };
   constexpr int NR = grad_nroots(LA + LB + LC + LD);
-  constexpr int NG = 32 / G;
   constexpr bool F32 = sizeof(R) == 4;
-  static_assert(!WSH || G == 1, "shared weights are per thread");
   // large shared weight arrays (more than 60 components) leave no room for a
   // second block beside the staged Rys table: those kernels read the table
   // through L1 instead
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
   for (int warp = next_task(args.next_task, lane); warp < args.ntasks; warp = next_task(args.next_task, lane)) {
   const QuartetTask task = args.tasks[warp];
   const ShellPair bp = args.pairs[task.bra];
-  const int grp = lane / G, sub = lane - grp * G;
+  const int lg = task.lg, NG = 32 >> lg, grp = lane >> lg, sub = lane & ((1 << lg) - 1);
   // this task's molecule block (bra and ket pairs always share a molecule)
   const int n = args.mol_n[bp.mol];
   const long long mb = args.mol_base[bp.mol];
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
             }
       const double CD[3] = {kp.A[0] - kp.B[0], kp.A[1] - kp.B[1], kp.A[2] - kp.B[2]};
       PrimPair k;
-      for (PrimItems it(bp.np, kp.np, sub, G); it.more(); it.next()) {  // ket-major order (see quartet)
+      for (PrimItems it(bp.np, kp.np, sub, 1 << lg); it.more(); it.next()) {  // ket-major order (see quartet)
         if (it.new_ket()) k = load_pp(args.pp + kp.pstart + it.j);
         const PrimPair b = load_pp(args.pp + bp.pstart + it.i);
         if (b.K * k.K < args.prim_thr) continue;
@@ -701,8 +706,8 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
     // ket atoms differ per group: segmented reduction, lane 0 of the group adds
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      const double c = group_sum<G>(gC[x]);
-      const double dsum = group_sum<G>(gAq[x] + gBq[x] + gC[x]);
+      const double c = group_sum(gC[x], lg);
+      const double dsum = group_sum(gAq[x] + gBq[x] + gC[x], lg);
       if (active && sub == 0) {
         atomicAdd(gout + 3 * kp.atom_a + x, c);
         atomicAdd(gout + 3 * kp.atom_b + x, -dsum);  // translational invariance

@@ -176,13 +176,33 @@ int basis_id(const char* name) {
   return -1;
 }
 
+// Lanes per quartet (a power of two, returned as its logarithm) of a task whose
+// quartets have `prims` primitive quartets each, when one lane should serve
+// about `per_lane` of them.  A thread that walks a deeply contracted quartet
+// alone is what a small build waits for: 36 x 36 primitive quartets of an
+// (ss|ss) quartet in 6-31G* took 0.68 ms of the 0.90 ms H2O Fock build, and
+// 64 x 64 in cc-pVDZ 3.0 ms, whatever the other 4000 warps did.
+int lanes_log2(double prims, double per_lane) {
+  int lg = 0;
+  while (lg < 5 && prims > per_lane * (1 << lg)) ++lg;
+  return lg;
+}
+
+// Primitive quartets per lane below which splitting a quartet further costs more
+// (group sums, digestion by one lane in 2^lg) than its shorter chain saves.
+constexpr double kMinPrimsPerLane = 16;
+constexpr double kResidentLanes = 148 * 16 * 32;  // SMs x resident warps of the thread kernels x lanes
+
 // Build class lists and quartet tasks from Schwarz bounds held in ctx->pairs.
 // Per molecule, each class list is split into buckets of equal primitive-pair
 // count (so the 32 kets of a warp share one primitive-loop length), each
 // bucket sorted by Q descending so that the Schwarz test Q_bra * Q_ket >= thr
 // keeps a prefix of it.  Unique quartets of a class with itself keep ket
 // position <= bra position.  Tasks never mix molecules; the tasks of one class
-// pair over all molecules form one range (one launch).
+// pair over all molecules form one range (one launch).  A task fills a warp:
+// 32 kets, or fewer with a group of lanes each where the quartets are deeply
+// contracted (more primitive quartets than the range's even share of a
+// resident lane) or where a bucket's last kets would leave lanes idle.
 void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetTask>& tasks) {
   const double thr = ctx->opt.schwarz_threshold;
   const int NC = kNumPairClasses;
@@ -217,36 +237,51 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
     for (int Y = 0; Y <= X; ++Y) {
       TaskRange r{X, Y, (int)tasks.size(), 0, 0, {default_mode(X, Y, 0), default_mode(X, Y, 1)},
                   {default_mode(X, Y, 0), default_mode(X, Y, 1)}, {1, 1}};
-      for (int m = 0; m < ctx->n_mol; ++m) {
-        const size_t lx = (size_t)m * NC + X, ly = (size_t)m * NC + Y;
-        const auto& LX = lists[lx];
-        const auto& LY = lists[ly];
-        for (int b = 0; b < (int)LX.size(); ++b) {
-          const double qb = ctx->pairs[LX[b]].Q;
-          for (const auto& bk : buckets[ly]) {
-            if (X == Y && bk.first > b) break;
-            const int hi_pos = (X == Y) ? std::min(bk.second, b + 1) : bk.second;
-            int lo = bk.first, hi = hi_pos;   // prefix of the bucket with qb * qk >= thr
-            while (lo < hi) {
-              const int mid = (lo + hi) / 2;
-              if (qb * ctx->pairs[LY[mid]].Q < thr) hi = mid; else lo = mid + 1;
-            }
-            const int nk = lo - bk.first;
-            ctx->n_quartets += nk;
-            r.quartets += nk;
-            for (int k0 = 0; k0 < nk; k0 += 32) {
-              QuartetTask t;
-              t.bra = LX[b];
-              t.ket0 = seg[ly] + bk.first + k0;
-              t.nket = std::min(32, nk - k0);
-              t.diag = (X == Y) ? 1 : 0;
-              t.bra_pos = seg[lx] + b;
-              t.flags = 0;
-              tasks.push_back(t);
+      // kets of bucket bk of molecule m that pass Schwarz with bra b: a prefix
+      auto bucket_kets = [&](const std::vector<int>& LY, const std::pair<int, int>& bk, int b, double qb) {
+        int lo = bk.first, hi = (X == Y) ? std::min(bk.second, b + 1) : bk.second;
+        while (lo < hi) {
+          const int mid = (lo + hi) / 2;
+          if (qb * ctx->pairs[LY[mid]].Q < thr) hi = mid; else lo = mid + 1;
+        }
+        return lo - bk.first;
+      };
+      auto for_buckets = [&](auto&& f) {
+        for (int m = 0; m < ctx->n_mol; ++m) {
+          const size_t lx = (size_t)m * NC + X, ly = (size_t)m * NC + Y;
+          const auto& LX = lists[lx];
+          const auto& LY = lists[ly];
+          for (int b = 0; b < (int)LX.size(); ++b) {
+            const ShellPair& bp = ctx->pairs[LX[b]];
+            for (const auto& bk : buckets[ly]) {
+              if (X == Y && bk.first > b) break;
+              const int nk = bucket_kets(LY, bk, b, bp.Q);
+              if (nk > 0) f(lx, ly, b, LX[b], bk.first, nk, (double)bp.np * ctx->pairs[LY[bk.first]].np);
             }
           }
         }
-      }
+      };
+      double work = 0.0;  // primitive quartets of the range
+      for_buckets([&](size_t, size_t, int, int, int, int nk, double prims) { work += nk * prims; });
+      const double per_lane = std::max(kMinPrimsPerLane, work / kResidentLanes);
+      for_buckets([&](size_t lx, size_t ly, int b, int bra, int first, int nk, double prims) {
+        ctx->n_quartets += nk;
+        r.quartets += nk;
+        const int lg = lanes_log2(prims, per_lane);
+        for (int k0 = 0; k0 < nk;) {
+          QuartetTask t;
+          t.bra = bra;
+          t.ket0 = seg[ly] + first + k0;
+          t.nket = std::min(32 >> lg, nk - k0);
+          t.diag = (X == Y) ? 1 : 0;
+          t.bra_pos = seg[lx] + b;
+          t.lg = lg;
+          // the bucket's last kets: spread over the lanes left, two primitive quartets a lane at least
+          while (t.lg < 5 && (t.nket << (t.lg + 1)) <= 32 && prims >= double(4 << t.lg)) ++t.lg;
+          k0 += t.nket;
+          tasks.push_back(t);
+        }
+      });
       r.count = (int)tasks.size() - r.first;
       ctx->ranges.push_back(r);
     }
