@@ -3,6 +3,7 @@
 // (eri_team.cuh); the small ones keep one quartet per thread.
 #pragma once
 #include "eri_group.cuh"
+#include "eri_md.cuh"
 
 namespace iqcp {
 
@@ -104,14 +105,29 @@ inline size_t max_smem_optin() {
 constexpr int kWshMinComp = 18, kWshMaxComp = 108;
 constexpr int kGroupGradMaxComp = 108;
 
+template <int LA, int LB, int LC>
+cudaError_t launch_grad_md(const GradArgs& args, cudaStream_t st) {
+  using G = GradMD<LA, LB, LC>;
+  GradArgs a = args;
+  // the per-block gradient accumulator only when it fits beside the tables
+  if (a.gsmem && sizeof(double) * (G::FIXED + 3 * a.natoms) > max_smem_optin()) a.gsmem = 0;
+  const size_t bytes = sizeof(double) * (G::FIXED + (a.gsmem ? 3 * a.natoms : 0));
+  IQCP_LAUNCH_T((grad_md_kernel<LA, LB, LC>), G::THREADS, bytes, a, st);
+  return cudaGetLastError();
+}
+
 template <typename R, int LA, int LB, int LC, int LD>
 cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr bool F32 = sizeof(R) == 4;
   constexpr int NRG = grad_nroots(LA + LB + LC + LD);
-  constexpr bool WSH_OK = !F32 && C::NCOMP >= kWshMinComp && C::NCOMP <= kWshMaxComp;
+  constexpr bool WSH_OK = !F32 && LC + LD > 1 && C::NCOMP >= kWshMinComp && C::NCOMP <= kWshMaxComp;
   using TG = TeamGrad2<LA, LB, LC, LD>;
+  // FP64 classes with an ss or ps ket: modes 0 and 2 are the Hermite kernel
+  constexpr bool MD = !F32 && LC + LD <= 1;
   const bool team = args.mode == 1 || (F32 && C::NCOMP > 324);
+  if constexpr (MD)
+    if (!team && args.mode != 3) return launch_grad_md<LA, LB, LC>(args, st);
   const bool wsh = !team && args.mode == 2 && WSH_OK;
   const bool group = !team && !wsh && (args.mode == 3 || (F32 && args.mode == 2)) && C::NCOMP <= kGroupGradMaxComp;
   // the team variant reads the Rys coefficients through L1 (no staged table)
@@ -136,7 +152,7 @@ cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
       if (F32) IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 8>), bytes, a, st);
       else IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 32>), bytes, a, st);
     }
-  } else if constexpr (!F32 || C::NCOMP <= 324) {
+  } else if constexpr (!MD && (!F32 || C::NCOMP <= 324)) {
     IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD>), bytes, a, st);
   }
   return cudaGetLastError();

@@ -511,6 +511,34 @@ __global__ void __launch_bounds__(128) store_kernel(StoreArgs args) {
         }
 }
 
+// Weight of component comp (a, b, c, d) of quartet (bp, kp): sum over the
+// distinct permutations of 1/2 D_ij D_kl - xs D_ik D_jl on the angular-scaled
+// density, zero where the reference weight is below 1e-15 (gradient.rs:1585-1640).
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ double grad_weight(const double* __restrict__ D, int n, const ShellPair& bp,
+                                              const ShellPair& kp, int comp, bool ij_same, bool kl_same,
+                                              bool bk_same, double xs) {
+  using C = Cls<LA, LB, LC, LD>;
+  const int d = comp % C::ND, c = (comp / C::ND) % C::NC, b = (comp / (C::ND * C::NC)) % C::NB,
+            a = comp / (C::ND * C::NC * C::NB);
+  const int i = bp.oa + a, j = bp.ob + b, k = kp.oa + c, l = kp.ob + d;
+  const double dij = __ldg(D + i * n + j), dkl = __ldg(D + k * n + l);
+  const double dik = __ldg(D + i * n + k), djl = __ldg(D + j * n + l);
+  const double dil = __ldg(D + i * n + l), djk = __ldg(D + j * n + k);
+  double t = 0.5 * dij * dkl - xs * dik * djl;
+  if (!ij_same) t += 0.5 * dij * dkl - xs * djk * dil;
+  if (!kl_same) t += 0.5 * dij * dkl - xs * dil * djk;
+  if (!ij_same && !kl_same) t += 0.5 * dij * dkl - xs * djl * dik;
+  if (!bk_same) {
+    t += 0.5 * dkl * dij - xs * dik * djl;
+    if (!kl_same) t += 0.5 * dkl * dij - xs * dil * djk;
+    if (!ij_same) t += 0.5 * dkl * dij - xs * djk * dil;
+    if (!ij_same && !kl_same) t += 0.5 * dkl * dij - xs * djl * dik;
+  }
+  const double angp = ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LC, c) * ang_factor(LD, d);
+  return (fabs(t / angp) < 1e-15) ? 0.0 : t;
+}
+
 // ---------------------------------------------------------------------------
 // Two-electron gradient (eri_gradient_fused, scf/gradient.rs:1430-1640).
 // WSH: the D x D weights of each lane's quartet live in shared memory (one

@@ -23,6 +23,11 @@
 // Tasym(n) is the first integer T from which that limit agrees with the exact
 // rule to the target accuracy everywhere in the sampled range.
 //
+// The Boys functions F_m(T), m = 0..kMaxBoys, are tabulated the same way on
+// half-unit intervals of [0, kBoysT): the Hermite gradient kernels read one
+// order and recur downwards.  From kBoysT = 36 on erf(sqrt(T)) is 1 to rounding
+// and the upward recurrence from F_0 = sqrt(pi/T)/2 loses nothing.
+//
 // Build/run:  g++ -O2 -o /tmp/gen gen_rys_tables.cpp -lquadmath && /tmp/gen rys_tables.inc
 #include <quadmath.h>
 
@@ -38,6 +43,7 @@ static const int kMaxN = 7;
 // 16-byte pairs) and intervals per unit of T
 static int deg_of(int n) { return n <= 2 ? 9 : 11; }
 static int per_unit(int n) { return n <= 2 ? 2 : 1; }
+static const int kMaxBoys = 9, kBoysT = 36, kBoysDeg = 9, kBoysPerUnit = 2;
 
 // F_k(T) = int_0^1 t^{2k} e^{-T t^2} dt, k = 0..m, by the series of F_m and
 // downward recurrence (all terms positive, no cancellation).
@@ -243,6 +249,38 @@ int main(int argc, char** argv) {
   fprintf(f, "};\n// [n][interval][root 0..n-1, weight 0..n-1][power of x, 0..NCOEF-1]\n");
   fprintf(f, "RYS_TAB_ALIGN RYS_TAB_QUAL double kRysPoly[%zu] = {\n", coef.size());
   for (size_t i = 0; i < coef.size(); ++i) fprintf(f, "%.17e,%s", coef[i], (i % 4 == 3) ? "\n" : " ");
+  fprintf(f, "};\n");
+  // Boys functions: [m][interval][power of x]
+  std::vector<double> boys;
+  double worst = 0;
+  for (int m = 0; m <= kMaxBoys; ++m)
+    for (int k = 0; k < kBoysT * kBoysPerUnit; ++k) {
+      const int np = kBoysDeg + 1;
+      const double width = 1.0 / kBoysPerUnit;
+      q F[kMaxBoys + 1];
+      std::vector<q> v(np), c(np);
+      for (int j = 0; j < np; ++j) {
+        boys_q(m, k * width + (cosq(M_PIq * (j + 0.5Q) / np) + 1) * 0.5Q * width, F);
+        v[j] = F[m];
+      }
+      for (int i = 0; i < np; ++i) {
+        q t = 0;
+        for (int j = 0; j < np; ++j) t += v[j] * cosq(i * M_PIq * (j + 0.5Q) / np);
+        c[i] = t * (i == 0 ? 1.0Q : 2.0Q) / np;
+      }
+      for (q t : to_powers(c)) boys.push_back((double)t);
+      for (int i = 0; i < 11; ++i) {
+        const double T = (k + (i + 0.37) / 11.0) * width, xx = 2 * (T - k * width) / width - 1;
+        boys_q(m, T, F);
+        worst = std::fmax(worst, (double)fabsq((horner(&boys[boys.size() - np], kBoysDeg, xx) - F[m]) / F[m]));
+      }
+    }
+  fprintf(stderr, "Boys F_0..F_%d: worst rel err %.3e\n", kMaxBoys, worst);
+  fprintf(f, "#define BOYS_TAB_MAXM %d\n#define BOYS_TAB_T %d\n#define BOYS_TAB_NCOEF %d\n#define BOYS_TAB_PER_UNIT %d\n",
+          kMaxBoys, kBoysT, kBoysDeg + 1, kBoysPerUnit);
+  fprintf(f, "// [order m][interval][power of x, 0..NCOEF-1]\n");
+  fprintf(f, "RYS_TAB_ALIGN RYS_TAB_QUAL double kBoysPoly[%zu] = {\n", boys.size());
+  for (size_t i = 0; i < boys.size(); ++i) fprintf(f, "%.17e,%s", boys[i], (i % 4 == 3) ? "\n" : " ");
   fprintf(f, "};\n");
   fclose(f);
   return 0;
