@@ -282,10 +282,10 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
 //             (ia, ib, ic, id), the four values I, dI/dA, dI/dB, dI/dC
 //             (d/dA: 2a E(ia+1) - ia E(ia-1), likewise B, C), stored as two
 //             planes of pairs (I, dA) and (dB, dC);
-//   phase B   each lane accumulates its components c = lane + 32 m: per root
-//             two vector loads per axis and 15 flops for the nine A/B/C
-//             derivatives (instead of ~21 scattered loads when each lane
-//             forms the derivatives from E itself).
+//   phase B   a lane takes an item (root, a, b[, c]): it loads the item's rows
+//             once, sums the weighted products of the other two axes per entry
+//             over the item's components, and contracts the sums with the
+//             entries' derivatives.
 // The Rys coefficients are read through L1 (the 3*NR lanes of a warp read one
 // T interval), so no table is staged per block, and the warps per block are
 // chosen so that the per-warp tables fit.
@@ -633,20 +633,23 @@ grad_team2_kernel(GradArgs args) {
           }
           const int ab = rest % (C::NA * C::NB), r = rest / (C::NA * C::NB);
           const int a = ab / C::NB, b = ab - a * C::NB;
-          // this item's rows: QI (I, dA) and (dB, dC) pairs per axis, loaded once
+          // Adjoint form: the sums X^[j] = sum w Iy Iz over the components whose x
+          // entry is j (likewise y, z) take five operations per component, and one
+          // dot product per axis with the entries' derivatives then gives all nine;
+          // forming the nine products per component took fifteen.
           constexpr int QI = TG::BYC ? LD + 1 : TG::KQ;
-          V2 q0[3][QI], q1[3][QI];
+          V2 q0[3][QI];   // I, dI/dA
+          R adj[3][QI];
+          int pos[3];
 #pragma unroll
           for (int ax = 0; ax < 3; ++ax) {
-            const int t = r * 3 + ax;
             const int row = cart_pow(LA, a, ax) * (LB + 1) + cart_pow(LB, b, ax);
-            const int pos = row * TG::KQP + (TG::BYC ? cart_pow(LC, c0, ax) * (LD + 1) : 0);
-            const V2* p0 = reinterpret_cast<const V2*>(qt + TG::pair(t, 0, pos) * 2);
-            const V2* p1 = reinterpret_cast<const V2*>(qt + TG::pair(t, 1, pos) * 2);
+            pos[ax] = row * TG::KQP + (TG::BYC ? cart_pow(LC, c0, ax) * (LD + 1) : 0);
+            const V2* p0 = reinterpret_cast<const V2*>(qt + TG::pair(r * 3 + ax, 0, pos[ax]) * 2);
 #pragma unroll
             for (int j = 0; j < QI; ++j) {
-              q0[ax][j] = p0[j];  // I, dI/dA
-              q1[ax][j] = p1[j];  // dI/dB, dI/dC
+              q0[ax][j] = p0[j];
+              adj[ax][j] = R(0);
             }
           }
           const R* wrow = Wsh + ab * (C::NC * C::ND) + c0 * C::ND;
@@ -655,18 +658,25 @@ grad_team2_kernel(GradArgs args) {
 #pragma unroll
             for (int d = 0; d < C::ND; ++d) {
               const R w = wrow[cc * C::ND + d];
-              V2 v0[3], v1[3];
-#pragma unroll
-              for (int ax = 0; ax < 3; ++ax) {
-                const int j = (TG::BYC ? 0 : cart_pow(LC, cc, ax) * (LD + 1)) + cart_pow(LD, d, ax);
-                v0[ax] = q0[ax][j];
-                v1[ax] = q1[ax][j];
-              }
-              const R wyz = w * v0[1].x * v0[2].x, wxz = w * v0[0].x * v0[2].x, wxy = w * v0[0].x * v0[1].x;
-              gl[0] = fma(wyz, v0[0].y, gl[0]); gl[1] = fma(wxz, v0[1].y, gl[1]); gl[2] = fma(wxy, v0[2].y, gl[2]);
-              gl[3] = fma(wyz, v1[0].x, gl[3]); gl[4] = fma(wxz, v1[1].x, gl[4]); gl[5] = fma(wxy, v1[2].x, gl[5]);
-              gl[6] = fma(wyz, v1[0].y, gl[6]); gl[7] = fma(wxz, v1[1].y, gl[7]); gl[8] = fma(wxy, v1[2].y, gl[8]);
+              const int jx = (TG::BYC ? 0 : cart_pow(LC, cc, 0) * (LD + 1)) + cart_pow(LD, d, 0);
+              const int jy = (TG::BYC ? 0 : cart_pow(LC, cc, 1) * (LD + 1)) + cart_pow(LD, d, 1);
+              const int jz = (TG::BYC ? 0 : cart_pow(LC, cc, 2) * (LD + 1)) + cart_pow(LD, d, 2);
+              const R x = q0[0][jx].x, y = q0[1][jy].x, wz = w * q0[2][jz].x;
+              adj[0][jx] = fma(wz, y, adj[0][jx]);
+              adj[1][jy] = fma(wz, x, adj[1][jy]);
+              adj[2][jz] = fma(w * x, y, adj[2][jz]);
             }
+#pragma unroll
+          for (int ax = 0; ax < 3; ++ax) {
+            const V2* p1 = reinterpret_cast<const V2*>(qt + TG::pair(r * 3 + ax, 1, pos[ax]) * 2);
+#pragma unroll
+            for (int j = 0; j < QI; ++j) {
+              const V2 q1 = p1[j];  // dI/dB, dI/dC
+              gl[ax] = fma(adj[ax][j], q0[ax][j].y, gl[ax]);
+              gl[3 + ax] = fma(adj[ax][j], q1.x, gl[3 + ax]);
+              gl[6 + ax] = fma(adj[ax][j], q1.y, gl[6 + ax]);
+            }
+          }
         }
         }  // root passes
 #pragma unroll

@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
   // the horizontal recurrence, I(a+1, b) + AB I(a, b), and the D derivative
   // follows from translational invariance
   constexpr int EA = LA + 1, EB = LB, EC = LC + 1, ED = LD;
-  constexpr int ESZ = (EA + 1) * (EB + 1) * (EC + 1) * (ED + 1);
+  constexpr int ESZ = (EA + 1) * (EB + 1) * (EC + 1) * (ED + 1), RSZ = C::TSZ;
   auto eidx = [](int a, int b, int c, int d) { return ((a * (EB + 1) + b) * (EC + 1) + c) * (ED + 1) + d; };
   constexpr int NR = grad_nroots(LA + LB + LC + LD);
   constexpr bool F32 = sizeof(R) == 4;
@@ -680,12 +680,23 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
           const double b00 = 0.5 * t2 * inv_s, h = 0.5 - 0.5 * t2;
           const double b10 = fma(h, b.inv_p, b00), b01 = fma(h, k.inv_p, b00);
           const double f2 = t2 * q * inv_s, f3 = t2 * p * inv_s;
-          R E[3][ESZ];
+          // Adjoint form: with the unextended tables I, the sums adj[x][e] = sum of
+          // w Iy Iz over the components whose x entry is e (likewise y, z) take
+          // five operations per component; the extended table of one axis at a
+          // time then gives its entries' derivatives and the nine dot products.
+          // Fifteen operations per component and three extended tables at once
+          // (108 doubles for (pp|pp)) spilled.
+          R c00[3], c0p[3], I[3][RSZ], adj[3][RSZ];
+          const R g00z = R(wt[r] * pref);
 #pragma unroll
-          for (int ax = 0; ax < 3; ++ax)
-            axis_table<R, LA + LB + 1, LC + LD + 1, EA, EB, EC, ED>(
-                R(PA[ax] - f2 * PQ[ax]), R(QC[ax] + f3 * PQ[ax]), R(b00), R(b10), R(b01), R(AB[ax]), R(CD[ax]),
-                R(ax == 2 ? wt[r] * pref : 1.0), E[ax]);
+          for (int ax = 0; ax < 3; ++ax) {
+            c00[ax] = R(PA[ax] - f2 * PQ[ax]);
+            c0p[ax] = R(QC[ax] + f3 * PQ[ax]);
+            axis_table<R, LA + LB, LC + LD, LA, LB, LC, LD>(c00[ax], c0p[ax], R(b00), R(b10), R(b01), R(AB[ax]),
+                                                            R(CD[ax]), ax == 2 ? g00z : R(1), I[ax]);
+#pragma unroll
+            for (int e = 0; e < RSZ; ++e) adj[ax][e] = R(0);
+          }
 #pragma unroll
           for (int a = 0; a < C::NA; ++a)
 #pragma unroll
@@ -696,30 +707,47 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
                 for (int d = 0; d < C::ND; ++d) {
                   const int wo = ((a * C::NB + bb) * C::NC + c) * C::ND + d;
                   const R w = WSH ? Wv[wo * 128] : W[WSH ? 0 : wo];
-                  R reg[3], dA[3], dB[3], dC[3];
-#pragma unroll
-                  for (int ax = 0; ax < 3; ++ax) {
-                    const int ia = cart_pow(LA, a, ax), ib = cart_pow(LB, bb, ax), ic = cart_pow(LC, c, ax),
-                              id = cart_pow(LD, d, ax);
-                    reg[ax] = E[ax][eidx(ia, ib, ic, id)];
-                    dA[ax] = a2 * E[ax][eidx(ia + 1, ib, ic, id)] -
-                             (ia > 0 ? R(ia) * E[ax][eidx(ia > 0 ? ia - 1 : 0, ib, ic, id)] : R(0));
-                    dB[ax] = b2 * (E[ax][eidx(ia + 1, ib, ic, id)] + R(AB[ax]) * E[ax][eidx(ia, ib, ic, id)]) -
-                             (ib > 0 ? R(ib) * E[ax][eidx(ia, ib > 0 ? ib - 1 : 0, ic, id)] : R(0));
-                    dC[ax] = c2 * E[ax][eidx(ia, ib, ic + 1, id)] -
-                             (ic > 0 ? R(ic) * E[ax][eidx(ia, ib, ic > 0 ? ic - 1 : 0, id)] : R(0));
-                  }
-                  const R wyz = w * reg[1] * reg[2], wxz = w * reg[0] * reg[2], wxy = w * reg[0] * reg[1];
-                  if constexpr (F32) {
-                    pA[0] = fmaf(wyz, dA[0], pA[0]); pA[1] = fmaf(wxz, dA[1], pA[1]); pA[2] = fmaf(wxy, dA[2], pA[2]);
-                    pB[0] = fmaf(wyz, dB[0], pB[0]); pB[1] = fmaf(wxz, dB[1], pB[1]); pB[2] = fmaf(wxy, dB[2], pB[2]);
-                    pC[0] = fmaf(wyz, dC[0], pC[0]); pC[1] = fmaf(wxz, dC[1], pC[1]); pC[2] = fmaf(wxy, dC[2], pC[2]);
-                  } else {
-                    gAq[0] = fma(wyz, dA[0], gAq[0]); gAq[1] = fma(wxz, dA[1], gAq[1]); gAq[2] = fma(wxy, dA[2], gAq[2]);
-                    gBq[0] = fma(wyz, dB[0], gBq[0]); gBq[1] = fma(wxz, dB[1], gBq[1]); gBq[2] = fma(wxy, dB[2], gBq[2]);
-                    gC[0] = fma(wyz, dC[0], gC[0]); gC[1] = fma(wxz, dC[1], gC[1]); gC[2] = fma(wxy, dC[2], gC[2]);
-                  }
+                  const int ex = C::tidx(cart_pow(LA, a, 0), cart_pow(LB, bb, 0), cart_pow(LC, c, 0), cart_pow(LD, d, 0));
+                  const int ey = C::tidx(cart_pow(LA, a, 1), cart_pow(LB, bb, 1), cart_pow(LC, c, 1), cart_pow(LD, d, 1));
+                  const int ez = C::tidx(cart_pow(LA, a, 2), cart_pow(LB, bb, 2), cart_pow(LC, c, 2), cart_pow(LD, d, 2));
+                  const R wz = w * I[2][ez];
+                  adj[0][ex] = fma(wz, I[1][ey], adj[0][ex]);
+                  adj[1][ey] = fma(wz, I[0][ex], adj[1][ey]);
+                  adj[2][ez] = fma(w * I[0][ex], I[1][ey], adj[2][ez]);
                 }
+#pragma unroll
+          for (int ax = 0; ax < 3; ++ax) {
+            R E[ESZ];
+            axis_table<R, LA + LB + 1, LC + LD + 1, EA, EB, EC, ED>(c00[ax], c0p[ax], R(b00), R(b10), R(b01), R(AB[ax]),
+                                                                    R(CD[ax]), ax == 2 ? g00z : R(1), E);
+            R sA = R(0), sB = R(0), sC = R(0);
+#pragma unroll
+            for (int ia = 0; ia <= LA; ++ia)
+#pragma unroll
+              for (int ib = 0; ib <= LB; ++ib)
+#pragma unroll
+                for (int ic = 0; ic <= LC; ++ic)
+#pragma unroll
+                  for (int id = 0; id <= LD; ++id) {
+                    const R v = adj[ax][C::tidx(ia, ib, ic, id)], up = E[eidx(ia + 1, ib, ic, id)];
+                    R dA = a2 * up, dB = b2 * (up + R(AB[ax]) * E[eidx(ia, ib, ic, id)]), dC = c2 * E[eidx(ia, ib, ic + 1, id)];
+                    if (ia > 0) dA -= R(ia) * E[eidx(ia > 0 ? ia - 1 : 0, ib, ic, id)];
+                    if (ib > 0) dB -= R(ib) * E[eidx(ia, ib > 0 ? ib - 1 : 0, ic, id)];
+                    if (ic > 0) dC -= R(ic) * E[eidx(ia, ib, ic > 0 ? ic - 1 : 0, id)];
+                    sA = fma(v, dA, sA);
+                    sB = fma(v, dB, sB);
+                    sC = fma(v, dC, sC);
+                  }
+            if constexpr (F32) {
+              pA[ax] += sA;
+              pB[ax] += sB;
+              pC[ax] += sC;
+            } else {
+              gAq[ax] += sA;
+              gBq[ax] += sB;
+              gC[ax] += sC;
+            }
+          }
         }
         if constexpr (F32) {
 #pragma unroll
