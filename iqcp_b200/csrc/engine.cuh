@@ -9,12 +9,6 @@ namespace iqcp {
 
 constexpr int kNumModes = 4;  // quartet-kernel variants per class
 
-// Default variant before autotuning: warp-cooperative for component-rich
-// classes, one quartet per thread for the rest.
-__host__ __device__ constexpr int default_mode(int X, int Y, int kind) {
-  return ((X == 5 || (X == 4 && Y >= 2)) && !(kind == 1 && X == 4 && Y == 3)) ? 1 : 0;
-}
-
 // Angular-momentum classes of a shell pair with la >= lb:
 // 0 ss, 1 ps, 2 pp, 3 ds, 4 dp, 5 dd  (index la*(la+1)/2 + lb)
 constexpr int kNumPairClasses = 6;
@@ -31,6 +25,40 @@ __host__ __device__ constexpr int grad_nroots(int L) { return (L + 1) / 2 + 1; }
 __host__ __device__ constexpr int pair_class(int la, int lb) { return la * (la + 1) / 2 + lb; }
 __host__ __device__ constexpr int class_la(int c) { return c == 0 ? 0 : (c <= 2 ? 1 : 2); }
 __host__ __device__ constexpr int class_lb(int c) { return c - class_la(c) * (class_la(c) + 1) / 2; }
+
+// Largest block (components) of the FP64 thread kernels; above, only the
+// warp-cooperative ones exist.  Measured on 40 atoms in 6-31G*: at 108
+// components ((dp|ds), (dd|ps)) a lane group per quartet takes 0.67 and 0.41 ms
+// against a warp's 1.40 and 0.81 (J/K), 2.37 and 1.56 against 3.02 and 2.06
+// (gradient); at 162 ((dp|pp)) the block no longer fits the registers and the
+// warp wins, 1.33 against 1.60 ms (J/K) and 3.33 against 8.2 (gradient).
+constexpr int kMaxThreadComp = 108;
+constexpr int kMaxThreadComp32 = 324;      // the same for the FP32 share of a mixed call
+constexpr int kMaxGroupGradComp = 108;     // gradient over (primitive quartet, root) items (eri_group.cuh)
+
+__host__ __device__ constexpr int class_comps(int X, int Y) {
+  return ncart(class_la(X)) * ncart(class_lb(X)) * ncart(class_la(Y)) * ncart(class_lb(Y));
+}
+// The variant that a requested mode runs (kind 0 J/K, 1 gradient): 1 a warp per
+// quartet, 0 a lane group per quartet, 3 (gradient) lanes over (primitive
+// quartet, root) items.
+__host__ __device__ constexpr int kernel_variant(int kind, int X, int Y, int mode, bool f32) {
+  const int n = class_comps(X, Y);
+  if (mode == 1 || n > (f32 ? kMaxThreadComp32 : kMaxThreadComp)) return 1;
+  if (kind == 1 && n <= kMaxGroupGradComp && (mode == 3 || (f32 && mode == 2))) return 3;
+  return 0;
+}
+// Variant before autotuning.  With fewer quartets than one wave of thread-kernel
+// lanes (148 SMs x 8 warps at 255 registers) the largest blocks leave most of the
+// chip idle behind a few long threads, and a warp per quartet is faster: 12 atoms
+// in 6-31G*, gradient (pp|pp) 0.12 against 0.17 ms, (dp|ds) 0.14 / 0.23, (dd|ps) 0.11 /
+// 0.25, J/K (dd|ps) 0.05 / 0.07; below those sizes of block the thread kernels stay
+// ahead ((ds|pp) gradient 0.12 against 0.19 ms).
+__host__ __device__ constexpr int default_mode(int X, int Y, int kind, long long quartets) {
+  const int n = class_comps(X, Y);
+  if (n > kMaxThreadComp) return 1;
+  return n >= (kind == 1 ? 81 : 108) && quartets < 148LL * 8 * 32 ? 1 : 0;
+}
 
 // Cartesian powers, reference order (integrals/cartesian.rs:113-136):
 // x exponent descending, then y exponent descending.

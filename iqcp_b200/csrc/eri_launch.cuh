@@ -2,38 +2,94 @@
 // Classes with many components use the warp-cooperative kernels
 // (eri_team.cuh); the small ones keep one quartet per thread.
 #pragma once
+#include <atomic>
+
 #include "eri_group.cuh"
 #include "eri_md.cuh"
 
 namespace iqcp {
 
 
-template <typename K>
-inline cudaError_t set_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// Device limits that every launch needs, asked once per device.
+struct DeviceLimits {
+  int sms = 0, smem_optin = 0;
+};
+inline DeviceLimits device_limits(int dev) {
+  static std::atomic<unsigned long long> known[64];  // SMs << 32 | opt-in shared memory; 0: not asked yet
+  const int slot = dev >= 0 && dev < 64 ? dev : -1;
+  unsigned long long v = slot >= 0 ? known[slot].load(std::memory_order_relaxed) : 0;
+  if (!v) {
+    int sms = 0, optin = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 1;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 0;
+    v = ((unsigned long long)sms << 32) | (unsigned)optin;
+    if (slot >= 0) known[slot].store(v, std::memory_order_relaxed);
+  }
+  DeviceLimits d;
+  d.sms = int(v >> 32);
+  d.smem_optin = int(v & 0xffffffffu);
+  return d;
+}
+inline size_t max_smem_optin() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return (size_t)device_limits(dev).smem_optin;
 }
 
-// Persistent grid: as many 128-thread blocks as are resident at once (capped
-// by the work), each looping over tasks; per-block set-up (the staged Rys
-// table, the gradient accumulator) is then paid once per resident block.
-template <typename K>
-inline int persistent_blocks(K kernel, size_t smem, int ntasks, int threads = 128) {
-  int per_sm = 0, dev = 0, sms = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+// Resident blocks of one kernel at one block size and shared-memory size, per
+// device.  The occupancy query and the shared-memory attribute cost as much
+// host time as the launch itself, 21 times per call; a kernel's answer for the
+// size last asked about is kept (a race between threads only asks again).  The
+// attribute is set to the device's limit, the same from every thread.
+struct LaunchCache {
+  std::atomic<unsigned long long> slot[64];  // (smem + 1) << 16 | blocks per SM; 0: not asked yet
+
+  template <typename K>
+  cudaError_t resident(K kernel, size_t smem, int threads, int* per_sm, int* sms) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const DeviceLimits lim = device_limits(dev);
+    *sms = lim.sms;
+    const unsigned long long key = (unsigned long long)(smem + 1) << 16;
+    if (dev < 64) {
+      const unsigned long long v = slot[dev].load(std::memory_order_relaxed);
+      if ((v >> 16 << 16) == key) {
+        *per_sm = int(v & 0xffff);
+        return cudaSuccess;
+      }
+    }
+    if (smem > 48 * 1024) {
+      if (smem > (size_t)lim.smem_optin) return cudaErrorInvalidValue;
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim.smem_optin);
+      if (e != cudaSuccess) return e;
+    }
+    int n = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    *per_sm = n > 0 ? n : 1;
+    if (dev < 64) slot[dev].store(key | (unsigned)*per_sm, std::memory_order_relaxed);
+    return cudaSuccess;
+  }
+};
+
+// Persistent grid: as many blocks as are resident at once (capped by the
+// work), each looping over tasks; per-block set-up (the staged tables, the
+// gradient accumulator) is then paid once per resident block.
+inline int persistent_blocks(int per_sm, int sms, int ntasks, int threads) {
   const int wpb = threads / 32;
   const int need = (ntasks + wpb - 1) / wpb;
-  const int cap = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
+  const int cap = per_sm * sms;
   return need < cap ? need : cap;
 }
 
-#define IQCP_LAUNCH_T(KERNEL, THREADS, SMEM, ARGS, ST)                                             \
-  do {                                                                                             \
-    cudaError_t e_ = set_smem(KERNEL, SMEM);                                                       \
-    if (e_ != cudaSuccess) return e_;                                                              \
-    KERNEL<<<persistent_blocks(KERNEL, SMEM, (ARGS).ntasks, THREADS), THREADS, SMEM, ST>>>(ARGS); \
+#define IQCP_LAUNCH_T(KERNEL, THREADS, SMEM, ARGS, ST)                                           \
+  do {                                                                                           \
+    static LaunchCache cache_;                                                                   \
+    int per_sm_ = 0, sms_ = 0;                                                                   \
+    cudaError_t e_ = cache_.resident(KERNEL, SMEM, THREADS, &per_sm_, &sms_);                    \
+    if (e_ != cudaSuccess) return e_;                                                            \
+    KERNEL<<<persistent_blocks(per_sm_, sms_, (ARGS).ntasks, THREADS), THREADS, SMEM, ST>>>(ARGS); \
   } while (0)
 #define IQCP_LAUNCH(KERNEL, SMEM, ARGS, ST) IQCP_LAUNCH_T(KERNEL, 128, SMEM, ARGS, ST)
 
@@ -42,42 +98,38 @@ inline int persistent_blocks(K kernel, size_t smem, int ntasks, int threads = 12
 // molecule: ~700 tasks for ~1300 warps) would leave SMs idle and end on its
 // longest task, so its tasks are split into 2, 4 or 8 slices of kets, each
 // a work item of its own.
-template <typename K>
-inline int team_ket_split(K kernel, size_t smem, int ntasks, int threads) {
-  int per_sm = 0, dev = 0, sms = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long warps = (long long)(per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1) * (threads / 32);
+inline int team_ket_split(int per_sm, int sms, int ntasks, int threads) {
+  const long long warps = (long long)per_sm * sms * (threads / 32);
   int s = 1;
   while (s < 8 && (long long)ntasks * s < 2 * warps) s *= 2;
   return s;
 }
 
-#define IQCP_LAUNCH_TEAM(KERNEL, THREADS, SMEM, ARGS, ST)                                                \
-  do {                                                                                                   \
-    cudaError_t e_ = set_smem(KERNEL, SMEM);                                                             \
-    if (e_ != cudaSuccess) return e_;                                                                    \
-    (ARGS).ket_split = team_ket_split(KERNEL, SMEM, (ARGS).ntasks, THREADS);                             \
-    KERNEL<<<persistent_blocks(KERNEL, SMEM, (ARGS).ntasks * (ARGS).ket_split, THREADS), THREADS, SMEM, \
-             ST>>>(ARGS);                                                                                \
+#define IQCP_LAUNCH_TEAM(KERNEL, THREADS, SMEM, ARGS, ST)                                                     \
+  do {                                                                                                        \
+    static LaunchCache cache_;                                                                                \
+    int per_sm_ = 0, sms_ = 0;                                                                                \
+    cudaError_t e_ = cache_.resident(KERNEL, SMEM, THREADS, &per_sm_, &sms_);                                 \
+    if (e_ != cudaSuccess) return e_;                                                                         \
+    (ARGS).ket_split = team_ket_split(per_sm_, sms_, (ARGS).ntasks, THREADS);                                 \
+    KERNEL<<<persistent_blocks(per_sm_, sms_, (ARGS).ntasks * (ARGS).ket_split, THREADS), THREADS, SMEM, ST>>>( \
+        ARGS);                                                                                                \
   } while (0)
 
-// J/K variants: 1 warp-cooperative (eri_team.cuh), every other mode a group of
-// lanes per quartet, as wide as the task says (build_tasks).  Above 324
-// components the FP32 share of a mixed call (pass 2) has the team kernel only.
+// J/K variants (kernel_variant): 1 warp-cooperative (eri_team.cuh), 0 a group of
+// lanes per quartet, as wide as the task says (build_tasks).
 template <typename R, int LA, int LB, int LC, int LD>
 cudaError_t launch_jk_variant(const JKArgs& a, cudaStream_t st) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr bool F32 = sizeof(R) == 4;
   const size_t tb = sizeof(double) * rys_tab_doubles<C::NR>();
-  const bool team = a.mode == 1 || (F32 && C::NCOMP > 324);
-  if (team) {
+  constexpr int X = pair_class(LA, LB), Y = pair_class(LC, LD);
+  if (kernel_variant(0, X, Y, a.mode, F32) == 1) {
     const size_t bytes = sizeof(double) * 4 * TeamJK<LA, LB, LC, LD>::PER_WARP + tb;
     JKArgs b = a;
     if (a.K) IQCP_LAUNCH_TEAM((jk_team_kernel<R, LA, LB, LC, LD, true>), 128, bytes, b, st);
     else IQCP_LAUNCH_TEAM((jk_team_kernel<R, LA, LB, LC, LD, false>), 128, bytes, b, st);
-  } else if constexpr (!F32 || C::NCOMP <= 324) {
+  } else if constexpr (C::NCOMP <= (F32 ? kMaxThreadComp32 : kMaxThreadComp)) {
     if (a.K) IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, true>), tb, a, st);
     else IQCP_LAUNCH((jk_kernel<R, LA, LB, LC, LD, false>), tb, a, st);
   }
@@ -90,21 +142,11 @@ cudaError_t launch_jk_class(const JKArgs& a, cudaStream_t st) {
   return launch_jk_variant<double, LA, LB, LC, LD>(a, st);
 }
 
-inline size_t max_smem_optin() {
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return (size_t)v;
-}
-
-// Gradient variants: mode 0 a group of lanes per quartet (build_tasks), mode 1
-// warp-cooperative, mode 2 as mode 0 with the D x D weights
-// in shared memory (classes of kWshMinComp..kWshMaxComp components; others map
-// to mode 0), mode 3 the grouped kernel of eri_group.cuh (up to
-// kGroupGradMaxComp components, 32 lanes per quartet; the FP32 share uses 8).
-constexpr int kWshMinComp = 18, kWshMaxComp = 108;
-constexpr int kGroupGradMaxComp = 108;
-
+// Gradient variants (kernel_variant): 1 warp-cooperative; 0 a group of lanes per
+// quartet, by Hermite expansions for FP64 classes with an ss or ps ket, by Rys
+// quadrature with the weights in shared memory for the other FP64 classes and
+// in registers for the FP32 share; 3 the grouped kernel of eri_group.cuh (32 lanes
+// per quartet, 8 for the FP32 share).
 template <int LA, int LB, int LC>
 cudaError_t launch_grad_md(const GradArgs& args, cudaStream_t st) {
   using G = GradMD<LA, LB, LC>;
@@ -120,40 +162,36 @@ template <typename R, int LA, int LB, int LC, int LD>
 cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr bool F32 = sizeof(R) == 4;
+  constexpr int X = pair_class(LA, LB), Y = pair_class(LC, LD);
   constexpr int NRG = grad_nroots(LA + LB + LC + LD);
-  constexpr bool WSH_OK = !F32 && LC + LD > 1 && C::NCOMP >= kWshMinComp && C::NCOMP <= kWshMaxComp;
-  using TG = TeamGrad2<LA, LB, LC, LD>;
-  // FP64 classes with an ss or ps ket: modes 0 and 2 are the Hermite kernel
   constexpr bool MD = !F32 && LC + LD <= 1;
-  const bool team = args.mode == 1 || (F32 && C::NCOMP > 324);
+  constexpr bool THREAD = !MD && C::NCOMP <= (F32 ? kMaxThreadComp32 : kMaxThreadComp);
+  using TG = TeamGrad2<LA, LB, LC, LD>;
+  const int variant = kernel_variant(1, X, Y, args.mode, F32);
   if constexpr (MD)
-    if (!team && args.mode != 3) return launch_grad_md<LA, LB, LC>(args, st);
-  const bool wsh = !team && args.mode == 2 && WSH_OK;
-  const bool group = !team && !wsh && (args.mode == 3 || (F32 && args.mode == 2)) && C::NCOMP <= kGroupGradMaxComp;
+    if (variant == 0) return launch_grad_md<LA, LB, LC>(args, st);
   // the team variant reads the Rys coefficients through L1 (no staged table)
   size_t fixed = sizeof(double) * rys_tab_doubles<NRG>();
-  if (team) fixed = sizeof(double) * TG::WPB * TG::PER_WARP;
-  else if (wsh)
+  if (variant == 1) fixed = sizeof(double) * TG::WPB * TG::PER_WARP;
+  else if (variant == 3)
+    fixed += sizeof(double) * (F32 ? GroupGrad<R, LA, LB, LC, LD, 8>::WDOUBLES : GroupGrad<R, LA, LB, LC, LD, 32>::WDOUBLES);
+  else if (!F32)
     fixed = sizeof(double) * (grad_stages_rys<LA, LB, LC, LD, true>() ? rys_tab_doubles<NRG>() : 0) +
             sizeof(R) * grad_wsh_doubles<LA, LB, LC, LD>();
-  else if (group)
-    fixed += sizeof(double) * (F32 ? GroupGrad<R, LA, LB, LC, LD, 8>::WDOUBLES : GroupGrad<R, LA, LB, LC, LD, 32>::WDOUBLES);
   // the per-block gradient accumulator only when it fits beside the tables
   GradArgs a = args;
   if (a.gsmem && fixed + sizeof(double) * 3 * a.natoms > max_smem_optin()) a.gsmem = 0;
   const size_t gacc = a.gsmem ? sizeof(double) * 3 * a.natoms : 0;
   const size_t bytes = fixed + gacc;
-  if (team) {
+  if (variant == 1) {
     IQCP_LAUNCH_TEAM((grad_team2_kernel<R, LA, LB, LC, LD>), 32 * TG::WPB, bytes, a, st);
-  } else if (wsh) {
-    if constexpr (WSH_OK) IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, true>), bytes, a, st);
-  } else if (group) {
-    if constexpr (C::NCOMP <= kGroupGradMaxComp) {
+  } else if (variant == 3) {
+    if constexpr (C::NCOMP <= kMaxGroupGradComp) {
       if (F32) IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 8>), bytes, a, st);
       else IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 32>), bytes, a, st);
     }
-  } else if constexpr (!MD && (!F32 || C::NCOMP <= 324)) {
-    IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD>), bytes, a, st);
+  } else if constexpr (THREAD) {
+    IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, !F32>), bytes, a, st);
   }
   return cudaGetLastError();
 }

@@ -295,11 +295,6 @@ __device__ __forceinline__ double group_sum(double v, int lg) {
   return v;
 }
 
-// Components up to which a quartet's primitive quartets can be shared by a
-// group of lanes (a task's `lg`); above, each lane takes a whole quartet
-// whatever the task says (the group's sum would cost more than it spreads).
-constexpr int kMaxGroupComp = 108;
-
 // J/K, one contracted quartet per group of 2^task.lg lanes: the groups of a warp
 // take consecutive kets of the task, the lanes of a group split the quartet's
 // primitive quartets and add their partial blocks by shuffles, and the first
@@ -315,7 +310,7 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
   const QuartetTask task = args.tasks[warp];
   const ShellPair bp = args.pairs[task.bra];
   if (task_inactive(args.mol_active, bp.mol)) continue;
-  const int lg = C::NCOMP <= kMaxGroupComp ? task.lg : 0;
+  const int lg = C::NCOMP <= kMaxThreadComp ? task.lg : 0;
   const int NG = 32 >> lg, grp = lane >> lg, sub = lane & ((1 << lg) - 1);
   // this task's molecule block (bra and ket pairs always share a molecule)
   const int n = args.mol_n[bp.mol];
@@ -343,7 +338,7 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
 #pragma unroll
       for (int i = 0; i < C::NCOMP; ++i) acc[i] = 0.0;
     }
-    if constexpr (C::NCOMP <= kMaxGroupComp) {
+    if constexpr (C::NCOMP <= kMaxThreadComp) {
       for (int o = (1 << lg) >> 1; o > 0; o >>= 1) {
 #pragma unroll
         for (int i = 0; i < C::NCOMP; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);

@@ -235,8 +235,7 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
   ctx->n_quartets = 0;
   for (int X = 0; X < NC; ++X)
     for (int Y = 0; Y <= X; ++Y) {
-      TaskRange r{X, Y, (int)tasks.size(), 0, 0, {default_mode(X, Y, 0), default_mode(X, Y, 1)},
-                  {default_mode(X, Y, 0), default_mode(X, Y, 1)}, {1, 1}};
+      TaskRange r{X, Y, (int)tasks.size(), 0, 0, {0, 0}, {0, 0}, {1, 1}};
       // kets of bucket bk of molecule m that pass Schwarz with bra b: a prefix
       auto bucket_kets = [&](const std::vector<int>& LY, const std::pair<int, int>& bk, int b, double qb) {
         int lo = bk.first, hi = (X == Y) ? std::min(bk.second, b + 1) : bk.second;
@@ -283,6 +282,7 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
         }
       });
       r.count = (int)tasks.size() - r.first;
+      for (int kind = 0; kind < 2; ++kind) r.mode[kind] = r.mode32[kind] = default_mode(X, Y, kind, r.quartets);
       ctx->ranges.push_back(r);
     }
 }
@@ -1428,7 +1428,9 @@ int iqcp_autotune(iqcp_ctx* ctx, const double* dD, int reps) {
                                      : r.count;
     float best = 1e30f;
     for (int mode = 0; mode < kNumModes; ++mode) {
-      if (pass == 2 && mode == 3) continue;  // the FP32 share has no 32-lane variant
+      // only modes that name their own kernel
+      if (kernel_variant(kind, r.X, r.Y, mode, pass == 2) != mode && !(pass == 2 && mode == 2)) continue;
+      if (pass == 2 && (mode == 3 || (kind == 0 && mode == 2))) continue;  // the FP32 share's lane groups are mode 2
       float tmin = 1e30f;
       for (int rep = 0; rep < reps + 1; ++rep) {  // first run warms caches and sets attributes
         CK(cudaMemsetAsync(ctx->d_Jt, 0, bytes, ctx->stream));
