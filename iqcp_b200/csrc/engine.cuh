@@ -95,6 +95,18 @@ struct __align__(16) ShellPair {
   int mol;        // molecule of a batched context (0 for a single geometry)
 };
 
+// Ket-side tables of the thread kernels, in the order of the ket lists: the lanes
+// of a warp take consecutive kets, so every field is an array of its own and a
+// warp's loads are contiguous.  The primitives of a bucket (m kets of np
+// primitives each) are stored [primitive][field][ket].
+struct KetTables {
+  const int4* i0;      // oa, ob, np, offset (unsigned) of the ket's first primitive field in prim
+  const int4* i1;      // atom_a, atom_b, comp, bucket size m (negative when both shells are the same)
+  const double* geom;  // A xyz, B xyz, Q: geom[f * n + position]
+  const double* prim;  // field f of primitive j: prim[offset + (8 j + f) m]; fields in PrimPair's order
+  int n;               // positions
+};
+
 // Unit of work for one warp: one bra pair against up to 32 consecutive ket
 // pairs of a class list.
 struct QuartetTask {
@@ -160,6 +172,7 @@ struct JKArgs {
   const ShellPair* pairs;
   const PrimPair* pp;
   const int* ket_list;
+  KetTables kets;
   const QuartetTask* tasks;
   int ntasks;
   const double* D;   // angular-scaled density
@@ -197,6 +210,7 @@ struct GradArgs {
   const ShellPair* pairs;
   const PrimPair* pp;
   const int* ket_list;
+  KetTables kets;
   const QuartetTask* tasks;
   int ntasks;
   const double* D;   // angular-scaled density
@@ -271,6 +285,9 @@ cudaError_t launch_shell_dmax(const double* D, const Packing& P, const int* shel
 // FP32 masks of the mixed form for every task (GRAD: density bound squared)
 cudaError_t launch_precision_masks(const ShellPair* pairs, const int* ket_list, const QuartetTask* tasks,
                                    int ntasks, const Mixed& mx, bool grad, unsigned* mask, cudaStream_t st);
+// Fill the ket tables: place[position] = {offset in prim, bucket size}
+cudaError_t launch_ket_tables(const ShellPair* pairs, const PrimPair* pp, const int* ket_list, const int2* place,
+                              int n, int4* i0, int4* i1, double* geom, double* prim, cudaStream_t st);
 cudaError_t launch_count_prim_quartets(const ShellPair* pairs, const PrimPair* pp, const int* ket_list,
                                        const QuartetTask* tasks, int ntasks, double thr,
                                        unsigned long long* out, cudaStream_t st);

@@ -172,6 +172,43 @@ cudaError_t launch_precision_masks(const ShellPair* pairs, const int* ket_list, 
   return cudaGetLastError();
 }
 
+// Ket tables from the pair and primitive records, a thread per position.
+__global__ void ket_tables_kernel(const ShellPair* __restrict__ pairs, const PrimPair* __restrict__ pp,
+                                  const int* __restrict__ ket_list, const int2* __restrict__ place, int n,
+                                  int4* __restrict__ i0, int4* __restrict__ i1, double* __restrict__ geom,
+                                  double* __restrict__ prim) {
+  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
+  if (pos >= n) return;
+  const ShellPair k = pairs[ket_list[pos]];
+  const int2 w = place[pos];
+  i0[pos] = make_int4(k.oa, k.ob, k.np, w.x);
+  i1[pos] = make_int4(k.atom_a, k.atom_b, k.comp, k.sa == k.sb ? -w.y : w.y);
+  for (int d = 0; d < 3; ++d) {
+    geom[(size_t)d * n + pos] = k.A[d];
+    geom[(size_t)(3 + d) * n + pos] = k.B[d];
+  }
+  geom[(size_t)6 * n + pos] = k.Q;
+  for (int j = 0; j < k.np; ++j) {
+    const PrimPair q = load_pp(pp + k.pstart + j);
+    double* o = prim + (unsigned)w.x + (size_t)8 * j * w.y;
+    o[0] = q.p;
+    o[(size_t)w.y] = q.P[0];
+    o[(size_t)2 * w.y] = q.P[1];
+    o[(size_t)3 * w.y] = q.P[2];
+    o[(size_t)4 * w.y] = q.K;
+    o[(size_t)5 * w.y] = q.cK;
+    o[(size_t)6 * w.y] = q.aa;
+    o[(size_t)7 * w.y] = q.inv_p;
+  }
+}
+
+cudaError_t launch_ket_tables(const ShellPair* pairs, const PrimPair* pp, const int* ket_list, const int2* place,
+                              int n, int4* i0, int4* i1, double* geom, double* prim, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  ket_tables_kernel<<<nblk(n, 128), 128, 0, st>>>(pairs, pp, ket_list, place, n, i0, i1, geom, prim);
+  return cudaGetLastError();
+}
+
 // Surviving primitive quartets (K_ij * K_kl >= thr) of a task range.
 __global__ void count_prim_quartets_kernel(const ShellPair* __restrict__ pairs, const PrimPair* __restrict__ pp,
                                            const int* __restrict__ ket_list, const QuartetTask* __restrict__ tasks,

@@ -268,10 +268,11 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
       const int kk = kbase + grp;
       bool active = kk < nsel;
       ShellPair kp = bp;
+      KetPrims ket{nullptr, 0};
       int kpos = 0;
       if (active) {
         kpos = task.ket0 + (args.mx.pass ? nth_set_bit(sel, kk) : kk);
-        kp = args.pairs[__ldg(args.ket_list + kpos)];
+        kp = load_ket(args.kets, kpos, bp.mol, &ket);
         // the reference skips when the Schwarz bound of its bra pair (the larger
         // composite index) is below threshold (gradient.rs:1457-1460)
         const double qref = bp.comp >= kp.comp ? bp.Q : kp.Q;
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
         if (!active) continue;
         PrimPair k;
         for (PrimItems it(nb, kp.np, sub, 1 << lg); it.more(); it.next()) {  // ket-major order (see quartet)
-          if (it.new_ket()) k = load_pp(args.pp + kp.pstart + it.j);
+          if (it.new_ket()) k = ket(it.j);
           const PrimPair b = load_pp(args.pp + bp.pstart + i0 + it.i);
           if (b.K * k.K < args.prim_thr) continue;
           const StagedPtr<HB::Main::TOTAL> E = Est + it.i * HB::PER;

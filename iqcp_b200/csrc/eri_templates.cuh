@@ -166,6 +166,57 @@ __device__ __forceinline__ PrimPair load_pp(const PrimPair* __restrict__ p) {
   return r;
 }
 
+// Primitive j of a ket: from the shell pair's own list (one pair per warp), or
+// from the ket tables, where neighbouring lanes read neighbouring words; a 64-byte
+// record per lane costs a cache line per lane and load.
+struct PairPrims {
+  const PrimPair* p;
+  __device__ __forceinline__ PrimPair operator()(int j) const { return load_pp(p + j); }
+};
+struct KetPrims {
+  const double* p;
+  int m;
+  __device__ __forceinline__ PrimPair operator()(int j) const {
+    const double* s = p + 8 * j * m;
+    PrimPair r;
+    r.p = __ldg(s);
+    r.P[0] = __ldg(s + m);
+    r.P[1] = __ldg(s + 2 * m);
+    r.P[2] = __ldg(s + 3 * m);
+    r.K = __ldg(s + 4 * m);
+    r.cK = __ldg(s + 5 * m);
+    r.aa = __ldg(s + 6 * m);
+    r.inv_p = __ldg(s + 7 * m);
+    return r;
+  }
+};
+
+// Ket at a position of the ket tables (sa == sb when its shells are the same;
+// otherwise the two are only unequal)
+__device__ __forceinline__ ShellPair load_ket(const KetTables& t, int pos, int mol, KetPrims* prims) {
+  const int4 a = __ldg(t.i0 + pos), b = __ldg(t.i1 + pos);
+  ShellPair k;
+  k.oa = a.x;
+  k.ob = a.y;
+  k.np = a.z;
+  k.atom_a = b.x;
+  k.atom_b = b.y;
+  k.comp = b.z;
+  k.sa = 0;
+  k.sb = b.w < 0 ? 0 : 1;
+  k.mol = mol;
+  k.pstart = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    k.A[d] = __ldg(t.geom + d * t.n + pos);
+    k.B[d] = __ldg(t.geom + (3 + d) * t.n + pos);
+  }
+  k.Q = __ldg(t.geom + 6 * t.n + pos);
+  prims->p = t.prim + (unsigned)a.w;
+  prims->m = b.w < 0 ? -b.w : b.w;
+  return k;
+}
+
 // The primitive quartets (i, j) of a contracted quartet with nb x nk primitive
 // pairs, in ket-major order (i fastest), starting at item `first` and stepping
 // by `stride`.  The division is done once per quartet: per step it would cost
@@ -208,9 +259,9 @@ struct PrimItems {
 // form, where the roots, weights and recurrence coefficients are formed in
 // FP64 and rounded once, and each primitive quartet's FP32 block is added to
 // the FP64 accumulators.
-template <typename R, int LA, int LB, int LC, int LD>
+template <typename R, int LA, int LB, int LC, int LD, typename KetLoad>
 __device__ __forceinline__ void quartet(const ShellPair& bp, const ShellPair& kp, const PrimPair* __restrict__ pp,
-                                        double thr, double* __restrict__ acc, int first = 0, int stride = 1,
+                                        const KetLoad& ket, double thr, double* __restrict__ acc, int first = 0, int stride = 1,
                                         const double* rtab = nullptr) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr bool F32 = sizeof(R) == 4;
@@ -223,7 +274,7 @@ __device__ __forceinline__ void quartet(const ShellPair& bp, const ShellPair& kp
   // across lanes, is loaded once per j
   PrimPair k;
   for (PrimItems it(bp.np, kp.np, first, stride); it.more(); it.next()) {
-    if (it.new_ket()) k = load_pp(pp + kp.pstart + it.j);
+    if (it.new_ket()) k = ket(it.j);
     const PrimPair b = load_pp(pp + bp.pstart + it.i);
     if (b.K * k.K < thr) continue;
     const double p = b.p, q = k.p, s = p + q;
@@ -299,8 +350,13 @@ __device__ __forceinline__ double group_sum(double v, int lg) {
 // take consecutive kets of the task, the lanes of a group split the quartet's
 // primitive quartets and add their partial blocks by shuffles, and the first
 // lane of each group digests the block.
+// Resident blocks asked of the compiler: up to L = 2 what the registers of a
+// spill-free build allow (left alone it takes 166 registers for (ps|ps), three
+// blocks, where 128 cost 12 bytes of spill).
+__host__ __device__ constexpr int jk_min_blocks(int L) { return L == 0 ? 6 : (L == 1 ? 5 : (L == 2 ? 4 : 1)); }
+
 template <typename R, int LA, int LB, int LC, int LD, bool DO_K>
-__global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
+__global__ void __launch_bounds__(128, jk_min_blocks(LA + LB + LC + LD)) jk_kernel(JKArgs args) {
   using C = Cls<LA, LB, LC, LD>;
   extern __shared__ __align__(16) double rtab[];
   rys_stage_table<C::NR>(rtab);
@@ -328,8 +384,9 @@ __global__ void __launch_bounds__(128) jk_kernel(JKArgs args) {
     ShellPair kp = bp;
     if (active) {
       const int kpos = task.ket0 + (args.mx.pass ? nth_set_bit(sel, kk) : kk);
-      kp = args.pairs[__ldg(args.ket_list + kpos)];
-      quartet<R, LA, LB, LC, LD>(bp, kp, args.pp, args.prim_thr, acc, sub, 1 << lg, rtab);
+      KetPrims ket;
+      kp = load_ket(args.kets, kpos, bp.mol, &ket);
+      quartet<R, LA, LB, LC, LD>(bp, kp, args.pp, ket, args.prim_thr, acc, sub, 1 << lg, rtab);
       f = 1.0;
       if (bp.sa == bp.sb) f *= 0.5;
       if (kp.sa == kp.sb) f *= 0.5;
@@ -455,7 +512,7 @@ __global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const Pr
   const int pid = list[t];
   const ShellPair bp = pairs[pid];
   double acc[C::NCOMP];
-  quartet<double, LA, LB, LA, LB>(bp, bp, pp, thr, acc);
+  quartet<double, LA, LB, LA, LB>(bp, bp, pp, PairPrims{pp + bp.pstart}, thr, acc);
   double mx = 0.0;
 #pragma unroll
   for (int a = 0; a < C::NA; ++a)
@@ -489,7 +546,7 @@ __global__ void __launch_bounds__(128) store_kernel(StoreArgs args) {
   const ShellPair bp = args.pairs[task.bra];
   const ShellPair kp = args.pairs[args.ket_list[task.ket0 + lane]];
   double acc[C::NCOMP];
-  quartet<double, LA, LB, LC, LD>(bp, kp, args.pp, args.prim_thr, acc);
+  quartet<double, LA, LB, LC, LD>(bp, kp, args.pp, PairPrims{args.pp + kp.pstart}, args.prim_thr, acc);
 #pragma unroll
   for (int a = 0; a < C::NA; ++a)
 #pragma unroll
@@ -601,10 +658,11 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
     const int kk = kbase + grp;
     bool active = kk < nsel;
     ShellPair kp = bp;
+    KetPrims ket{nullptr, 0};
     int kpos = 0;
     if (active) {
       kpos = task.ket0 + (args.mx.pass ? nth_set_bit(sel, kk) : kk);
-      kp = args.pairs[__ldg(args.ket_list + kpos)];
+      kp = load_ket(args.kets, kpos, bp.mol, &ket);
       // the reference skips when the Schwarz bound of its bra pair (the larger
       // composite index) is below threshold (gradient.rs:1457-1460)
       const double qref = bp.comp >= kp.comp ? bp.Q : kp.Q;
@@ -649,7 +707,7 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
       const double CD[3] = {kp.A[0] - kp.B[0], kp.A[1] - kp.B[1], kp.A[2] - kp.B[2]};
       PrimPair k;
       for (PrimItems it(bp.np, kp.np, sub, 1 << lg); it.more(); it.next()) {  // ket-major order (see quartet)
-        if (it.new_ket()) k = load_pp(args.pp + kp.pstart + it.j);
+        if (it.new_ket()) k = ket(it.j);
         const PrimPair b = load_pp(args.pp + bp.pstart + it.i);
         if (b.K * k.K < args.prim_thr) continue;
         const double p = b.p, q = k.p, s = p + q;

@@ -59,6 +59,7 @@ struct iqcp_ctx {
   ShellPair* d_pairs = nullptr;
   PrimPair* d_pp = nullptr;
   int* d_ket_list = nullptr;      // class lists concatenated
+  KetTables kets{};               // the same order (device arrays)
   QuartetTask* d_tasks = nullptr;
   double* d_ang = nullptr;        // per basis function angular factor
   double* d_Ds = nullptr;         // scaled density
@@ -203,7 +204,9 @@ constexpr double kResidentLanes = 148 * 16 * 32;  // SMs x resident warps of the
 // 32 kets, or fewer with a group of lanes each where the quartets are deeply
 // contracted (more primitive quartets than the range's even share of a
 // resident lane) or where a bucket's last kets would leave lanes idle.
-void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetTask>& tasks) {
+// place: per ket-list position its primitives' place in the ket tables.
+int build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<int2>& place, long long* prim_doubles,
+                std::vector<QuartetTask>& tasks) {
   const double thr = ctx->opt.schwarz_threshold;
   const int NC = kNumPairClasses;
   std::vector<std::vector<int>> lists((size_t)ctx->n_mol * NC);
@@ -214,6 +217,8 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
   std::vector<int> seg((size_t)ctx->n_mol * NC);
   std::vector<std::vector<std::pair<int, int>>> buckets((size_t)ctx->n_mol * NC);
   ket_list.clear();
+  place.clear();
+  long long prims = 0;
   for (size_t li = 0; li < lists.size(); ++li) {
     auto& v = lists[li];
     std::stable_sort(v.begin(), v.end(), [&](int a, int b) {
@@ -225,11 +230,16 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
       size_t e0 = s0;
       while (e0 < v.size() && ctx->pairs[v[e0]].np == ctx->pairs[v[s0]].np) ++e0;
       buckets[li].push_back({(int)s0, (int)e0});
+      for (size_t k = s0; k < e0; ++k)
+        place.push_back(make_int2((int)(unsigned)(prims + (long long)(k - s0)), (int)(e0 - s0)));
+      prims += 8LL * ctx->pairs[v[s0]].np * (long long)(e0 - s0);
       s0 = e0;
     }
     seg[li] = (int)ket_list.size();
     ket_list.insert(ket_list.end(), v.begin(), v.end());
   }
+  if (prims > 0xffffffffLL) return fail(ctx, IQCP_ERR_NOMEM, "more primitive pairs than the ket tables address");
+  *prim_doubles = prims;
   tasks.clear();
   ctx->ranges.clear();
   ctx->n_quartets = 0;
@@ -285,6 +295,7 @@ void build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<QuartetT
       for (int kind = 0; kind < 2; ++kind) r.mode[kind] = r.mode32[kind] = default_mode(X, Y, kind, r.quartets);
       ctx->ranges.push_back(r);
     }
+  return IQCP_OK;
 }
 
 int ensure_device(iqcp_ctx* ctx) {
@@ -321,6 +332,7 @@ JKArgs jk_args(const iqcp_ctx* ctx, const TaskRange& r, const double* Ds, double
   a.pairs = ctx->d_pairs;
   a.pp = ctx->d_pp;
   a.ket_list = ctx->d_ket_list;
+  a.kets = ctx->kets;
   a.tasks = ctx->d_tasks + r.first;
   a.ntasks = r.count;
   a.D = Ds;
@@ -346,6 +358,7 @@ GradArgs grad_args(const iqcp_ctx* ctx, const TaskRange& r, const double* Ds, do
   a.pairs = ctx->d_pairs;
   a.pp = ctx->d_pp;
   a.ket_list = ctx->d_ket_list;
+  a.kets = ctx->kets;
   a.tasks = ctx->d_tasks + r.first;
   a.ntasks = r.count;
   a.D = Ds;
@@ -745,14 +758,39 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
     CK(cudaMemcpy(ctx->pairs.data(), ctx->d_pairs, sizeof(ShellPair) * npairs, cudaMemcpyDeviceToHost));
   }
   std::vector<int> ket_list;
+  std::vector<int2> place;
   std::vector<QuartetTask> tasks;
-  build_tasks(ctx, ket_list, tasks);
+  long long prim_doubles = 0;
+  {
+    const int rc = build_tasks(ctx, ket_list, place, &prim_doubles, tasks);
+    if (rc) return rc;
+  }
   if (ket_list.empty()) ket_list.push_back(0);
   if (tasks.empty()) tasks.push_back(QuartetTask());
   ctx->n_tasks = (int)tasks.size();
   CK(cudaMalloc(&ctx->d_mask, sizeof(unsigned) * tasks.size()));
   CK(cudaMalloc(&ctx->d_ket_list, sizeof(int) * ket_list.size()));
   CK(cudaMemcpy(ctx->d_ket_list, ket_list.data(), sizeof(int) * ket_list.size(), cudaMemcpyHostToDevice));
+  {
+    const int n = (int)place.size();
+    int2* d_place = nullptr;
+    int4 *i0 = nullptr, *i1 = nullptr;
+    double *geom = nullptr, *prim = nullptr;
+    CK(cudaMalloc(&d_place, sizeof(int2) * (n > 0 ? n : 1)));
+    CK(cudaMalloc(&i0, sizeof(int4) * (n > 0 ? n : 1)));
+    ctx->kets.i0 = i0;
+    CK(cudaMalloc(&i1, sizeof(int4) * (n > 0 ? n : 1)));
+    ctx->kets.i1 = i1;
+    CK(cudaMalloc(&geom, sizeof(double) * 7 * (n > 0 ? n : 1)));
+    ctx->kets.geom = geom;
+    CK(cudaMalloc(&prim, sizeof(double) * (prim_doubles > 0 ? prim_doubles : 1)));
+    ctx->kets.prim = prim;
+    ctx->kets.n = n;
+    CK(cudaMemcpy(d_place, place.data(), sizeof(int2) * n, cudaMemcpyHostToDevice));
+    CK(launch_ket_tables(ctx->d_pairs, ctx->d_pp, ctx->d_ket_list, d_place, n, i0, i1, geom, prim, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaFree(d_place));
+  }
   CK(cudaMalloc(&ctx->d_tasks, sizeof(QuartetTask) * tasks.size()));
   CK(cudaMemcpy(ctx->d_tasks, tasks.data(), sizeof(QuartetTask) * tasks.size(), cudaMemcpyHostToDevice));
 
@@ -811,6 +849,10 @@ void iqcp_destroy(iqcp_ctx* ctx) {
   cudaFree(ctx->d_pairs);
   cudaFree(ctx->d_pp);
   cudaFree(ctx->d_ket_list);
+  cudaFree(const_cast<int4*>(ctx->kets.i0));
+  cudaFree(const_cast<int4*>(ctx->kets.i1));
+  cudaFree(const_cast<double*>(ctx->kets.geom));
+  cudaFree(const_cast<double*>(ctx->kets.prim));
   cudaFree(ctx->d_tasks);
   cudaFree(ctx->d_ang);
   cudaFree(ctx->d_Ds);
