@@ -11,18 +11,16 @@
 #include <vector>
 
 #include "../../include/iqcp.h"
+#include "device_pool.h"
 #include "engine.cuh"
 #include "internal.h"
+#include "tasks.h"
 
 #include "basis_tables.inc"
 
 using namespace iqcp;
 
 namespace {
-
-struct ClassList {
-  std::vector<int> pairs;   // ShellPair ids sorted by Q descending
-};
 
 struct TaskRange {
   int X, Y;
@@ -39,8 +37,10 @@ struct iqcp_ctx {
   std::string err;
   int device = 0;
   iqcp_options opt;
+  StreamSet streams;               // the context's own stream and kSide side streams
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
+  DeviceBlock block[3];            // tables and work buffers; ket tables; tasks
   int nbf = 0, n_shells = 0, n_atoms = 0;   // totals over the molecules of the context
   // batched contexts: molecule m owns rows/cols [0, mol_nbf[m]) of the block at
   // mol_base[m] in every packed matrix (D, J, K, F, H, S) and atoms
@@ -93,8 +93,6 @@ struct iqcp_ctx {
   int* d_cls_list = nullptr;
   // host copies
   std::vector<ShellPair> pairs;
-  std::vector<int> list_offset;   // per class, into d_ket_list
-  std::vector<ClassList> classes;
   std::vector<TaskRange> ranges;
   long long n_quartets = 0;
   double stats[4] = {0, 0, 0, 0};
@@ -102,7 +100,7 @@ struct iqcp_ctx {
   // class launches run concurrently on the context stream and these side
   // streams (forked and joined with events), so one class's tail overlaps
   // the next class's start
-  static constexpr int kSide = 3;
+  static constexpr int kSide = kSetStreams - 1;
   cudaStream_t side[kSide] = {nullptr, nullptr, nullptr};
   cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {nullptr, nullptr, nullptr};
   // per-launch timing of the quartet kernels (off unless requested)
@@ -177,124 +175,150 @@ int basis_id(const char* name) {
   return -1;
 }
 
-// Lanes per quartet (a power of two, returned as its logarithm) of a task whose
-// quartets have `prims` primitive quartets each, when one lane should serve
-// about `per_lane` of them.  A thread that walks a deeply contracted quartet
-// alone is what a small build waits for: 36 x 36 primitive quartets of an
-// (ss|ss) quartet in 6-31G* took 0.68 ms of the 0.90 ms H2O Fock build, and
-// 64 x 64 in cc-pVDZ 3.0 ms, whatever the other 4000 warps did.
-int lanes_log2(double prims, double per_lane) {
-  int lg = 0;
-  while (lg < 5 && prims > per_lane * (1 << lg)) ++lg;
-  return lg;
-}
-
 // Primitive quartets per lane below which splitting a quartet further costs more
 // (group sums, digestion by one lane in 2^lg) than its shorter chain saves.
 constexpr double kMinPrimsPerLane = 16;
 constexpr double kResidentLanes = 148 * 16 * 32;  // SMs x resident warps of the thread kernels x lanes
 
-// Build class lists and quartet tasks from Schwarz bounds held in ctx->pairs.
-// Per molecule, each class list is split into buckets of equal primitive-pair
-// count (so the 32 kets of a warp share one primitive-loop length), each
-// bucket sorted by Q descending so that the Schwarz test Q_bra * Q_ket >= thr
-// keeps a prefix of it.  Unique quartets of a class with itself keep ket
-// position <= bra position.  Tasks never mix molecules; the tasks of one class
-// pair over all molecules form one range (one launch).  A task fills a warp:
-// 32 kets, or fewer with a group of lanes each where the quartets are deeply
-// contracted (more primitive quartets than the range's even share of a
-// resident lane) or where a bucket's last kets would leave lanes idle.
-// place: per ket-list position its primitives' place in the ket tables.
-int build_tasks(iqcp_ctx* ctx, std::vector<int>& ket_list, std::vector<int2>& place, long long* prim_doubles,
-                std::vector<QuartetTask>& tasks) {
-  const double thr = ctx->opt.schwarz_threshold;
-  const int NC = kNumPairClasses;
-  std::vector<std::vector<int>> lists((size_t)ctx->n_mol * NC);
-  for (int i = 0; i < (int)ctx->pairs.size(); ++i) {
+// Class lists, ket tables and quartet tasks from the Schwarz bounds in
+// ctx->pairs.  Per molecule, each class list is split into buckets of equal
+// primitive-pair count (so the 32 kets of a warp share one primitive-loop
+// length), each bucket sorted by Q descending so that the Schwarz test
+// Q_bra * Q_ket >= thr keeps a prefix of it.  Unique quartets of a class with
+// itself keep ket position <= bra position.  Tasks never mix molecules; the
+// tasks of one class pair over all molecules form one range (one launch).
+//
+// A task fills a warp: 32 kets, or fewer with a group of 2^lg lanes each where
+// the quartets are deeply contracted (more primitive quartets than the range's
+// even share of a resident lane) or where a bucket's last kets would leave lanes
+// idle.  A thread that walks a deeply contracted quartet alone is what a small
+// build waits for: 36 x 36 primitive quartets of an (ss|ss) quartet in 6-31G* took
+// 0.68 ms of the 0.90 ms H2O Fock build, and 64 x 64 in cc-pVDZ 3.0 ms, whatever the
+// other 4000 warps did.
+int build_tasks(iqcp_ctx* ctx) {
+  const int NC = kNumPairClasses, nseg = ctx->n_mol * NC, n = (int)ctx->pairs.size();
+  struct Key {
+    double Q;
+    int np, id;
+  };
+  std::vector<int> seg(nseg + 1, 0), rank(nseg, 0), bucket0(nseg + 1, 0), pos_seg(n), ket_list(n);
+  std::vector<int> seg_of(n);
+  for (int i = 0; i < n; ++i) {
     const ShellPair& p = ctx->pairs[i];
-    lists[(size_t)p.mol * NC + pair_class(ctx->shell_l[p.sa], ctx->shell_l[p.sb])].push_back(i);
+    seg_of[i] = p.mol * NC + pair_class(ctx->shell_l[p.sa], ctx->shell_l[p.sb]);
+    ++seg[seg_of[i] + 1];
   }
-  std::vector<int> seg((size_t)ctx->n_mol * NC);
-  std::vector<std::vector<std::pair<int, int>>> buckets((size_t)ctx->n_mol * NC);
-  ket_list.clear();
-  place.clear();
+  for (int s = 0; s < nseg; ++s) seg[s + 1] += seg[s];
+  std::vector<Key> keys(n);
+  {
+    std::vector<int> at(seg.begin(), seg.end() - 1);
+    for (int i = 0; i < n; ++i) keys[at[seg_of[i]]++] = Key{ctx->pairs[i].Q, ctx->pairs[i].np, i};
+  }
+  std::vector<int4> bucket;
+  std::vector<int2> place(n);
+  std::vector<double> Q(n);
   long long prims = 0;
-  for (size_t li = 0; li < lists.size(); ++li) {
-    auto& v = lists[li];
-    std::stable_sort(v.begin(), v.end(), [&](int a, int b) {
-      const ShellPair &pa = ctx->pairs[a], &pb = ctx->pairs[b];
-      if (pa.np != pb.np) return pa.np > pb.np;
-      return pa.Q > pb.Q;
+  int count[kNumPairClasses] = {0};
+  for (int s = 0; s < nseg; ++s) {
+    std::stable_sort(keys.begin() + seg[s], keys.begin() + seg[s + 1], [](const Key& a, const Key& b) {
+      return a.np != b.np ? a.np > b.np : a.Q > b.Q;
     });
-    for (size_t s0 = 0; s0 < v.size();) {
-      size_t e0 = s0;
-      while (e0 < v.size() && ctx->pairs[v[e0]].np == ctx->pairs[v[s0]].np) ++e0;
-      buckets[li].push_back({(int)s0, (int)e0});
-      for (size_t k = s0; k < e0; ++k)
-        place.push_back(make_int2((int)(unsigned)(prims + (long long)(k - s0)), (int)(e0 - s0)));
-      prims += 8LL * ctx->pairs[v[s0]].np * (long long)(e0 - s0);
-      s0 = e0;
+    rank[s] = count[s % NC];
+    count[s % NC] += seg[s + 1] - seg[s];
+    bucket0[s] = (int)bucket.size();
+    for (int k0 = seg[s]; k0 < seg[s + 1];) {
+      int k1 = k0;
+      while (k1 < seg[s + 1] && keys[k1].np == keys[k0].np) ++k1;
+      const int m = k1 - k0;
+      bucket.push_back(make_int4(k0, m, keys[k0].np, 0));
+      for (int k = k0; k < k1; ++k) {
+        place[k] = make_int2((int)(unsigned)(prims + (k - k0)), m);
+        ket_list[k] = keys[k].id;
+        pos_seg[k] = s;
+        Q[k] = keys[k].Q;
+      }
+      prims += 8LL * keys[k0].np * m;
+      k0 = k1;
     }
-    seg[li] = (int)ket_list.size();
-    ket_list.insert(ket_list.end(), v.begin(), v.end());
   }
+  bucket0[nseg] = (int)bucket.size();
   if (prims > 0xffffffffLL) return fail(ctx, IQCP_ERR_NOMEM, "more primitive pairs than the ket tables address");
-  *prim_doubles = prims;
-  tasks.clear();
+
+  TaskLists t{};
+  t.n = n;
+  t.n_seg = nseg;
+  t.thr = ctx->opt.schwarz_threshold;
+  for (int X = 0; X < NC; ++X)
+    for (int Y = 0; Y <= X; ++Y) t.entry0[range_of(X, Y) + 1] = t.entry0[range_of(X, Y)] + count[X];
+  const int entries = t.entry0[kNumRanges];
+  // the ket tables stay; the lists only serve the construction
+  int4 *i0 = nullptr, *i1 = nullptr;
+  double *geom = nullptr, *prim = nullptr;
+  ctx->block[1].upload(&ctx->d_ket_list, ket_list.data(), n);
+  ctx->block[1].want(&i0, n);
+  ctx->block[1].want(&i1, n);
+  ctx->block[1].want(&geom, (size_t)7 * n);
+  ctx->block[1].want(&prim, (size_t)prims);
+  CK(ctx->block[1].alloc(ctx->device, ctx->stream));
+  ctx->kets = KetTables{i0, i1, geom, prim, n};
+  DeviceBlock tmp;
+  struct Release {
+    DeviceBlock& b;
+    cudaStream_t st;
+    ~Release() { b.free(st); }
+  } release{tmp, ctx->stream};
+  int2* d_place = nullptr;
+  int *d_pos_seg = nullptr, *d_seg = nullptr, *d_rank = nullptr, *d_bucket0 = nullptr, *offset = nullptr,
+      *part = nullptr, *first = nullptr;
+  int4* d_bucket = nullptr;
+  unsigned long long* sums = nullptr;
+  tmp.upload(&d_place, place.data(), n);
+  tmp.upload(&d_pos_seg, pos_seg.data(), n);
+  tmp.upload(&d_seg, seg.data(), seg.size());
+  tmp.upload(&d_rank, rank.data(), rank.size());
+  tmp.upload(&d_bucket0, bucket0.data(), bucket0.size());
+  tmp.upload(&d_bucket, bucket.data(), bucket.size());
+  tmp.want(&offset, (size_t)entries + 1);
+  tmp.want(&part, (size_t)entries / 1024 + 2);
+  tmp.want(&first, kNumRanges + 1);
+  tmp.want(&sums, 2 * kNumRanges);
+  CK(tmp.alloc(ctx->device, ctx->stream));
+  t.ket_list = ctx->d_ket_list;
+  t.pos_seg = d_pos_seg;
+  t.seg = d_seg;
+  t.seg_rank = d_rank;
+  t.bucket0 = d_bucket0;
+  t.bucket = d_bucket;
+  t.i0 = i0;
+  t.Q = geom + (size_t)6 * n;
+  CK(launch_ket_tables(ctx->d_pairs, ctx->d_pp, ctx->d_ket_list, d_place, n, i0, i1, geom, prim, ctx->stream));
+  CK(launch_task_work(t, sums, ctx->stream));
+  unsigned long long work[2 * kNumRanges];
+  CK(cudaMemcpyAsync(work, sums, sizeof(work), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  PerLane per;
+  for (int r = 0; r < kNumRanges; ++r) per.v[r] = std::max(kMinPrimsPerLane, (double)work[2 * r] / kResidentLanes);
+  CK(launch_task_offsets(t, per, offset, part, first, ctx->stream));
+  int h_first[kNumRanges + 1];
+  CK(cudaMemcpyAsync(h_first, first, sizeof(h_first), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  if (h_first[kNumRanges] < 0) return fail(ctx, IQCP_ERR_NOMEM, "more than 2^31 quartet tasks");
+  ctx->n_tasks = h_first[kNumRanges];
   ctx->ranges.clear();
   ctx->n_quartets = 0;
   for (int X = 0; X < NC; ++X)
     for (int Y = 0; Y <= X; ++Y) {
-      TaskRange r{X, Y, (int)tasks.size(), 0, 0, {0, 0}, {0, 0}, {1, 1}};
-      // kets of bucket bk of molecule m that pass Schwarz with bra b: a prefix
-      auto bucket_kets = [&](const std::vector<int>& LY, const std::pair<int, int>& bk, int b, double qb) {
-        int lo = bk.first, hi = (X == Y) ? std::min(bk.second, b + 1) : bk.second;
-        while (lo < hi) {
-          const int mid = (lo + hi) / 2;
-          if (qb * ctx->pairs[LY[mid]].Q < thr) hi = mid; else lo = mid + 1;
-        }
-        return lo - bk.first;
-      };
-      auto for_buckets = [&](auto&& f) {
-        for (int m = 0; m < ctx->n_mol; ++m) {
-          const size_t lx = (size_t)m * NC + X, ly = (size_t)m * NC + Y;
-          const auto& LX = lists[lx];
-          const auto& LY = lists[ly];
-          for (int b = 0; b < (int)LX.size(); ++b) {
-            const ShellPair& bp = ctx->pairs[LX[b]];
-            for (const auto& bk : buckets[ly]) {
-              if (X == Y && bk.first > b) break;
-              const int nk = bucket_kets(LY, bk, b, bp.Q);
-              if (nk > 0) f(lx, ly, b, LX[b], bk.first, nk, (double)bp.np * ctx->pairs[LY[bk.first]].np);
-            }
-          }
-        }
-      };
-      double work = 0.0;  // primitive quartets of the range
-      for_buckets([&](size_t, size_t, int, int, int, int nk, double prims) { work += nk * prims; });
-      const double per_lane = std::max(kMinPrimsPerLane, work / kResidentLanes);
-      for_buckets([&](size_t lx, size_t ly, int b, int bra, int first, int nk, double prims) {
-        ctx->n_quartets += nk;
-        r.quartets += nk;
-        const int lg = lanes_log2(prims, per_lane);
-        for (int k0 = 0; k0 < nk;) {
-          QuartetTask t;
-          t.bra = bra;
-          t.ket0 = seg[ly] + first + k0;
-          t.nket = std::min(32 >> lg, nk - k0);
-          t.diag = (X == Y) ? 1 : 0;
-          t.bra_pos = seg[lx] + b;
-          t.lg = lg;
-          // the bucket's last kets: spread over the lanes left, two primitive quartets a lane at least
-          while (t.lg < 5 && (t.nket << (t.lg + 1)) <= 32 && prims >= double(4 << t.lg)) ++t.lg;
-          k0 += t.nket;
-          tasks.push_back(t);
-        }
-      });
-      r.count = (int)tasks.size() - r.first;
+      const int k = range_of(X, Y);
+      TaskRange r{X, Y, h_first[k], h_first[k + 1] - h_first[k], (long long)work[2 * k + 1], {0, 0}, {0, 0}, {1, 1}};
       for (int kind = 0; kind < 2; ++kind) r.mode[kind] = r.mode32[kind] = default_mode(X, Y, kind, r.quartets);
+      ctx->n_quartets += r.quartets;
       ctx->ranges.push_back(r);
     }
+  ctx->block[2].want(&ctx->d_tasks, ctx->n_tasks);
+  ctx->block[2].want(&ctx->d_mask, ctx->n_tasks);
+  ctx->block[2].want(&ctx->d_counters, 4 * (ctx->ranges.size() + 1));
+  CK(ctx->block[2].alloc(ctx->device, ctx->stream));
+  CK(launch_task_fill(t, per, offset, ctx->d_tasks, ctx->stream));
   return IQCP_OK;
 }
 
@@ -573,17 +597,18 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= ctx->device)
     return fail(ctx, IQCP_ERR_NODEVICE, "no CUDA device available");
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, ctx->device));
-  if (prop.major != 10) return fail(ctx, IQCP_ERR_NODEVICE, "libiqcp_gpu is built for sm_100a only");
+  int major = 0;
+  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->device));
+  if (major != 10) return fail(ctx, IQCP_ERR_NODEVICE, "libiqcp_gpu is built for sm_100a only");
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking));
+  CK(streams_take(ctx->device, &ctx->streams));
+  ctx->own_stream = ctx->streams.s[0];
   ctx->stream = ctx->own_stream;
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
   CK(cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming));
   for (int s = 0; s < iqcp_ctx::kSide; ++s) {
-    CK(cudaStreamCreateWithFlags(&ctx->side[s], cudaStreamNonBlocking));
+    ctx->side[s] = ctx->streams.s[1 + s];
     CK(cudaEventCreateWithFlags(&ctx->join_ev[s], cudaEventDisableTiming));
   }
   ctx->n_mol = nmol;
@@ -686,46 +711,33 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   ctx->mol_shell0.push_back(ctx->n_shells);
   ctx->packed = base;
   ctx->n_prims = (int)bex.size();
-  {
-    std::vector<int> bi;
-    bi.insert(bi.end(), bl.begin(), bl.end());
-    bi.insert(bi.end(), bnp.begin(), bnp.end());
-    bi.insert(bi.end(), bps.begin(), bps.end());
-    bi.insert(bi.end(), boff.begin(), boff.end());
-    bi.insert(bi.end(), bz.begin(), bz.end());
-    bi.insert(bi.end(), bat.begin(), bat.end());
-    std::vector<double> bd;
-    bd.insert(bd.end(), bc.begin(), bc.end());
-    bd.insert(bd.end(), bex.begin(), bex.end());
-    bd.insert(bd.end(), bco.begin(), bco.end());
-    bd.insert(bd.end(), bxyz.begin(), bxyz.end());
-    CK(cudaMalloc(&ctx->d_bint, sizeof(int) * bi.size()));
-    CK(cudaMalloc(&ctx->d_bdbl, sizeof(double) * bd.size()));
-    CK(cudaMemcpy(ctx->d_bint, bi.data(), sizeof(int) * bi.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_bdbl, bd.data(), sizeof(double) * bd.size(), cudaMemcpyHostToDevice));
-  }
-  CK(cudaMalloc(&ctx->d_mol_base, sizeof(long long) * (nmol + 1)));
-  CK(cudaMalloc(&ctx->d_mol_n, sizeof(int) * nmol));
-  CK(cudaMalloc(&ctx->d_mol_bf0, sizeof(int) * nmol));
-  CK(cudaMemcpy(ctx->d_mol_base, ctx->mol_base.data(), sizeof(long long) * (nmol + 1), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->d_mol_n, ctx->mol_nbf.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->d_mol_bf0, ctx->mol_bf0.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&ctx->d_mol_atom0, sizeof(int) * (nmol + 1)));
-  CK(cudaMemcpy(ctx->d_mol_atom0, ctx->mol_atom0.data(), sizeof(int) * (nmol + 1), cudaMemcpyHostToDevice));
-  ctx->pack = Packing{ctx->d_mol_base, ctx->d_mol_n, ctx->d_mol_bf0, nmol, ctx->packed};
-
+  std::vector<int> bi;
+  bi.insert(bi.end(), bl.begin(), bl.end());
+  bi.insert(bi.end(), bnp.begin(), bnp.end());
+  bi.insert(bi.end(), bps.begin(), bps.end());
+  bi.insert(bi.end(), boff.begin(), boff.end());
+  bi.insert(bi.end(), bz.begin(), bz.end());
+  bi.insert(bi.end(), bat.begin(), bat.end());
+  std::vector<double> bd;
+  bd.insert(bd.end(), bc.begin(), bc.end());
+  bd.insert(bd.end(), bex.begin(), bex.end());
+  bd.insert(bd.end(), bco.begin(), bco.end());
+  bd.insert(bd.end(), bxyz.begin(), bxyz.end());
   if (pps.empty()) pps.push_back(PrimPair());
   const int npairs = (int)ctx->pairs.size();
-  CK(cudaMalloc(&ctx->d_pairs, sizeof(ShellPair) * npairs));
-  CK(cudaMalloc(&ctx->d_pp, sizeof(PrimPair) * pps.size()));
-  CK(cudaMemcpy(ctx->d_pairs, ctx->pairs.data(), sizeof(ShellPair) * npairs, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ctx->d_pp, pps.data(), sizeof(PrimPair) * pps.size(), cudaMemcpyHostToDevice));
-
+  // mixed form: per molecule the shell-block density bounds
+  std::vector<long long> dbase(nmol + 1, 0);
+  std::vector<int> ns(nmol);
+  for (int m = 0; m < nmol; ++m) {
+    ns[m] = ctx->mol_shell0[m + 1] - ctx->mol_shell0[m];
+    dbase[m + 1] = dbase[m] + (long long)ns[m] * ns[m];
+  }
+  ctx->dmax_total = dbase[nmol];
   // class-sorted pair lists of the one-electron launches; the Schwarz bounds on
   // the device take them too, one launch per class and run of molecules
+  std::vector<int> list;
+  list.reserve(npairs);
   {
-    std::vector<int> list;
-    list.reserve(npairs);
     int p0 = 0;
     for (int m = 0; m < nmol;) {
       iqcp_ctx::OneEChunk ch{};
@@ -747,79 +759,42 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
       ctx->onee.push_back(ch);
       m = m1;
     }
-    CK(cudaMalloc(&ctx->d_cls_list, sizeof(int) * npairs));
-    CK(cudaMemcpy(ctx->d_cls_list, list.data(), sizeof(int) * npairs, cudaMemcpyHostToDevice));
-    for (const auto& ch : ctx->onee)
-      for (int c = 0; c < kNumPairClasses; ++c)
-        if (ch.first[c + 1] > ch.first[c])
-          CK(launch_schwarz(c, ctx->d_pairs, ctx->d_pp, ctx->d_cls_list + ch.list0 + ch.first[c],
-                            ch.first[c + 1] - ch.first[c], kthr, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaMemcpy(ctx->pairs.data(), ctx->d_pairs, sizeof(ShellPair) * npairs, cudaMemcpyDeviceToHost));
   }
-  std::vector<int> ket_list;
-  std::vector<int2> place;
-  std::vector<QuartetTask> tasks;
-  long long prim_doubles = 0;
-  {
-    const int rc = build_tasks(ctx, ket_list, place, &prim_doubles, tasks);
-    if (rc) return rc;
-  }
-  if (ket_list.empty()) ket_list.push_back(0);
-  if (tasks.empty()) tasks.push_back(QuartetTask());
-  ctx->n_tasks = (int)tasks.size();
-  CK(cudaMalloc(&ctx->d_mask, sizeof(unsigned) * tasks.size()));
-  CK(cudaMalloc(&ctx->d_ket_list, sizeof(int) * ket_list.size()));
-  CK(cudaMemcpy(ctx->d_ket_list, ket_list.data(), sizeof(int) * ket_list.size(), cudaMemcpyHostToDevice));
-  {
-    const int n = (int)place.size();
-    int2* d_place = nullptr;
-    int4 *i0 = nullptr, *i1 = nullptr;
-    double *geom = nullptr, *prim = nullptr;
-    CK(cudaMalloc(&d_place, sizeof(int2) * (n > 0 ? n : 1)));
-    CK(cudaMalloc(&i0, sizeof(int4) * (n > 0 ? n : 1)));
-    ctx->kets.i0 = i0;
-    CK(cudaMalloc(&i1, sizeof(int4) * (n > 0 ? n : 1)));
-    ctx->kets.i1 = i1;
-    CK(cudaMalloc(&geom, sizeof(double) * 7 * (n > 0 ? n : 1)));
-    ctx->kets.geom = geom;
-    CK(cudaMalloc(&prim, sizeof(double) * (prim_doubles > 0 ? prim_doubles : 1)));
-    ctx->kets.prim = prim;
-    ctx->kets.n = n;
-    CK(cudaMemcpy(d_place, place.data(), sizeof(int2) * n, cudaMemcpyHostToDevice));
-    CK(launch_ket_tables(ctx->d_pairs, ctx->d_pp, ctx->d_ket_list, d_place, n, i0, i1, geom, prim, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaFree(d_place));
-  }
-  CK(cudaMalloc(&ctx->d_tasks, sizeof(QuartetTask) * tasks.size()));
-  CK(cudaMemcpy(ctx->d_tasks, tasks.data(), sizeof(QuartetTask) * tasks.size(), cudaMemcpyHostToDevice));
-
   const size_t nn = (size_t)ctx->packed;
-  CK(cudaMalloc(&ctx->d_ang, sizeof(double) * ctx->nbf));
-  CK(cudaMemcpy(ctx->d_ang, ang.data(), sizeof(double) * ctx->nbf, cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&ctx->d_Ds, sizeof(double) * nn));
-  CK(cudaMalloc(&ctx->d_Jt, sizeof(double) * nn));
-  CK(cudaMalloc(&ctx->d_Kt, sizeof(double) * nn));
-  for (int i = 0; i < 4; ++i) CK(cudaMalloc(&ctx->d_io[i], sizeof(double) * nn));
-  CK(cudaMalloc(&ctx->d_grad, sizeof(double) * 3 * ctx->n_atoms));
-  {
-    std::vector<long long> dbase(nmol + 1, 0);
-    std::vector<int> ns(nmol);
-    for (int m = 0; m < nmol; ++m) {
-      ns[m] = ctx->mol_shell0[m + 1] - ctx->mol_shell0[m];
-      dbase[m + 1] = dbase[m] + (long long)ns[m] * ns[m];
-    }
-    ctx->dmax_total = dbase[nmol];
-    CK(cudaMalloc(&ctx->d_dmax, sizeof(double) * ctx->dmax_total));
-    CK(cudaMalloc(&ctx->d_dbase, sizeof(long long) * (nmol + 1)));
-    CK(cudaMalloc(&ctx->d_mol_shell0, sizeof(int) * nmol));
-    CK(cudaMalloc(&ctx->d_mol_ns, sizeof(int) * nmol));
-    CK(cudaMemcpy(ctx->d_dbase, dbase.data(), sizeof(long long) * (nmol + 1), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_mol_shell0, ctx->mol_shell0.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_mol_ns, ns.data(), sizeof(int) * nmol, cudaMemcpyHostToDevice));
-  }
-  CK(cudaMalloc(&ctx->d_counters, sizeof(int) * 4 * (ctx->ranges.size() + 1)));
-  CK(cudaMalloc(&ctx->d_fp32, sizeof(unsigned long long)));
+  DeviceBlock& blk = ctx->block[0];
+  blk.upload(&ctx->d_bint, bi.data(), bi.size());
+  blk.upload(&ctx->d_bdbl, bd.data(), bd.size());
+  blk.upload(&ctx->d_mol_base, ctx->mol_base.data(), nmol + 1);
+  blk.upload(&ctx->d_mol_n, ctx->mol_nbf.data(), nmol);
+  blk.upload(&ctx->d_mol_bf0, ctx->mol_bf0.data(), nmol);
+  blk.upload(&ctx->d_mol_atom0, ctx->mol_atom0.data(), nmol + 1);
+  blk.upload(&ctx->d_pairs, ctx->pairs.data(), npairs);
+  blk.upload(&ctx->d_pp, pps.data(), pps.size());
+  blk.upload(&ctx->d_cls_list, list.data(), npairs);
+  blk.upload(&ctx->d_ang, ang.data(), ctx->nbf);
+  blk.upload(&ctx->d_dbase, dbase.data(), nmol + 1);
+  blk.upload(&ctx->d_mol_shell0, ctx->mol_shell0.data(), nmol);
+  blk.upload(&ctx->d_mol_ns, ns.data(), nmol);
+  blk.want(&ctx->d_Ds, nn);
+  blk.want(&ctx->d_Jt, nn);
+  blk.want(&ctx->d_Kt, nn);
+  for (int i = 0; i < 4; ++i) blk.want(&ctx->d_io[i], nn);
+  blk.want(&ctx->d_grad, 3 * (size_t)ctx->n_atoms);
+  blk.want(&ctx->d_dmax, ctx->dmax_total);
+  blk.want(&ctx->d_fp32, 1);
+  CK(blk.alloc(ctx->device, ctx->stream));
+  ctx->pack = Packing{ctx->d_mol_base, ctx->d_mol_n, ctx->d_mol_bf0, nmol, ctx->packed};
+  for (const auto& ch : ctx->onee)
+    for (int c = 0; c < kNumPairClasses; ++c)
+      if (ch.first[c + 1] > ch.first[c])
+        CK(launch_schwarz(c, ctx->d_pairs, ctx->d_pp, ctx->d_cls_list + ch.list0 + ch.first[c],
+                          ch.first[c + 1] - ch.first[c], kthr, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->pairs.data(), ctx->d_pairs, sizeof(ShellPair) * npairs, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  const int rc = build_tasks(ctx);
+  if (rc) return rc;
+  // other streams may use the arrays once the call has returned
+  CK(cudaStreamSynchronize(ctx->stream));
   return IQCP_OK;
 }
 
@@ -845,47 +820,21 @@ int iqcp_batch_layout(const iqcp_ctx* ctx, long long* mat_offset, int* nbf, int*
 void iqcp_destroy(iqcp_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
-  if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  cudaFree(ctx->d_pairs);
-  cudaFree(ctx->d_pp);
-  cudaFree(ctx->d_ket_list);
-  cudaFree(const_cast<int4*>(ctx->kets.i0));
-  cudaFree(const_cast<int4*>(ctx->kets.i1));
-  cudaFree(const_cast<double*>(ctx->kets.geom));
-  cudaFree(const_cast<double*>(ctx->kets.prim));
-  cudaFree(ctx->d_tasks);
-  cudaFree(ctx->d_ang);
-  cudaFree(ctx->d_Ds);
-  cudaFree(ctx->d_Jt);
-  cudaFree(ctx->d_Kt);
-  for (int i = 0; i < 4; ++i) cudaFree(ctx->d_io[i]);
-  cudaFree(ctx->d_grad);
-  cudaFree(ctx->d_bint);
-  cudaFree(ctx->d_bdbl);
-  cudaFree(ctx->d_dmax);
-  cudaFree(ctx->d_dbase);
-  cudaFree(ctx->d_mol_shell0);
-  cudaFree(ctx->d_mol_ns);
-  cudaFree(ctx->d_mask);
-  cudaFree(ctx->d_mol_base);
-  cudaFree(ctx->d_mol_n);
-  cudaFree(ctx->d_mol_bf0);
-  cudaFree(ctx->d_mol_atom0);
-  cudaFree(ctx->d_cls_list);
-  cudaFree(ctx->d_counters);
-  cudaFree(ctx->d_fp32);
+  // calls that only enqueue may have left work on any stream the context was
+  // given: the device is idle before memory and streams are handed on
+  cudaDeviceSynchronize();
+  for (DeviceBlock& b : ctx->block) b.free(ctx->own_stream);
   cudaFree(ctx->d_multi);
   cudaFree(ctx->d_multi_io);
   cudaFree(ctx->d_cart_info);
   cudaFree(ctx->d_sph_info);
+  for (cudaEvent_t e : ctx->pev) cudaEventDestroy(e);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
-  for (int s = 0; s < iqcp_ctx::kSide; ++s) {
+  for (int s = 0; s < iqcp_ctx::kSide; ++s)
     if (ctx->join_ev[s]) cudaEventDestroy(ctx->join_ev[s]);
-    if (ctx->side[s]) cudaStreamDestroy(ctx->side[s]);
-  }
-  if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+  streams_give(ctx->device, ctx->streams);
   delete ctx;
 }
 

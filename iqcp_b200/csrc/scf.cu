@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "../../include/iqcp.h"
+#include "device_pool.h"
 #include "internal.h"
 
 namespace iqcp {
@@ -433,20 +434,6 @@ __global__ void identity_error_kernel(const long long* __restrict__ base, const 
 namespace iqcp {
 namespace {
 
-struct ScfBuffers {
-  std::vector<void*> owned;
-  ~ScfBuffers() {
-    for (void* p : owned) cudaFree(p);
-  }
-  template <typename T>
-  cudaError_t get(T** p, long long n) {
-    *p = nullptr;
-    const cudaError_t e = cudaMalloc(p, sizeof(T) * (size_t)std::max(n, 1LL));
-    if (e == cudaSuccess) owned.push_back(*p);
-    return e;
-  }
-};
-
 struct ScfRun {
   iqcp_ctx* ctx = nullptr;
   cudaStream_t st = nullptr;
@@ -582,8 +569,9 @@ int iqcp_batch_scf(iqcp_ctx* ctx, const iqcp_scf_options* opts_in, const double*
   int rc = cudaSetDevice(ctx_device(ctx)) == cudaSuccess ? IQCP_OK : IQCP_ERR_CUDA;
   if (rc) return ctx_fail(ctx, rc, "cudaSetDevice");
   const cudaStream_t caller = ctx_stream(ctx);
-  ScfBuffers buf;
+  DeviceBlock buf;
   ScfRun r;
+  StreamSet set;
   cudaStream_t own = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -604,22 +592,26 @@ int iqcp_batch_scf(iqcp_ctx* ctx, const iqcp_scf_options* opts_in, const double*
   r.nm = pk.n;
   // work on a private stream: capture needs one, and the caller's may be the legacy default stream
   SCF_CK(cudaStreamSynchronize(caller));
-  SCF_CK(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+  SCF_CK(streams_take(ctx_device(ctx), &set));
+  own = set.s[0];
   r.st = own;
   iqcp_set_stream(ctx, own);
   for (double** p : {&r.S, &r.H, &r.X, &r.D, &r.F, &r.Fx, &r.P, &r.P2, &r.P3, &r.T1, &r.T2, &r.Dn})
-    SCF_CK(buf.get(p, r.total));
-  SCF_CK(buf.get(&r.Fbuf, r.total * r.K));
-  SCF_CK(buf.get(&r.Ebuf, r.total * r.K));
-  SCF_CK(buf.get(&r.Bm, (long long)nmol * r.K * r.K));
-  SCF_CK(buf.get(&r.coef, (long long)nmol * r.K));
-  for (double** p : {&r.enuc, &r.E, &r.dE, &r.dD, &r.err, &r.scale}) SCF_CK(buf.get(p, nmol));
-  SCF_CK(buf.get(&r.tr, 2LL * nmol));
-  SCF_CK(buf.get(&r.nocc, nmol));
-  SCF_CK(buf.get(&r.slot, 1));
-  SCF_CK(buf.get(&r.count, 1));
+    buf.want(p, r.total);
+  buf.want(&r.Fbuf, r.total * r.K);
+  buf.want(&r.Ebuf, r.total * r.K);
+  buf.want(&r.Bm, (size_t)nmol * r.K * r.K);
+  buf.want(&r.coef, (size_t)nmol * r.K);
+  for (double** p : {&r.enuc, &r.E, &r.dE, &r.dD, &r.err, &r.scale}) buf.want(p, nmol);
+  buf.want(&r.tr, 2 * (size_t)nmol);
+  buf.want(&r.nocc, nmol);
+  buf.want(&r.slot, 1);
+  buf.want(&r.count, 1);
   int* d_active;
-  SCF_CK(buf.get(&d_active, nmol));
+  double* d_grad;
+  buf.want(&d_active, nmol);
+  buf.want(&d_grad, grad ? 3 * (size_t)a0[nmol] : 0);
+  SCF_CK(buf.alloc(ctx_device(ctx), own));
   SCF_CK(cudaMemsetAsync(r.Ebuf, 0, sizeof(double) * r.total * r.K, own));
   SCF_CK(cudaMemsetAsync(r.Fbuf, 0, sizeof(double) * r.total * r.K, own));
   SCF_CK(cudaMemsetAsync(r.Bm, 0, sizeof(double) * nmol * r.K * r.K, own));
@@ -727,9 +719,8 @@ int iqcp_batch_scf(iqcp_ctx* ctx, const iqcp_scf_options* opts_in, const double*
   if (D_out) SCF_CK(cudaMemcpyAsync(D_out, r.D, sizeof(double) * r.total, cudaMemcpyDeviceToHost, own));
   if (grad) {
     // W = 1/2 D F D at the final density, then the one- and two-electron parts
-    double* g = nullptr;
+    double* g = d_grad;
     const int natoms = a0[nmol];
-    SCF_CK(buf.get(&g, 3LL * natoms));
     rc = iqcp_fock_device(ctx, r.H, r.D, 1.0, r.F);
     if (rc) goto done;
     SCF_CK(r.gemm(false, false, r.D, r.F, r.T1, 1.0, 0.0));
@@ -750,7 +741,9 @@ done:
   if (graph) cudaGraphDestroy(graph);
   if (own) cudaStreamSynchronize(own);
   iqcp_set_stream(ctx, caller);
-  if (own) cudaStreamDestroy(own);
+  buf.free(own);
+  if (own) cudaStreamSynchronize(own);
+  streams_give(ctx_device(ctx), set);
   return rc;
 }
 
