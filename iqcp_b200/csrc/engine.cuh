@@ -34,19 +34,14 @@ __host__ __device__ constexpr int class_lb(int c) { return c - class_la(c) * (cl
 // warp wins, 1.33 against 1.60 ms (J/K) and 3.33 against 8.2 (gradient).
 constexpr int kMaxThreadComp = 108;
 constexpr int kMaxThreadComp32 = 324;      // the same for the FP32 share of a mixed call
-constexpr int kMaxGroupGradComp = 108;     // gradient over (primitive quartet, root) items (eri_group.cuh)
 
 __host__ __device__ constexpr int class_comps(int X, int Y) {
   return ncart(class_la(X)) * ncart(class_lb(X)) * ncart(class_la(Y)) * ncart(class_lb(Y));
 }
-// The variant that a requested mode runs (kind 0 J/K, 1 gradient): 1 a warp per
-// quartet, 0 a lane group per quartet, 3 (gradient) lanes over (primitive
-// quartet, root) items.
-__host__ __device__ constexpr int kernel_variant(int kind, int X, int Y, int mode, bool f32) {
-  const int n = class_comps(X, Y);
-  if (mode == 1 || n > (f32 ? kMaxThreadComp32 : kMaxThreadComp)) return 1;
-  if (kind == 1 && n <= kMaxGroupGradComp && (mode == 3 || (f32 && mode == 2))) return 3;
-  return 0;
+// The variant that a requested mode runs: 1 a warp per quartet, 0 a lane group per
+// quartet (also for modes 2 and 3, which had kernels of their own)
+__host__ __device__ constexpr int kernel_variant(int X, int Y, int mode, bool f32) {
+  return mode == 1 || class_comps(X, Y) > (f32 ? kMaxThreadComp32 : kMaxThreadComp) ? 1 : 0;
 }
 // Variant before autotuning.  With fewer quartets than one wave of thread-kernel
 // lanes (148 SMs x 8 warps at 255 registers) the largest blocks leave most of the
@@ -219,7 +214,7 @@ struct GradArgs {
   double* grad;      // natoms x 3
   double prim_thr;
   double schwarz_thr;
-  int mode;          // kernel variant: 0 group of lanes per quartet, 1 warp-cooperative, 2 / 3 see eri_launch.cuh
+  int mode;          // kernel variant: 1 warp-cooperative, else a group of lanes per quartet
   int natoms;        // gradient rows; accumulated per block in shared memory when gsmem
   int gsmem;
   Mixed mx;

@@ -4,8 +4,8 @@
 #pragma once
 #include <atomic>
 
-#include "eri_group.cuh"
 #include "eri_md.cuh"
+#include "eri_team.cuh"
 
 namespace iqcp {
 
@@ -96,12 +96,13 @@ inline int persistent_blocks(int per_sm, int sms, int ntasks, int threads) {
 // Team kernels walk a task's kets in one warp, one after the other.  A class
 // with fewer tasks than twice the resident warps ((dd|dd) on a 40-atom
 // molecule: ~700 tasks for ~1300 warps) would leave SMs idle and end on its
-// longest task, so its tasks are split into 2, 4 or 8 slices of kets, each
-// a work item of its own.
+// longest task, so its tasks are split into up to 32 slices of kets, each
+// a work item of its own; a (dd|dd) quartet alone is 30 us of one warp, so with
+// slices of four kets a 12-atom gradient waited 0.12 ms for 190 quartets.
 inline int team_ket_split(int per_sm, int sms, int ntasks, int threads) {
   const long long warps = (long long)per_sm * sms * (threads / 32);
   int s = 1;
-  while (s < 8 && (long long)ntasks * s < 2 * warps) s *= 2;
+  while (s < 32 && (long long)ntasks * s < 2 * warps) s *= 2;
   return s;
 }
 
@@ -124,7 +125,7 @@ cudaError_t launch_jk_variant(const JKArgs& a, cudaStream_t st) {
   constexpr bool F32 = sizeof(R) == 4;
   const size_t tb = sizeof(double) * rys_tab_doubles<C::NR>();
   constexpr int X = pair_class(LA, LB), Y = pair_class(LC, LD);
-  if (kernel_variant(0, X, Y, a.mode, F32) == 1) {
+  if (kernel_variant(X, Y, a.mode, F32) == 1) {
     const size_t bytes = sizeof(double) * 4 * TeamJK<LA, LB, LC, LD>::PER_WARP + tb;
     JKArgs b = a;
     if (a.K) IQCP_LAUNCH_TEAM((jk_team_kernel<R, LA, LB, LC, LD, true>), 128, bytes, b, st);
@@ -145,8 +146,7 @@ cudaError_t launch_jk_class(const JKArgs& a, cudaStream_t st) {
 // Gradient variants (kernel_variant): 1 warp-cooperative; 0 a group of lanes per
 // quartet, by Hermite expansions for FP64 classes with an ss or ps ket, by Rys
 // quadrature with the weights in shared memory for the other FP64 classes and
-// in registers for the FP32 share; 3 the grouped kernel of eri_group.cuh (32 lanes
-// per quartet, 8 for the FP32 share).
+// in registers for the FP32 share.
 template <int LA, int LB, int LC>
 cudaError_t launch_grad_md(const GradArgs& args, cudaStream_t st) {
   using G = GradMD<LA, LB, LC>;
@@ -167,14 +167,12 @@ cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
   constexpr bool MD = !F32 && LC + LD <= 1;
   constexpr bool THREAD = !MD && C::NCOMP <= (F32 ? kMaxThreadComp32 : kMaxThreadComp);
   using TG = TeamGrad2<LA, LB, LC, LD>;
-  const int variant = kernel_variant(1, X, Y, args.mode, F32);
+  const int variant = kernel_variant(X, Y, args.mode, F32);
   if constexpr (MD)
     if (variant == 0) return launch_grad_md<LA, LB, LC>(args, st);
   // the team variant reads the Rys coefficients through L1 (no staged table)
   size_t fixed = sizeof(double) * rys_tab_doubles<NRG>();
   if (variant == 1) fixed = sizeof(double) * TG::WPB * TG::PER_WARP;
-  else if (variant == 3)
-    fixed += sizeof(double) * (F32 ? GroupGrad<R, LA, LB, LC, LD, 8>::WDOUBLES : GroupGrad<R, LA, LB, LC, LD, 32>::WDOUBLES);
   else if (!F32)
     fixed = sizeof(double) * (grad_stages_rys<LA, LB, LC, LD, true>() ? rys_tab_doubles<NRG>() : 0) +
             sizeof(R) * grad_wsh_doubles<LA, LB, LC, LD>();
@@ -185,11 +183,6 @@ cudaError_t launch_grad_variant(const GradArgs& args, cudaStream_t st) {
   const size_t bytes = fixed + gacc;
   if (variant == 1) {
     IQCP_LAUNCH_TEAM((grad_team2_kernel<R, LA, LB, LC, LD>), 32 * TG::WPB, bytes, a, st);
-  } else if (variant == 3) {
-    if constexpr (C::NCOMP <= kMaxGroupGradComp) {
-      if (F32) IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 8>), bytes, a, st);
-      else IQCP_LAUNCH((grad_group_kernel<R, LA, LB, LC, LD, 32>), bytes, a, st);
-    }
   } else if constexpr (THREAD) {
     IQCP_LAUNCH((grad_kernel<R, LA, LB, LC, LD, !F32>), bytes, a, st);
   }

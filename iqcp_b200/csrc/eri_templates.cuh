@@ -352,7 +352,7 @@ __device__ __forceinline__ double group_sum(double v, int lg) {
 // lane of each group digests the block.
 // Resident blocks asked of the compiler: up to L = 2 what the registers of a
 // spill-free build allow (left alone it takes 166 registers for (ps|ps), three
-// blocks, where 128 cost 12 bytes of spill).
+// blocks, where 128 do without a spill).
 __host__ __device__ constexpr int jk_min_blocks(int L) { return L == 0 ? 6 : (L == 1 ? 5 : (L == 2 ? 4 : 1)); }
 
 template <typename R, int LA, int LB, int LC, int LD, bool DO_K>

@@ -1419,9 +1419,7 @@ int iqcp_autotune(iqcp_ctx* ctx, const double* dD, int reps) {
                                      : r.count;
     float best = 1e30f;
     for (int mode = 0; mode < kNumModes; ++mode) {
-      // only modes that name their own kernel
-      if (kernel_variant(kind, r.X, r.Y, mode, pass == 2) != mode && !(pass == 2 && mode == 2)) continue;
-      if (pass == 2 && (mode == 3 || (kind == 0 && mode == 2))) continue;  // the FP32 share's lane groups are mode 2
+      if (kernel_variant(r.X, r.Y, mode, pass == 2) != mode) continue;  // runs another mode's kernel
       float tmin = 1e30f;
       for (int rep = 0; rep < reps + 1; ++rep) {  // first run warms caches and sets attributes
         CK(cudaMemsetAsync(ctx->d_Jt, 0, bytes, ctx->stream));

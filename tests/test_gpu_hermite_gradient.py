@@ -1,6 +1,6 @@
 """The Hermite gradient kernel (ss and ps kets) at the sizes where it changes:
 T = 0 and both sides of the Boys table's end, more bra primitives than a warp
-stages at a time, and the Rys kernels (mode 3, lane groups over roots) on the
+stages at a time, and the Rys kernels (mode 1, a warp per quartet) on the
 same quartets.
 
 Tolerance: every term is formed to a few ulp and the sums cancel by translation
@@ -46,7 +46,7 @@ def test_against_oracle_and_rys(oracle_mod, name):
         oracle_mod.set_root_precision(False)
     out = []
     with FockEngine(b) as eng:
-        for mode in (0, 3):
+        for mode in (0, 1):
             eng.set_kernel_mode("grad", mode=mode)
             out.append(eng.eri_gradient(D, 0.7))
     scale = max(1.0, np.abs(go).max())
