@@ -80,7 +80,7 @@ __global__ void rys_batch_kernel(int nr, int n, const double* __restrict__ T, do
 cudaError_t launch_schwarz(int X, ShellPair* pairs, const PrimPair* pp, const int* list, int n,
                            double thr, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  const int blocks = (n + 127) / 128;
+  const int blocks = (n + 3) / 4;  // a warp per pair
   switch (X) {
     case 0: schwarz_kernel<0, 0><<<blocks, 128, 0, st>>>(pairs, pp, list, n, thr); break;
     case 1: schwarz_kernel<1, 0><<<blocks, 128, 0, st>>>(pairs, pp, list, n, thr); break;

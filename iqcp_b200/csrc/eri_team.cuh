@@ -52,17 +52,18 @@ struct TeamJK {
 // quartets, accumulating this lane's components into acc (FP64).  R is the
 // quadrature type: double, or float for the mixed form (roots, weights and
 // recurrence coefficients are formed in FP64 and rounded once).
-template <typename R, int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void team_prim_loop(const JKArgs& args, const ShellPair& bp, const ShellPair& kp,
-                                               const double* AB, const double* CD, const int* offs, double* acc,
-                                               R* tab, int lane, const double* rtab) {
+// LDG: the Rys table through L1 instead of staged at rtab.
+template <typename R, int LA, int LB, int LC, int LD, bool LDG = false>
+__device__ __forceinline__ void team_prim_loop(const PrimPair* __restrict__ pp, double prim_thr, const ShellPair& bp,
+                                               const ShellPair& kp, const double* AB, const double* CD,
+                                               const int* offs, double* acc, R* tab, int lane, const double* rtab) {
   using C = Cls<LA, LB, LC, LD>;
   constexpr int NR = C::NR, TSZ = TeamJK<LA, LB, LC, LD>::TSP, CPL = TeamJK<LA, LB, LC, LD>::CPL;
   for (int i = 0; i < bp.np; ++i) {
-    const PrimPair pb = load_pp(args.pp + bp.pstart + i);
+    const PrimPair pb = load_pp(pp + bp.pstart + i);
     for (int j = 0; j < kp.np; ++j) {
-      const PrimPair pk = load_pp(args.pp + kp.pstart + j);
-      if (pb.K * pk.K < args.prim_thr) continue;
+      const PrimPair pk = load_pp(pp + kp.pstart + j);
+      if (pb.K * pk.K < prim_thr) continue;
       if (lane < 3 * NR) {
         const int r = lane / 3, ax = lane - 3 * r;
         const double p = pb.p, q = pk.p, s = p + q;
@@ -71,7 +72,7 @@ __device__ __forceinline__ void team_prim_loop(const JKArgs& args, const ShellPa
         const double rho = p * q * inv_s;
         const double T = rho * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
         double t2, wr;
-        rys_rule_one<NR>(T, r, rtab, &t2, &wr);
+        rys_rule_one<NR, LDG>(T, r, rtab, &t2, &wr);
         const double b00 = 0.5 * t2 * inv_s, h = 0.5 - 0.5 * t2;
         const double b10 = fma(h, pb.inv_p, b00), b01 = fma(h, pk.inv_p, b00);
         const double pa = pick3(ax, pb.P[0] - bp.A[0], pb.P[1] - bp.A[1], pb.P[2] - bp.A[2]);
@@ -100,6 +101,26 @@ __device__ __forceinline__ void team_prim_loop(const JKArgs& args, const ShellPa
   }
 }
 
+// Packed table offsets of a lane's components (lane + 32 m): x | y << 8 | z << 16
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void team_offsets(int lane, int* offs) {
+  using C = Cls<LA, LB, LC, LD>;
+  constexpr int TSZ = TeamJK<LA, LB, LC, LD>::TSP, CPL = TeamJK<LA, LB, LC, LD>::CPL;
+#pragma unroll
+  for (int m = 0; m < CPL; ++m) {
+    int comp = lane + 32 * m;
+    if (comp >= C::NCOMP) comp = 0;
+    const int d = comp % C::ND, c = (comp / C::ND) % C::NC, b = (comp / (C::ND * C::NC)) % C::NB,
+              a = comp / (C::ND * C::NC * C::NB);
+    int o = 0;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax)
+      o |= (ax * TSZ + C::tidx(cart_pow(LA, a, ax), cart_pow(LB, b, ax), cart_pow(LC, c, ax),
+                               cart_pow(LD, d, ax))) << (8 * ax);
+    offs[m] = o;
+  }
+}
+
 template <typename R, int LA, int LB, int LC, int LD, bool DO_K>
 __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_kernel(JKArgs args) {
   using C = Cls<LA, LB, LC, LD>;
@@ -119,21 +140,8 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
   double* Dbc = Dad + C::NA * C::ND;
   double* Dac = Dbc + C::NB * C::NC;
 
-  // packed table offsets of this lane's components: x | y << 8 | z << 16
   int offs[CPL];
-#pragma unroll
-  for (int m = 0; m < CPL; ++m) {
-    int comp = lane + 32 * m;
-    if (comp >= C::NCOMP) comp = 0;
-    const int d = comp % C::ND, c = (comp / C::ND) % C::NC, b = (comp / (C::ND * C::NC)) % C::NB,
-              a = comp / (C::ND * C::NC * C::NB);
-    int o = 0;
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax)
-      o |= (ax * TSZ + C::tidx(cart_pow(LA, a, ax), cart_pow(LB, b, ax), cart_pow(LC, c, ax),
-                               cart_pow(LD, d, ax))) << (8 * ax);
-    offs[m] = o;
-  }
+  team_offsets<LA, LB, LC, LD>(lane, offs);
 
   const int S = args.ket_split;  // work items per task (slices of its kets)
   for (int item = next_task(args.next_task, lane); item < args.ntasks * S; item = next_task(args.next_task, lane)) {
@@ -162,7 +170,8 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
     double acc[CPL];
 #pragma unroll
     for (int m = 0; m < CPL; ++m) acc[m] = 0.0;
-    team_prim_loop<R, LA, LB, LC, LD>(args, bp, kp, AB, CD, offs, acc, reinterpret_cast<R*>(work), lane, rtab);
+    team_prim_loop<R, LA, LB, LC, LD>(args.pp, args.prim_thr, bp, kp, AB, CD, offs, acc,
+                                      reinterpret_cast<R*>(work), lane, rtab);
     ++nf32;
     // ---- digestion ----
     double f = 1.0;
@@ -263,6 +272,55 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
   }
   if (sizeof(R) == 4 && lane == 0 && args.mx.fp32_count && nf32) atomicAdd(args.mx.fp32_count, (unsigned long long)nf32);
   }  // task loop
+}
+
+// ---------------------------------------------------------------------------
+// Schwarz bounds: Q = sqrt(max |(ab|ab)|) over the block with the angular
+// factors applied (compute_schwarz_bounds, eri/mod.rs:1263-1290).  One warp per
+// pair: up to 81 components its lanes split the primitive quartets, above they
+// split the components as in the team kernel.  A thread per pair walked 36 x 36
+// primitive quartets of a contracted ss pair alone, and a dd pair with its 1296
+// components in local memory; a context of three atoms waited for it like one
+// of forty.
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const PrimPair* pp, const int* list, int n,
+                                                      double thr) {
+  using C = Cls<LA, LB, LA, LB>;
+  using TM = TeamJK<LA, LB, LA, LB>;
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= n) return;  // whole warps
+  const int pid = list[w];
+  const ShellPair bp = pairs[pid];
+  double mx = 0.0;
+  if constexpr (C::NCOMP <= 81) {
+    double acc[C::NCOMP];
+    quartet<double, LA, LB, LA, LB>(bp, bp, pp, PairPrims{pp + bp.pstart}, thr, acc, lane, 32);
+#pragma unroll
+    for (int i = 0; i < C::NCOMP; ++i) {
+      const int d = i % C::ND, c = (i / C::ND) % C::NC, b = (i / (C::ND * C::NC)) % C::NB, a = i / (C::ND * C::NC * C::NB);
+      mx = fmax(mx, fabs(warp_sum(acc[i]) * ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LA, c) * ang_factor(LB, d)));
+    }
+  } else {
+    __shared__ double tabs[4][TM::TAB];
+    const double AB[3] = {bp.A[0] - bp.B[0], bp.A[1] - bp.B[1], bp.A[2] - bp.B[2]};
+    int offs[TM::CPL];
+    team_offsets<LA, LB, LA, LB>(lane, offs);
+    double acc[TM::CPL];
+#pragma unroll
+    for (int m = 0; m < TM::CPL; ++m) acc[m] = 0.0;
+    team_prim_loop<double, LA, LB, LA, LB, true>(pp, thr, bp, bp, AB, AB, offs, acc, tabs[threadIdx.x >> 5], lane, nullptr);
+#pragma unroll
+    for (int m = 0; m < TM::CPL; ++m) {
+      const int i = lane + 32 * m;
+      if (i < C::NCOMP) {
+        const int d = i % C::ND, c = (i / C::ND) % C::NC, b = (i / (C::ND * C::NC)) % C::NB, a = i / (C::ND * C::NC * C::NB);
+        mx = fmax(mx, fabs(acc[m] * ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LA, c) * ang_factor(LB, d)));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (lane == 0) pairs[pid].Q = sqrt(mx);
 }
 
 // ---------------------------------------------------------------------------

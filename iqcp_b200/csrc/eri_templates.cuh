@@ -501,35 +501,6 @@ __global__ void __launch_bounds__(128, jk_min_blocks(LA + LB + LC + LD)) jk_kern
 }
 
 // ---------------------------------------------------------------------------
-// Schwarz bounds: Q = sqrt(max |(ab|ab)|) over the block with the angular
-// factors applied (compute_schwarz_bounds, eri/mod.rs:1263-1290).
-template <int LA, int LB>
-__global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const PrimPair* pp,
-                                                      const int* list, int n, double thr) {
-  using C = Cls<LA, LB, LA, LB>;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int pid = list[t];
-  const ShellPair bp = pairs[pid];
-  double acc[C::NCOMP];
-  quartet<double, LA, LB, LA, LB>(bp, bp, pp, PairPrims{pp + bp.pstart}, thr, acc);
-  double mx = 0.0;
-#pragma unroll
-  for (int a = 0; a < C::NA; ++a)
-#pragma unroll
-    for (int b = 0; b < C::NB; ++b)
-#pragma unroll
-      for (int c = 0; c < C::NC; ++c)
-#pragma unroll
-        for (int d = 0; d < C::ND; ++d) {
-          const double v = acc[((a * C::NB + b) * C::NC + c) * C::ND + d] * ang_factor(LA, a) *
-                           ang_factor(LB, b) * ang_factor(LA, c) * ang_factor(LB, d);
-          mx = fmax(mx, fabs(v));
-        }
-  pairs[pid].Q = sqrt(mx);
-}
-
-// ---------------------------------------------------------------------------
 // 8-fold compressed ERI store (eri_compressed layout, eri/mod.rs:946-1070).
 __device__ __forceinline__ long long pair_index(long long i, long long j) {
   return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i;
