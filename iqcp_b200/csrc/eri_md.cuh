@@ -228,7 +228,13 @@ struct GradMD {
   static constexpr int WARP = HermiteBra<LA, LB>::WARP;
   // warps per block: four; six where the weights (110 KB for four warps of
   // (dd|ps)) leave no room for a second block
-  static constexpr int WPB = C::NCOMP > 60 ? 6 : 4, THREADS = 32 * WPB, MINB = C::NCOMP > 60 ? 1 : (L == 0 ? 4 : (L <= 2 ? 3 : 2));
+  static constexpr int WPB = C::NCOMP > 60 ? 6 : 4, THREADS = 32 * WPB;
+  // resident blocks asked of the compiler: these kernels wait on their own FP64
+  // chains, and warps pay more than the spills of up to 250 bytes that make room
+  // for them: 40 atoms in 6-31G*, (ss|ss) 4 -> 5 blocks and (ps|ss), (pp|ss), (ds|ss) 3 -> 4:
+  // 1.20 -> 1.01, 2.61 -> 2.11, 0.95 -> 0.86, 0.97 -> 0.81 ms; (ps|ps) stays at 3
+  // (1.44 against 1.49 ms)
+  static constexpr int MINB = C::NCOMP > 60 ? 1 : (L == 0 ? 5 : (LC == 1 && L == 2 ? 3 : (L <= 2 ? 4 : 2)));
   // shared memory (doubles) beside the gradient accumulator
   static constexpr int FIXED = TAB + WPB * WARP + THREADS * C::NCOMP;
 };
@@ -246,7 +252,9 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
   double* Est = smem + G::TAB + wib * G::WARP;
   double* Etab = Est + HB::CHUNK * HB::PER;
   double* Wsh = smem + G::TAB + G::WPB * G::WARP + threadIdx.x;  // weight of component c at Wsh[c * THREADS]
-  const volatile double* Wv = Wsh;  // kept in shared memory, not hoisted into registers
+  // blocks of more than nine components: read through a volatile view, so that
+  // the weights stay in shared memory instead of being hoisted into registers
+  const std::conditional_t<(C::NCOMP > 9), const volatile double*, const double*> Wv = Wsh;
   double* gacc = smem + G::FIXED;
   if (args.gsmem)
     for (int i = threadIdx.x; i < 3 * args.natoms; i += blockDim.x) gacc[i] = 0.0;
