@@ -367,6 +367,169 @@ __global__ void purify_update_kernel(const long long* __restrict__ base, const i
   }
 }
 
+// ---------------------------------------------------------------------------
+// Canonical purification, one step in one kernel, for molecules of up to
+// kStepMaxN functions.  A step is P2 = P P, P3 = P2 P, two traces and the element
+// update; as four kernels it cost 40 us at 100 functions, 64 times per SCF
+// iteration, most of it kernel starts and the latency of short k loops.  Here a
+// block takes kStepRows rows: it applies the previous step's update while it
+// brings the whole P into shared memory (up to 205 KB; every block does, from
+// L2), forms its rows of P2 and then of P3 from there, and leaves its share of the
+// traces for the next step, which adds the shares in a fixed order.  In- and
+// output triples (P, P2, P3) alternate, since other blocks still read the input.
+// A molecule whose P was idempotent to rounding (|Tr(P - P2)| < 1e-13) at two steps
+// running has nothing left to purify: its remaining steps return at once, and the
+// last triple of either parity gives the same projector.
+constexpr int kStepRows = 16, kStepMaxN = 160, kStepMaxBlocks = kStepMaxN / kStepRows;
+
+struct PurifyTriple {
+  double *P, *P2, *P3;
+};
+
+// Update coefficient of a step: < 0.5 and >= 0.5 are the two forms of the update
+__device__ __forceinline__ double purify_coefficient(double t1, double t2) { return fabs(t1) < 1e-13 ? 0.5 : t2 / t1; }
+__device__ __forceinline__ double purify_element(double c, double p, double p2, double p3) {
+  return c >= 0.5 ? ((1.0 + c) * p2 - p3) / fmax(c, 1e-30)
+                  : ((1.0 - 2.0 * c) * p + (1.0 + c) * p2 - p3) / fmax(1.0 - c, 1e-30);
+}
+// Traces of a step from its blocks' shares: part[(ring m) block], pairs
+__device__ __forceinline__ void purify_traces(const double* __restrict__ part, int m, int nblk, double* t1, double* t2) {
+  double a = 0.0, b = 0.0;
+  for (int k = 0; k < nblk; ++k) {
+    a += part[2 * (m * kStepMaxBlocks + k)];
+    b += part[2 * (m * kStepMaxBlocks + k) + 1];
+  }
+  *t1 = a;
+  *t2 = b;
+}
+
+// step: 0 takes in.P as it is.  prev, prev2: shares of the steps before (step >= 1, 2).
+template <int CT>
+__global__ void __launch_bounds__(128) purify_step_kernel(const long long* __restrict__ base, const int* __restrict__ nm,
+                                                          const int* __restrict__ active, int step, PurifyTriple in,
+                                                          PurifyTriple out, const double* __restrict__ prev,
+                                                          const double* __restrict__ prev2, double* __restrict__ part) {
+  const int m = blockIdx.y, n = nm[m], r0 = blockIdx.x * kStepRows;
+  if (r0 >= n || frozen(active, m)) return;
+  extern __shared__ double sm[];
+  double* Ps = sm;                   // n x n
+  double* Rs = sm + (size_t)n * n;   // kStepRows x n: this block's rows of P2
+  __shared__ double red[2][4];
+  const int nblk = (n + kStepRows - 1) / kStepRows, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double c = -1.0;
+  if (step > 0) {
+    double t1, t2;
+    purify_traces(prev, m, nblk, &t1, &t2);
+    if (step > 1) {
+      double u1, u2;
+      purify_traces(prev2, m, nblk, &u1, &u2);
+      if (fabs(t1) < 1e-13 && fabs(u1) < 1e-13) {  // the same in every block of the molecule
+        if (threadIdx.x == 0) part[2 * (m * kStepMaxBlocks + blockIdx.x)] = part[2 * (m * kStepMaxBlocks + blockIdx.x) + 1] = 0.0;
+        return;
+      }
+    }
+    c = purify_coefficient(t1, t2);
+  }
+  const long long o = base[m];
+  const int nn = n * n;
+  for (int e = threadIdx.x; e < nn; e += 128) {
+    const double p = in.P[o + e];
+    Ps[e] = step > 0 ? purify_element(c, p, in.P2[o + e], in.P3[o + e]) : p;
+  }
+  __syncthreads();
+  const int rows = n - r0 < kStepRows ? n - r0 : kStepRows, rw = 4 * w;  // a warp takes four rows
+  for (int e = threadIdx.x; e < rows * n; e += 128) out.P[o + (long long)r0 * n + e] = Ps[r0 * n + e];
+  double t1 = 0.0, t2 = 0.0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {  // P2 rows = P rows x P, then P3 rows = P2 rows x P
+    const double* A = pass == 0 ? Ps + r0 * n : Rs;
+    double acc[4][CT];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int u = 0; u < CT; ++u) acc[r][u] = 0.0;
+    if (rw < rows) {
+      // rows and columns past the end repeat the last one and are not stored
+      int ar[4], bc[CT];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) ar[r] = (rw + r < rows ? rw + r : rows - 1) * n;
+#pragma unroll
+      for (int u = 0; u < CT; ++u) bc[u] = lane + 32 * u < n ? lane + 32 * u : n - 1;
+#pragma unroll 2
+      for (int k = 0; k < n; ++k) {
+        double a[4], b[CT];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) a[r] = A[ar[r] + k];
+#pragma unroll
+        for (int u = 0; u < CT; ++u) b[u] = Ps[k * n + bc[u]];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int u = 0; u < CT; ++u) acc[r][u] = fma(a[r], b[u], acc[r][u]);
+      }
+    }
+    double* O = pass == 0 ? out.P2 : out.P3;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int u = 0; u < CT; ++u) {
+        const int row = rw + r, col = lane + 32 * u;
+        if (row < rows && col < n) {
+          if (pass == 0) Rs[row * n + col] = acc[r][u];
+          O[o + (long long)(r0 + row) * n + col] = acc[r][u];
+          if (col == r0 + row) {
+            if (pass == 0) {
+              t1 += Ps[col * n + col] - acc[r][u];
+              t2 += acc[r][u];
+            } else {
+              t2 -= acc[r][u];
+            }
+          }
+        }
+      }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    t1 += __shfl_xor_sync(0xffffffffu, t1, s);
+    t2 += __shfl_xor_sync(0xffffffffu, t2, s);
+  }
+  if (lane == 0) {
+    red[0][w] = t1;
+    red[1][w] = t2;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2)
+    part[2 * (m * kStepMaxBlocks + blockIdx.x) + threadIdx.x] =
+        red[threadIdx.x][0] + red[threadIdx.x][1] + red[threadIdx.x][2] + red[threadIdx.x][3];
+}
+
+// The last step's update: P = f(in) (grid: chunks x molecules)
+__global__ void purify_finish_kernel(const long long* __restrict__ base, const int* __restrict__ nm,
+                                     const int* __restrict__ active, PurifyTriple in, const double* __restrict__ part,
+                                     double* __restrict__ P) {
+  const int m = blockIdx.y, n = nm[m];
+  if (frozen(active, m)) return;
+  double t1, t2;
+  purify_traces(part, m, (n + kStepRows - 1) / kStepRows, &t1, &t2);
+  const double c = purify_coefficient(t1, t2);
+  const long long o = base[m], nn = (long long)n * n;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x)
+    P[o + e] = purify_element(c, in.P[o + e], in.P2[o + e], in.P3[o + e]);
+}
+
+template <int CT>
+cudaError_t launch_purify_step(size_t smem, dim3 grid, const long long* base, const int* nm, const int* active, int step,
+                               PurifyTriple in, PurifyTriple out, const double* prev, const double* prev2, double* part,
+                               cudaStream_t st) {
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(purify_step_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  purify_step_kernel<CT><<<grid, 128, smem, st>>>(base, nm, active, step, in, out, prev, prev2, part);
+  return cudaGetLastError();
+}
+
 // 3 I - X per molecule (grid: chunks x molecules)
 __global__ void three_minus_kernel(const long long* __restrict__ base, const int* __restrict__ nm,
                                    const double* __restrict__ X, double* __restrict__ out) {
@@ -442,7 +605,7 @@ struct ScfRun {
   const long long* base = nullptr;  // device, n_mol + 1
   const int* nm = nullptr;          // device, n_mol
   double *S, *H, *X, *D, *F, *Fx, *P, *P2, *P3, *T1, *T2, *Dn, *Fbuf, *Ebuf;
-  double *Bm, *coef, *enuc, *E, *dE, *dD, *err, *scale, *tr;
+  double *Bm, *coef, *enuc, *E, *dE, *dD, *err, *scale, *tr, *part;
   int *nocc, *slot, *count;
   int* active = nullptr;  // per molecule: 1 while iterating (null during set-up and the final gradient)
 
@@ -459,13 +622,38 @@ struct ScfRun {
     else gemm_packed_kernel<true, true><<<grid, 256, 0, st>>>(base, nm, active, A, B, C, alpha, beta);
     return cudaGetLastError();
   }
-  // Dout = 2 X P X^T with P the purified projector of Fp (Fp is left intact);
-  // iters purification steps (default purify_iters)
+  // The purification steps of a batch of small molecules; leaves the result in P
+  cudaError_t purify_small(double* spare, int iters) const {
+    const PurifyTriple t[2] = {{P, P2, P3}, {T1, Fx, spare}};
+    const size_t share = 2 * (size_t)nmol * kStepMaxBlocks;
+    const size_t smem = sizeof(double) * ((size_t)nmax * nmax + (size_t)kStepRows * nmax);
+    const dim3 grid((nmax + kStepRows - 1) / kStepRows, nmol);
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < iters && e == cudaSuccess; ++s) {
+      // step 0 updates nothing: it reads the start from t[0] as every even step
+      const PurifyTriple in = t[s & 1], out = t[(s + 1) & 1];
+      double* now = part + (s % 3) * share;
+      const double *p1 = part + ((s + 2) % 3) * share, *p2 = part + ((s + 1) % 3) * share;
+      switch ((nmax + 31) / 32) {
+        case 1: e = launch_purify_step<1>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
+        case 2: e = launch_purify_step<2>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
+        case 3: e = launch_purify_step<3>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
+        case 4: e = launch_purify_step<4>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
+        default: e = launch_purify_step<5>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
+      }
+    }
+    if (e != cudaSuccess) return e;
+    purify_finish_kernel<<<elem_grid(), 256, 0, st>>>(base, nm, active, t[iters & 1], part + ((iters + 2) % 3) * share, P);
+    return cudaGetLastError();
+  }
+  // Dout = 2 X P X^T with P the purified projector of Fp (which may be any matrix
+  // but P, P2, P3, T1 and Fx); iters purification steps (default purify_iters)
   cudaError_t purify_density(const double* Fp, double* Dout, int iters = 0) const {
     if (iters <= 0) iters = purify_iters;
     purify_start_kernel<<<nmol, 256, 0, st>>>(base, nm, active, nocc, Fp, P);
     cudaError_t e = cudaGetLastError();
-    for (int it = 0; it < iters && e == cudaSuccess; ++it) {
+    if (e == cudaSuccess && nmax <= kStepMaxN) e = purify_small(Dout, iters);
+    for (int it = 0; nmax > kStepMaxN && it < iters && e == cudaSuccess; ++it) {
       if ((e = gemm(false, false, P, P, P2, 1.0, 0.0)) != cudaSuccess) break;
       if ((e = gemm(false, false, P2, P, P3, 1.0, 0.0)) != cudaSuccess) break;
       purify_trace_kernel<<<nmol, 256, 0, st>>>(base, nm, active, P, P2, P3, tr);
@@ -604,6 +792,7 @@ int iqcp_batch_scf(iqcp_ctx* ctx, const iqcp_scf_options* opts_in, const double*
   buf.want(&r.coef, (size_t)nmol * r.K);
   for (double** p : {&r.enuc, &r.E, &r.dE, &r.dD, &r.err, &r.scale}) buf.want(p, nmol);
   buf.want(&r.tr, 2 * (size_t)nmol);
+  buf.want(&r.part, 3 * 2 * (size_t)nmol * kStepMaxBlocks);
   buf.want(&r.nocc, nmol);
   buf.want(&r.slot, 1);
   buf.want(&r.count, 1);
