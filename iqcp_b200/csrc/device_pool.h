@@ -24,12 +24,13 @@ constexpr unsigned long long kPoolKeep = 64ull << 20, kPoolMax = 16ull << 20;
 cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t stream);
 void pool_free(void* p, cudaStream_t stream);
 
-// Four non-blocking streams.  Returned sets are handed on to later contexts of
+// Eight non-blocking streams (a small molecule's class kernels are a block or two
+// each, and their launches the longer the more of them run at once).  Returned sets are handed on to later contexts of
 // the same device, at most kKeepStreams idle sets per device.  A set is returned
 // only when its streams are idle.
-constexpr int kSetStreams = 4, kKeepStreams = 8;
+constexpr int kSetStreams = 8, kKeepStreams = 8;
 struct StreamSet {
-  cudaStream_t s[kSetStreams] = {nullptr, nullptr, nullptr, nullptr};
+  cudaStream_t s[kSetStreams] = {};
 };
 cudaError_t streams_take(int device, StreamSet* set);
 void streams_give(int device, const StreamSet& set);

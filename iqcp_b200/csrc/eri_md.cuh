@@ -161,8 +161,9 @@ __device__ __forceinline__ void boys_stage(double* s) {
   double2* d = reinterpret_cast<double2*>(s);
   for (int i = threadIdx.x; i < N * W; i += blockDim.x) {
     const int k = i / W;
-    d[k * (W + 1) + (i - k * W)] = __ldg(g + i);  // rows padded to 6 pairs
+    copy16_async(d + k * (W + 1) + (i - k * W), g + i);  // rows padded to 6 pairs
   }
+  copy_async_wait();
 }
 
 template <int M>
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
     const QuartetTask task = args.tasks[warp];
     const ShellPair bp = args.pairs[task.bra];
     const int lg = task.lg, NG = 32 >> lg, grp = lane >> lg, sub = lane & ((1 << lg) - 1);
+    if (C::NCOMP <= kPrefetchMaxComp && lg > 0) prefetch_bra(args.pp, bp, lane);
     // this task's molecule block (bra and ket pairs always share a molecule)
     const int n = args.mol_n[bp.mol];
     const double* __restrict__ D = args.D + args.mol_base[bp.mol];
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
       if (active) {
         kpos = task.ket0 + (args.mx.pass ? nth_set_bit(sel, kk) : kk);
         kp = load_ket(args.kets, kpos, bp.mol, &ket);
+        if (C::NCOMP <= kPrefetchMaxComp && lg > 0) ket.prefetch(kp.np, sub, 1 << lg);
         // the reference skips when the Schwarz bound of its bra pair (the larger
         // composite index) is below threshold (gradient.rs:1457-1460)
         const double qref = bp.comp >= kp.comp ? bp.Q : kp.Q;

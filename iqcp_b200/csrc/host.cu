@@ -101,8 +101,8 @@ struct iqcp_ctx {
   // streams (forked and joined with events), so one class's tail overlaps
   // the next class's start
   static constexpr int kSide = kSetStreams - 1;
-  cudaStream_t side[kSide] = {nullptr, nullptr, nullptr};
-  cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {nullptr, nullptr, nullptr};
+  cudaStream_t side[kSide] = {};
+  cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {};
   // per-launch timing of the quartet kernels (off unless requested)
   bool profile = false;
   std::vector<cudaEvent_t> pev;

@@ -52,9 +52,20 @@ __host__ __device__ constexpr int rys_nint() { return rys_tasym(N) * rys_per_uni
 template <int N>
 __host__ __device__ constexpr int rys_tab_doubles() { return rys_nint<N>() * rys_tab_stride<N>(); }
 
-// Copy the order-N table into shared memory (all threads of the block).  Each
-// lane reads the interval of its own T, so table reads are scattered: from
-// shared memory they cost a few bank wavefronts, from L1 one cache line per lane.
+// Asynchronous copy of 16 bytes from global to shared memory.  A block's table of
+// 12 to 61 KB is 6 to 30 such copies per thread: issued back to back they cost one
+// trip to L2, as loads followed by stores one trip each, 5 to 10 us at the start of
+// a kernel that has little else to do in a small molecule.
+__device__ __forceinline__ void copy16_async(void* s, const void* g) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(g) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Copy the order-N table into shared memory (all threads of the block; a barrier
+// has to follow).  Each lane reads the interval of its own T, so table reads are
+// scattered: from shared memory they cost a few bank wavefronts, from L1 one
+// cache line per lane.
 template <int N>
 __device__ __forceinline__ void rys_stage_table(double* __restrict__ s) {
   constexpr int W = rys_tab_width<N>() / 2;
@@ -62,8 +73,9 @@ __device__ __forceinline__ void rys_stage_table(double* __restrict__ s) {
   double2* d = reinterpret_cast<double2*>(s);
   for (int i = threadIdx.x; i < rys_nint<N>() * W; i += blockDim.x) {
     const int k = i / W;
-    d[k * (rys_tab_stride<N>() / 2) + (i - k * W)] = __ldg(g + i);
+    copy16_async(d + k * (rys_tab_stride<N>() / 2) + (i - k * W), g + i);
   }
+  copy_async_wait();
 }
 
 // Polynomial of NC coefficients (16-byte aligned) at x in [-1, 1]; LDG: through
