@@ -233,9 +233,10 @@ struct GradMD {
   // resident blocks asked of the compiler: these kernels wait on their own FP64
   // chains, and warps pay more than the spills of up to 250 bytes that make room
   // for them: 40 atoms in 6-31G*, (ss|ss) 4 -> 5 blocks and (ps|ss), (pp|ss), (ds|ss) 3 -> 4:
-  // 1.20 -> 1.01, 2.61 -> 2.11, 0.95 -> 0.86, 0.97 -> 0.81 ms; (ps|ps) stays at 3
-  // (1.44 against 1.49 ms)
-  static constexpr int MINB = C::NCOMP > 60 ? 1 : (L == 0 ? 5 : (LC == 1 && L == 2 ? 3 : (L <= 2 ? 4 : 2)));
+  // 1.20 -> 1.01, 2.61 -> 2.11, 0.95 -> 0.86, 0.97 -> 0.81 ms; (dp|ss) 2 -> 3 1.24 -> 1.14.
+  // One more costs: (ps|ps) at 4 1.49 against 1.44, (pp|ps) at 3 1.87 against 1.66,
+  // (dp|ps) at 3 3.5 against 2.84
+  static constexpr int MINB = C::NCOMP > 60 ? 1 : (L == 0 ? 5 : (LC == 1 && L == 2 ? 3 : (L <= 2 ? 4 : (L == 3 && LC == 0 ? 3 : 2))));
   // shared memory (doubles) beside the gradient accumulator
   static constexpr int FIXED = TAB + WPB * WARP + THREADS * C::NCOMP;
 };

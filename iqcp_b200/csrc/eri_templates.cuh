@@ -362,13 +362,19 @@ __device__ __forceinline__ double group_sum(double v, int lg) {
 // take consecutive kets of the task, the lanes of a group split the quartet's
 // primitive quartets and add their partial blocks by shuffles, and the first
 // lane of each group digests the block.
-// Resident blocks asked of the compiler: up to L = 2 what the registers of a
-// spill-free build allow (left alone it takes 166 registers for (ps|ps), three
-// blocks, where 128 do without a spill).
-__host__ __device__ constexpr int jk_min_blocks(int L) { return L == 0 ? 6 : (L == 1 ? 5 : (L == 2 ? 4 : 1)); }
+// Resident blocks asked of the compiler, from sweeps at 40 atoms in 6-31G* and 30
+// in cc-pVDZ: these kernels wait for loads and FP64 chains, and up to L = 3 another
+// block of warps pays for a few hundred bytes of spill ((pp|ps) 2 -> 3 blocks 0.74 ->
+// 0.64 ms, (ds|ps) 0.88 -> 0.78, (dp|ss) 2 -> 4 0.47 -> 0.36; one more costs: (ps|ss) at 6
+// 1.26 against 1.15, (ps|ps) at 5 1.05 against 0.93, (pp|ps) at 4 0.71, (dp|ps) at 3 0.98
+// against 0.71).
+__host__ __device__ constexpr int jk_min_blocks(int L, int ncomp) {
+  return L == 0 ? 7 : (L == 1 ? 5 : (L == 2 ? 4 : (L == 3 ? (ncomp <= 18 ? 4 : 3) : 1)));
+}
 
 template <typename R, int LA, int LB, int LC, int LD, bool DO_K>
-__global__ void __launch_bounds__(128, jk_min_blocks(LA + LB + LC + LD)) jk_kernel(JKArgs args) {
+__global__ void __launch_bounds__(128, jk_min_blocks(LA + LB + LC + LD, Cls<LA, LB, LC, LD>::NCOMP))
+jk_kernel(JKArgs args) {
   using C = Cls<LA, LB, LC, LD>;
   extern __shared__ __align__(16) double rtab[];
   rys_stage_table<C::NR>(rtab);
