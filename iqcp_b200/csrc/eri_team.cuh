@@ -6,8 +6,8 @@
 //            the tables, the recurrence coefficients (rys_coefficients.rs:94),
 //            the 2D VRR (vrr_2d.rs:143) and the horizontal transfer to B and D
 //            (htr_4d.rs), written as one 1D table to shared memory;
-//   phase B  every lane accumulates its own components c = lane + 32 m of the
-//            block, sum over roots of Ix * Iy * Iz, from packed per-component
+//   phase B  a lane takes items (b, c, d) = lane + 32 m and accumulates their
+//            components, sum over roots of Ix * Iy * Iz, from packed per-item
 //            table offsets held in registers.
 // The contracted block is then staged in shared memory and digested into J/K
 // (8-fold symmetry, degeneracy factors) with one atomic per output element, or
@@ -38,7 +38,10 @@ struct TeamJK {
   static constexpr int DB = C::NA * C::NB + C::NC * C::ND + C::NB * C::ND + C::NA * C::ND + C::NB * C::NC +
                             C::NA * C::NC;
   static constexpr int PER_WARP = WORK + DB;
-  static constexpr int CPL = (C::NCOMP + 31) / 32;
+  // items (b, c, d) of phase B, rounds of 32 of them, and a lane's components: the
+  // NA components of A for each of its items
+  static constexpr int NIT = C::NB * C::NC * C::ND, ROUNDS = (NIT + 31) / 32, CPL = ROUNDS * C::NA;
+  static constexpr int SA = (LB + 1) * (LC + 1) * (LD + 1);  // table entries per power of A
   // resident 128-thread blocks asked of the compiler: 4 (128 registers, 16
   // warps per SM) where shared memory admits them and the tables are small
   // enough not to spill (<= 36 entries: ptxas 0-52 bytes); 1 otherwise (the
@@ -58,7 +61,8 @@ __device__ __forceinline__ void team_prim_loop(const PrimPair* __restrict__ pp, 
                                                const ShellPair& kp, const double* AB, const double* CD,
                                                const int* offs, double* acc, R* tab, int lane, const double* rtab) {
   using C = Cls<LA, LB, LC, LD>;
-  constexpr int NR = C::NR, TSZ = TeamJK<LA, LB, LC, LD>::TSP, CPL = TeamJK<LA, LB, LC, LD>::CPL;
+  using TM = TeamJK<LA, LB, LC, LD>;
+  constexpr int NR = C::NR, TSZ = TM::TSP;
   for (int i = 0; i < bp.np; ++i) {
     const PrimPair pb = load_pp(pp + bp.pstart + i);
     for (int j = 0; j < kp.np; ++j) {
@@ -84,39 +88,51 @@ __device__ __forceinline__ void team_prim_loop(const PrimPair* __restrict__ pp, 
             R(pick3(ax, AB[0], AB[1], AB[2])), R(pick3(ax, CD[0], CD[1], CD[2])), R(g00), tab + (r * 3 + ax) * TSZ);
       }
       __syncwarp();
+      // phase B: an item's row of each axis (the powers of A) is loaded once and
+      // serves the NA components of A, nine loads for six components of a d
+      // shell; loading three entries per component kept the load pipe at 81 %
 #pragma unroll
-      for (int m = 0; m < CPL; ++m) {
+      for (int m = 0; m < TM::ROUNDS; ++m) {
         const int o = offs[m];
-        const int ox = o & 0xff, oy = (o >> 8) & 0xff, oz = (o >> 16) & 0xff;
-        R sum = R(0);
+        const R* t = tab;
+        R sum[C::NA];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const R* t = tab + r * 3 * TSZ;
-          sum = fma(t[ox] * t[oy], t[oz], sum);
+        for (int a = 0; a < C::NA; ++a) sum[a] = R(0);
+#pragma unroll
+        for (int r = 0; r < NR; ++r, t += 3 * TSZ) {
+          R x[LA + 1], y[LA + 1], z[LA + 1];
+#pragma unroll
+          for (int p = 0; p <= LA; ++p) {
+            x[p] = t[(o & 0xff) + p * TM::SA];
+            y[p] = t[((o >> 8) & 0xff) + p * TM::SA];
+            z[p] = t[((o >> 16) & 0xff) + p * TM::SA];
+          }
+#pragma unroll
+          for (int a = 0; a < C::NA; ++a)
+            sum[a] = fma(x[cart_pow(LA, a, 0)] * y[cart_pow(LA, a, 1)], z[cart_pow(LA, a, 2)], sum[a]);
         }
-        acc[m] += double(sum);
+#pragma unroll
+        for (int a = 0; a < C::NA; ++a) acc[m * C::NA + a] += double(sum[a]);
       }
       __syncwarp();
     }
   }
 }
 
-// Packed table offsets of a lane's components (lane + 32 m): x | y << 8 | z << 16
+// Packed table offsets of a lane's items (lane + 32 m) at power 0 of A: x | y << 8 |
+// z << 16; items past the last one read item 0 and are not stored
 template <int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void team_offsets(int lane, int* offs) {
   using C = Cls<LA, LB, LC, LD>;
-  constexpr int TSZ = TeamJK<LA, LB, LC, LD>::TSP, CPL = TeamJK<LA, LB, LC, LD>::CPL;
+  using TM = TeamJK<LA, LB, LC, LD>;
 #pragma unroll
-  for (int m = 0; m < CPL; ++m) {
-    int comp = lane + 32 * m;
-    if (comp >= C::NCOMP) comp = 0;
-    const int d = comp % C::ND, c = (comp / C::ND) % C::NC, b = (comp / (C::ND * C::NC)) % C::NB,
-              a = comp / (C::ND * C::NC * C::NB);
+  for (int m = 0; m < TM::ROUNDS; ++m) {
+    const int it = lane + 32 * m < TM::NIT ? lane + 32 * m : 0;
+    const int d = it % C::ND, c = (it / C::ND) % C::NC, b = it / (C::ND * C::NC);
     int o = 0;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax)
-      o |= (ax * TSZ + C::tidx(cart_pow(LA, a, ax), cart_pow(LB, b, ax), cart_pow(LC, c, ax),
-                               cart_pow(LD, d, ax))) << (8 * ax);
+      o |= (ax * TM::TSP + C::tidx(0, cart_pow(LB, b, ax), cart_pow(LC, c, ax), cart_pow(LD, d, ax))) << (8 * ax);
     offs[m] = o;
   }
 }
@@ -140,7 +156,7 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
   double* Dbc = Dad + C::NA * C::ND;
   double* Dac = Dbc + C::NB * C::NC;
 
-  int offs[CPL];
+  int offs[TM::ROUNDS];
   team_offsets<LA, LB, LC, LD>(lane, offs);
 
   const int S = args.ket_split;  // work items per task (slices of its kets)
@@ -180,8 +196,8 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
     if (task.diag && kpos == task.bra_pos) f *= 0.5;
 #pragma unroll
     for (int m = 0; m < CPL; ++m) {
-      const int comp = lane + 32 * m;
-      if (comp < C::NCOMP) work[comp] = f * acc[m];
+      const int it = lane + 32 * (m / C::NA);
+      if (it < TM::NIT) work[(m % C::NA) * TM::NIT + it] = f * acc[m];
     }
     // every density of the call (nset > 1: response densities) is digested
     // with the same integrals
@@ -303,7 +319,7 @@ __global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const Pr
   } else {
     __shared__ double tabs[4][TM::TAB];
     const double AB[3] = {bp.A[0] - bp.B[0], bp.A[1] - bp.B[1], bp.A[2] - bp.B[2]};
-    int offs[TM::CPL];
+    int offs[TM::ROUNDS];
     team_offsets<LA, LB, LA, LB>(lane, offs);
     double acc[TM::CPL];
 #pragma unroll
@@ -311,8 +327,8 @@ __global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const Pr
     team_prim_loop<double, LA, LB, LA, LB, true>(pp, thr, bp, bp, AB, AB, offs, acc, tabs[threadIdx.x >> 5], lane, nullptr);
 #pragma unroll
     for (int m = 0; m < TM::CPL; ++m) {
-      const int i = lane + 32 * m;
-      if (i < C::NCOMP) {
+      const int it = lane + 32 * (m / C::NA), i = (m % C::NA) * TM::NIT + it;
+      if (it < TM::NIT) {
         const int d = i % C::ND, c = (i / C::ND) % C::NC, b = (i / (C::ND * C::NC)) % C::NB, a = i / (C::ND * C::NC * C::NB);
         mx = fmax(mx, fabs(acc[m] * ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LA, c) * ang_factor(LB, d)));
       }
