@@ -32,7 +32,12 @@ struct TeamJK {
   // (root, axis) tables TSP = TSZ | 1 entries apart, so that the lanes of
   // phase A, writing the same entry of consecutive tables, spread over the banks
   static constexpr int TSP = C::TSZ | 1;
-  static constexpr int TAB = C::NR * 3 * TSP;
+  // primitive quartets per pass of phase A, a lane per (primitive, root, axis):
+  // one left 9 lanes of 32 busy for (dp|pp), whose phase A is most of its time
+  // (1.14 -> 0.91 ms on 40 atoms in 6-31G*).  The second set of larger tables costs a
+  // resident block: (dp|dp) 0.56 -> 0.62 ms, (dd|pp) 0.20 -> 0.23 on 30 in cc-pVDZ.
+  static constexpr int JB = C::TSZ <= 27 ? 32 / (3 * C::NR) : 1;
+  static constexpr int TAB1 = C::NR * 3 * TSP, TAB = JB * TAB1;
   static constexpr int BLK = C::NCOMP;
   static constexpr int WORK = TAB > BLK ? TAB : BLK;
   static constexpr int DB = C::NA * C::NB + C::NC * C::ND + C::NB * C::ND + C::NA * C::ND + C::NB * C::NC +
@@ -51,69 +56,115 @@ struct TeamJK {
   static constexpr int MINB = C::TSZ <= 36 ? (SMEM_BLOCKS < 4 ? (SMEM_BLOCKS > 0 ? SMEM_BLOCKS : 1) : 4) : 1;
 };
 
+// Phase A for one primitive quartet: root r and axis ax of it into tab (TSP
+// entries).  LDG: the Rys table through L1 instead of staged at rtab.
+template <typename R, int LA, int LB, int LC, int LD, bool LDG>
+__device__ __forceinline__ void team_phase_a(const PrimPair& pb, const PrimPair& pk, const ShellPair& bp,
+                                             const ShellPair& kp, const double* AB, const double* CD, int r, int ax,
+                                             const double* rtab, R* tab) {
+  using C = Cls<LA, LB, LC, LD>;
+  const double p = pb.p, q = pk.p, s = p + q;
+  const double PQ[3] = {pb.P[0] - pk.P[0], pb.P[1] - pk.P[1], pb.P[2] - pk.P[2]};
+  const double rs = rsqrt(s), inv_s = rs * rs;  // 1/(p+q), 1/sqrt(p+q): one rsqrt
+  const double rho = p * q * inv_s;
+  const double T = rho * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+  double t2, wr;
+  rys_rule_one<C::NR, LDG>(T, r, rtab, &t2, &wr);
+  const double b00 = 0.5 * t2 * inv_s, h = 0.5 - 0.5 * t2;
+  const double b10 = fma(h, pb.inv_p, b00), b01 = fma(h, pk.inv_p, b00);
+  const double pa = pick3(ax, pb.P[0] - bp.A[0], pb.P[1] - bp.A[1], pb.P[2] - bp.A[2]);
+  const double qc = pick3(ax, pk.P[0] - kp.A[0], pk.P[1] - kp.A[1], pk.P[2] - kp.A[2]);
+  const double pq = pick3(ax, PQ[0], PQ[1], PQ[2]);
+  const double g00 = ax == 2 ? wr * kTwoPi52 * pb.cK * pk.cK * pb.inv_p * pk.inv_p * rs : 1.0;
+  axis_table<R, C::NBRA, C::NKET, LA, LB, LC, LD>(
+      R(pa - t2 * q * inv_s * pq), R(qc + t2 * p * inv_s * pq), R(b00), R(b10), R(b01),
+      R(pick3(ax, AB[0], AB[1], AB[2])), R(pick3(ax, CD[0], CD[1], CD[2])), R(g00), tab);
+}
+
+// Phase B for one primitive quartet.  An item's row of each axis (the powers of
+// A) is loaded once and serves the NA components of A, nine loads for six
+// components of a d shell; loading three entries per component kept the load
+// pipe at 81 % ((dp|dp) 0.73 -> 0.56 ms on 40 atoms in 6-31G*).
+template <typename R, int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void team_phase_b(const R* __restrict__ tab, const int* offs, double* acc) {
+  using C = Cls<LA, LB, LC, LD>;
+  using TM = TeamJK<LA, LB, LC, LD>;
+#pragma unroll
+  for (int m = 0; m < TM::ROUNDS; ++m) {
+    const int o = offs[m];
+    const R* t = tab;
+    R sum[C::NA];
+#pragma unroll
+    for (int a = 0; a < C::NA; ++a) sum[a] = R(0);
+#pragma unroll
+    for (int r = 0; r < C::NR; ++r, t += 3 * TM::TSP) {
+      R x[LA + 1], y[LA + 1], z[LA + 1];
+#pragma unroll
+      for (int p = 0; p <= LA; ++p) {
+        x[p] = t[(o & 0xff) + p * TM::SA];
+        y[p] = t[((o >> 8) & 0xff) + p * TM::SA];
+        z[p] = t[((o >> 16) & 0xff) + p * TM::SA];
+      }
+#pragma unroll
+      for (int a = 0; a < C::NA; ++a)
+        sum[a] = fma(x[cart_pow(LA, a, 0)] * y[cart_pow(LA, a, 1)], z[cart_pow(LA, a, 2)], sum[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < C::NA; ++a) acc[m * C::NA + a] += double(sum[a]);
+  }
+}
+
 // One contracted quartet: phases A and B over all surviving primitive
-// quartets, accumulating this lane's components into acc (FP64).  R is the
-// quadrature type: double, or float for the mixed form (roots, weights and
-// recurrence coefficients are formed in FP64 and rounded once).
-// LDG: the Rys table through L1 instead of staged at rtab.
-template <typename R, int LA, int LB, int LC, int LD, bool LDG = false>
+// quartets, JB per pass, accumulating this lane's components into acc (FP64).
+// R is the quadrature type: double, or float for the mixed form (roots, weights
+// and recurrence coefficients are formed in FP64 and rounded once).
+template <typename R, int LA, int LB, int LC, int LD, int JB = TeamJK<LA, LB, LC, LD>::JB, bool LDG = false>
 __device__ __forceinline__ void team_prim_loop(const PrimPair* __restrict__ pp, double prim_thr, const ShellPair& bp,
                                                const ShellPair& kp, const double* AB, const double* CD,
                                                const int* offs, double* acc, R* tab, int lane, const double* rtab) {
-  using C = Cls<LA, LB, LC, LD>;
   using TM = TeamJK<LA, LB, LC, LD>;
-  constexpr int NR = C::NR, TSZ = TM::TSP;
-  for (int i = 0; i < bp.np; ++i) {
-    const PrimPair pb = load_pp(pp + bp.pstart + i);
-    for (int j = 0; j < kp.np; ++j) {
-      const PrimPair pk = load_pp(pp + kp.pstart + j);
-      if (pb.K * pk.K < prim_thr) continue;
-      if (lane < 3 * NR) {
-        const int r = lane / 3, ax = lane - 3 * r;
-        const double p = pb.p, q = pk.p, s = p + q;
-        const double PQ[3] = {pb.P[0] - pk.P[0], pb.P[1] - pk.P[1], pb.P[2] - pk.P[2]};
-        const double rs = rsqrt(s), inv_s = rs * rs;  // 1/(p+q), 1/sqrt(p+q): one rsqrt
-        const double rho = p * q * inv_s;
-        const double T = rho * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-        double t2, wr;
-        rys_rule_one<NR, LDG>(T, r, rtab, &t2, &wr);
-        const double b00 = 0.5 * t2 * inv_s, h = 0.5 - 0.5 * t2;
-        const double b10 = fma(h, pb.inv_p, b00), b01 = fma(h, pk.inv_p, b00);
-        const double pa = pick3(ax, pb.P[0] - bp.A[0], pb.P[1] - bp.A[1], pb.P[2] - bp.A[2]);
-        const double qc = pick3(ax, pk.P[0] - kp.A[0], pk.P[1] - kp.A[1], pk.P[2] - kp.A[2]);
-        const double pq = pick3(ax, PQ[0], PQ[1], PQ[2]);
-        const double g00 = ax == 2 ? wr * kTwoPi52 * pb.cK * pk.cK * pb.inv_p * pk.inv_p * rs : 1.0;
-        axis_table<R, C::NBRA, C::NKET, LA, LB, LC, LD>(
-            R(pa - t2 * q * inv_s * pq), R(qc + t2 * p * inv_s * pq), R(b00), R(b10), R(b01),
-            R(pick3(ax, AB[0], AB[1], AB[2])), R(pick3(ax, CD[0], CD[1], CD[2])), R(g00), tab + (r * 3 + ax) * TSZ);
+  constexpr int NRAX = 3 * Cls<LA, LB, LC, LD>::NR;
+  if constexpr (JB == 1) {
+    for (int i = 0; i < bp.np; ++i) {
+      const PrimPair pb = load_pp(pp + bp.pstart + i);
+      for (int j = 0; j < kp.np; ++j) {
+        const PrimPair pk = load_pp(pp + kp.pstart + j);
+        if (pb.K * pk.K < prim_thr) continue;
+        if (lane < NRAX)
+          team_phase_a<R, LA, LB, LC, LD, LDG>(pb, pk, bp, kp, AB, CD, lane / 3, lane % 3, rtab, tab + lane * TM::TSP);
+        __syncwarp();
+        team_phase_b<R, LA, LB, LC, LD>(tab, offs, acc);
+        __syncwarp();
       }
-      __syncwarp();
-      // phase B: an item's row of each axis (the powers of A) is loaded once and
-      // serves the NA components of A, nine loads for six components of a d
-      // shell; loading three entries per component kept the load pipe at 81 %
-#pragma unroll
-      for (int m = 0; m < TM::ROUNDS; ++m) {
-        const int o = offs[m];
-        const R* t = tab;
-        R sum[C::NA];
-#pragma unroll
-        for (int a = 0; a < C::NA; ++a) sum[a] = R(0);
-#pragma unroll
-        for (int r = 0; r < NR; ++r, t += 3 * TSZ) {
-          R x[LA + 1], y[LA + 1], z[LA + 1];
-#pragma unroll
-          for (int p = 0; p <= LA; ++p) {
-            x[p] = t[(o & 0xff) + p * TM::SA];
-            y[p] = t[((o >> 8) & 0xff) + p * TM::SA];
-            z[p] = t[((o >> 16) & 0xff) + p * TM::SA];
-          }
-#pragma unroll
-          for (int a = 0; a < C::NA; ++a)
-            sum[a] = fma(x[cart_pow(LA, a, 0)] * y[cart_pow(LA, a, 1)], z[cart_pow(LA, a, 2)], sum[a]);
+    }
+  } else {
+    // slot: this lane's primitive quartet of a pass
+    const int slot = lane / NRAX, rax = lane - NRAX * slot;
+    int i = 0, j = -1;
+    for (bool more = bp.np > 0 && kp.np > 0; more;) {
+      // the next JB surviving primitive quartets (the same on every lane)
+      int cnt = 0, si = 0, sj = 0;
+      while (cnt < JB) {
+        if (++j == kp.np) {
+          j = 0;
+          ++i;
         }
-#pragma unroll
-        for (int a = 0; a < C::NA; ++a) acc[m * C::NA + a] += double(sum[a]);
+        if (i == bp.np) {
+          more = false;
+          break;
+        }
+        if (__ldg(&pp[bp.pstart + i].K) * __ldg(&pp[kp.pstart + j].K) < prim_thr) continue;
+        if (cnt == slot) {
+          si = i;
+          sj = j;
+        }
+        ++cnt;
       }
+      if (slot < cnt)
+        team_phase_a<R, LA, LB, LC, LD, LDG>(load_pp(pp + bp.pstart + si), load_pp(pp + kp.pstart + sj), bp, kp, AB, CD,
+                                             rax / 3, rax % 3, rtab, tab + lane * TM::TSP);
+      __syncwarp();
+      for (int g = 0; g < cnt; ++g) team_phase_b<R, LA, LB, LC, LD>(tab + g * TM::TAB1, offs, acc);
       __syncwarp();
     }
   }
@@ -317,14 +368,14 @@ __global__ void __launch_bounds__(128) schwarz_kernel(ShellPair* pairs, const Pr
       mx = fmax(mx, fabs(warp_sum(acc[i]) * ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LA, c) * ang_factor(LB, d)));
     }
   } else {
-    __shared__ double tabs[4][TM::TAB];
+    __shared__ double tabs[4][TM::TAB1];
     const double AB[3] = {bp.A[0] - bp.B[0], bp.A[1] - bp.B[1], bp.A[2] - bp.B[2]};
     int offs[TM::ROUNDS];
     team_offsets<LA, LB, LA, LB>(lane, offs);
     double acc[TM::CPL];
 #pragma unroll
     for (int m = 0; m < TM::CPL; ++m) acc[m] = 0.0;
-    team_prim_loop<double, LA, LB, LA, LB, true>(pp, thr, bp, bp, AB, AB, offs, acc, tabs[threadIdx.x >> 5], lane, nullptr);
+    team_prim_loop<double, LA, LB, LA, LB, 1, true>(pp, thr, bp, bp, AB, AB, offs, acc, tabs[threadIdx.x >> 5], lane, nullptr);
 #pragma unroll
     for (int m = 0; m < TM::CPL; ++m) {
       const int it = lane + 32 * (m / C::NA), i = (m % C::NA) * TM::NIT + it;
