@@ -666,37 +666,20 @@ __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_ke
       const bool kl_same = kp.sa == kp.sb;
       const bool bk_same = task.diag && kpos == task.bra_pos;
       R W[WSH ? 1 : C::NCOMP];
+      constexpr int NKC = C::NC * C::ND;
+      if constexpr (WSH) {
+        // not unrolled over the bra components: 108 copies of the weight were most
+        // of (dp|ds)'s code, and the kernel waited for instructions
+#pragma unroll 1
+        for (int ab = 0; ab < C::NA * C::NB; ++ab)
 #pragma unroll
-      for (int a = 0; a < C::NA; ++a)
+          for (int cd = 0; cd < NKC; ++cd)
+            Wsh[(ab * NKC + cd) * 128] = R(grad_weight<LA, LB, LC, LD>(D, n, bp, kp, ab * NKC + cd, ij_same, kl_same, bk_same, xs));
+      } else {
 #pragma unroll
-        for (int b = 0; b < C::NB; ++b)
-#pragma unroll
-          for (int c = 0; c < C::NC; ++c)
-#pragma unroll
-            for (int d = 0; d < C::ND; ++d) {
-              const int i = bp.oa + a, j = bp.ob + b, k = kp.oa + c, l = kp.ob + d;
-              const double dij = __ldg(D + i * n + j), dkl = __ldg(D + k * n + l);
-              const double dik = __ldg(D + i * n + k), djl = __ldg(D + j * n + l);
-              const double dil = __ldg(D + i * n + l), djk = __ldg(D + j * n + k);
-              // compute_symmetry_weight (gradient.rs:1570-1640) with D symmetric
-              double t = 0.5 * dij * dkl - xs * dik * djl;
-              if (!ij_same) t += 0.5 * dij * dkl - xs * djk * dil;
-              if (!kl_same) t += 0.5 * dij * dkl - xs * dil * djk;
-              if (!ij_same && !kl_same) t += 0.5 * dij * dkl - xs * djl * dik;
-              if (!bk_same) {
-                t += 0.5 * dkl * dij - xs * dik * djl;
-                if (!kl_same) t += 0.5 * dkl * dij - xs * dil * djk;
-                if (!ij_same) t += 0.5 * dkl * dij - xs * djk * dil;
-                if (!ij_same && !kl_same) t += 0.5 * dkl * dij - xs * djl * dik;
-              }
-              // D is angular-scaled: t = w_ref * (ang_a ang_b ang_c ang_d); the
-              // |w| < 1e-15 skip applies to the reference weight w_ref
-              const double angp = ang_factor(LA, a) * ang_factor(LB, b) * ang_factor(LC, c) * ang_factor(LD, d);
-              const R wt = R((fabs(t / angp) < 1e-15) ? 0.0 : t);
-              const int o = ((a * C::NB + b) * C::NC + c) * C::ND + d;
-              if constexpr (WSH) Wsh[o * 128] = wt;
-              else W[o] = wt;
-            }
+        for (int o = 0; o < C::NCOMP; ++o)
+          W[o] = R(grad_weight<LA, LB, LC, LD>(D, n, bp, kp, o, ij_same, kl_same, bk_same, xs));
+      }
       const double CD[3] = {kp.A[0] - kp.B[0], kp.A[1] - kp.B[1], kp.A[2] - kp.B[2]};
       PrimPair k;
       for (PrimItems it(bp.np, kp.np, sub, 1 << lg); it.more(); it.next()) {  // ket-major order (see quartet)
