@@ -549,6 +549,7 @@ grad_team2_kernel(GradArgs args) {
   R* Wsh = reinterpret_cast<R*>(wbase + TG::WOFF);   // weights of the current quartet
   double* rts_all = wbase + TG::ROFF;                // t^2 and weight of each (ket primitive, root)
 
+  const int slot = scatter_slot<9>(lane);
   const int S = args.ket_split;  // work items per task (slices of its kets)
   for (int item = next_task(args.next_task, lane); item < args.ntasks * S; item = next_task(args.next_task, lane)) {
   const int warp = item / S;     // the task
@@ -808,17 +809,13 @@ grad_team2_kernel(GradArgs args) {
         for (int x = 0; x < 9; ++x) g[x] += double(gl[x]);
       }
     }
-    // warp reduction of the nine derivatives, then atomics (D by invariance)
-#pragma unroll
-    for (int x = 0; x < 9; ++x) g[x] = warp_sum(g[x]);
-    if (lane == 0) {
-#pragma unroll
-      for (int ax = 0; ax < 3; ++ax) {
-        atomicAdd(gout + 3 * bp.atom_a + ax, g[ax]);
-        atomicAdd(gout + 3 * bp.atom_b + ax, g[3 + ax]);
-        atomicAdd(gout + 3 * kp.atom_a + ax, g[6 + ax]);
-        atomicAdd(gout + 3 * kp.atom_b + ax, -(g[ax] + g[3 + ax] + g[6 + ax]));
-      }
+    // warp sums of the nine derivatives, each on a lane of its own, then atomics;
+    // D's by invariance from the three of its axis
+    const double t = scatter_sum<9>(g, lane);
+    if (slot >= 0) {
+      const int x = slot % 3;
+      atomicAdd(gout + 3 * (slot < 3 ? bp.atom_a : (slot < 6 ? bp.atom_b : kp.atom_a)) + x, t);
+      atomicAdd(gout + 3 * kp.atom_b + x, -t);
     }
     __syncwarp();
   }

@@ -352,6 +352,47 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Sums over the warp of N values per lane, each left on one lane: the lanes halve the
+// values among themselves at each of the five exchanges, ceil(N/2) + ceil(N/4) + ...
+// of them instead of 5 N (12 for nine values, 45 by warp_sum), and one atomic
+// instruction adds them.  J/K at 40 atoms in 6-31G*: (dp|ps) 0.71 -> 0.61 ms,
+// (dd|ss) 0.13 -> 0.10, (dp|ss) 0.35 -> 0.33, all 10.13 -> 9.90; nine densities at
+// once on 16 atoms 1.23 -> 1.18.  scatter_slot gives the index of the value whose
+// sum a lane holds, or -1.
+template <int N, int O = 16>
+__device__ __forceinline__ double scatter_sum(double* v, int lane) {
+  if constexpr (O == 0) {
+    static_assert(N == 1, "at most 32 values");
+    return v[0];
+  } else if constexpr (N == 1) {
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+    return scatter_sum<1, O / 2>(v, lane);
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const bool up = lane & O;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      const double hi = i + H < N ? v[i + H < N ? i + H : i] : 0.0;
+      const double send = up ? v[i] : hi, keep = up ? hi : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+    }
+    return scatter_sum<H, O / 2>(v, lane);
+  }
+}
+template <int N, int O = 16>
+__device__ __forceinline__ int scatter_slot(int lane) {
+  if constexpr (O == 0) {
+    return 0;
+  } else if constexpr (N == 1) {
+    const int s = scatter_slot<1, O / 2>(lane);
+    return lane & O ? -1 : s;
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const int s = scatter_slot<H, O / 2>(lane), t = s + (lane & O ? H : 0);
+    return s < 0 || t >= N ? -1 : t;
+  }
+}
+
 // Sum over the 2^lg consecutive lanes of a group, on every lane of it.
 __device__ __forceinline__ double group_sum(double v, int lg) {
   for (int o = (1 << lg) >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -428,23 +469,29 @@ jk_kernel(JKArgs args) {
       const double* __restrict__ Dm = D + s * args.set_stride;
       double* Jm = args.J + mb + s * args.set_stride;
       double* Km = DO_K ? args.K + mb + s * args.set_stride : nullptr;
-      // J~_ab += 2f sum_cd (ab|cd) D_cd  -- same bra on every group: warp reduction
+      // J~_ab += 2f sum_cd (ab|cd) D_cd  -- same bra on every group: warp sums, up to
+      // nine components at a time
+      constexpr int NAB = C::NA * C::NB, NV = NAB <= 9 ? NAB : (NAB % 9 == 0 ? 9 : 6);
+      const int slot = scatter_slot<NV>(lane);
 #pragma unroll
-      for (int a = 0; a < C::NA; ++a)
+      for (int ab0 = 0; ab0 < NAB; ab0 += NV) {
+        double v[NV];
 #pragma unroll
-        for (int b = 0; b < C::NB; ++b) {
-          double v = 0.0;
+        for (int i = 0; i < NV; ++i) {
+          v[i] = 0.0;
           if (digest) {
 #pragma unroll
             for (int c = 0; c < C::NC; ++c)
 #pragma unroll
               for (int d = 0; d < C::ND; ++d)
-                v = fma(acc[((a * C::NB + b) * C::NC + c) * C::ND + d], __ldg(Dm + (kp.oa + c) * n + kp.ob + d), v);
-            v *= 2.0 * f;
+                v[i] = fma(acc[((ab0 + i) * C::NC + c) * C::ND + d], __ldg(Dm + (kp.oa + c) * n + kp.ob + d), v[i]);
+            v[i] *= 2.0 * f;
           }
-          v = warp_sum(v);
-          if (lane == 0) atomicAdd(Jm + (bp.oa + a) * n + bp.ob + b, v);
         }
+        const double t = scatter_sum<NV>(v, lane);
+        const int ab = ab0 + slot;
+        if (slot >= 0) atomicAdd(Jm + (bp.oa + ab / C::NB) * n + bp.ob + ab % C::NB, t);
+      }
       if (digest) {
       // J~_cd += 2f sum_ab (ab|cd) D_ab
       {
