@@ -93,16 +93,17 @@ inline int persistent_blocks(int per_sm, int sms, int ntasks, int threads) {
   } while (0)
 #define IQCP_LAUNCH(KERNEL, SMEM, ARGS, ST) IQCP_LAUNCH_T(KERNEL, 128, SMEM, ARGS, ST)
 
-// Team kernels walk a task's kets in one warp, one after the other.  A class
-// with fewer tasks than twice the resident warps ((dd|dd) on a 40-atom
-// molecule: ~700 tasks for ~1300 warps) would leave SMs idle and end on its
-// longest task, so its tasks are split into up to 32 slices of kets, each
-// a work item of its own; a (dd|dd) quartet alone is 30 us of one warp, so with
-// slices of four kets a 12-atom gradient waited 0.12 ms for 190 quartets.
+// Team kernels walk a task's kets in one warp, one after the other: 32 quartets of
+// (dp|dp) are 0.4 ms of one warp, and a launch ends on its longest work item.
+// Tasks are therefore split into up to 32 slices of kets, each a work item of its
+// own, until there are eight items per resident warp.  Against two, 40 atoms in
+// 6-31G*: J/K (dp|dp) 0.55 -> 0.48 ms, (dd|pp) 0.32 -> 0.25; gradient (dp|dp) 2.29 ->
+// 1.84, (dd|pp) 1.19 -> 0.88, (dp|pp) 3.35 -> 3.11, all 27.7 -> 27.2; 30 in cc-pVDZ,
+// gradient (dp|dp) 2.14 -> 1.23.  Sixteen: 27.2, J/K 9.78 -> 9.85.
 inline int team_ket_split(int per_sm, int sms, int ntasks, int threads) {
   const long long warps = (long long)per_sm * sms * (threads / 32);
   int s = 1;
-  while (s < 32 && (long long)ntasks * s < 2 * warps) s *= 2;
+  while (s < 32 && (long long)ntasks * s < 8 * warps) s *= 2;
   return s;
 }
 
