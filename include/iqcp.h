@@ -114,7 +114,10 @@ int iqcp_nbf(const iqcp_ctx* ctx);
  * and weights, recurrence coefficients and all accumulation stay FP64).  max|D|
  * is the largest density element over the six shell blocks the quartet
  * digests with; gradients use its square (D x D weights).  Applies to J/K,
- * Fock and ERI-gradient calls, single or batched contexts.
+ * Fock and ERI-gradient calls, single or batched contexts.  Classes whose FP32
+ * share costs as much as the whole class in FP64 (blocks of up to 108
+ * components, unless no class of the context is larger) run wholly in FP64 until
+ * iqcp_autotune or iqcp_set_kernel_mode says otherwise.
  */
 int iqcp_set_precision(iqcp_ctx* ctx, int precision, double mixed_cutoff);
 
@@ -123,7 +126,7 @@ int iqcp_set_precision(iqcp_ctx* ctx, int precision, double mixed_cutoff);
  * context's own stream, which is created non-blocking (it does not order with
  * the legacy default stream).  A caller working on the legacy default stream
  * passes cudaStreamLegacy, not NULL.  Inside a J/K build or gradient the
- * class kernels also run on three side streams of the context, forked from
+ * class kernels also run on eight side streams of the context, forked from
  * this stream by an event and joined back to it before the call's last
  * operation, so work queued on this stream before the call precedes all of
  * them and work queued after it follows all of them (in stream capture too).
@@ -341,7 +344,7 @@ int iqcp_measure_peak(int which, double* tflops);
 
 /*
  * Kernel-variant autotuner (no reference counterpart): for every (bra class,
- * ket class) time each quartet-kernel variant (0: one quartet per thread,
+ * ket class) time each quartet-kernel variant (0: a group of lanes per quartet,
  * 1: one warp per quartet with shared-memory 1D tables) on this device-resident
  * density, best of `reps`, and keep the fastest for J/K and for gradients.
  * With precision IQCP_MIXED the FP64 and FP32 shares of every class are tuned
@@ -351,7 +354,8 @@ int iqcp_measure_peak(int which, double* tflops);
  * modes[(kind*6 + X)*6 + Y], kind 0 J/K, 1 gradient, 2 / 3 their FP32 share
  * (-1: class has no quartets; 4 for kinds 2 / 3: the class runs wholly in FP64
  * in the mixed form); iqcp_set_kernel_mode forces one (kind 0..3, mode 0..3,
- * or 4 for kinds 2 / 3; X or Y = -1: all classes).
+ * or 4 for kinds 2 / 3; X or Y = -1: all classes).  Modes 2 and 3 run variant 0,
+ * and an FP64 class of more than 108 components always runs variant 1.
  */
 int iqcp_autotune(iqcp_ctx* ctx, const double* d_D, int reps);
 int iqcp_kernel_modes(const iqcp_ctx* ctx, int* modes);

@@ -55,6 +55,21 @@ __host__ __device__ constexpr int default_mode(int X, int Y, int kind, long long
   return n >= (kind == 1 ? 81 : 108) && quartets < 148LL * 8 * 32 ? 1 : 0;
 }
 
+// Whether a mixed call runs a class twice, FP64 share and FP32 share, before
+// autotuning; otherwise the whole class runs in FP64.  Roots, weights, pair data
+// and digestion are FP64 in both, so up to 108 components the FP32 share alone
+// takes what the class takes in FP64 and the other share comes on top: J/K of 40
+// atoms in 6-31G* at cutoff 1e-3 (96 % FP32), (ps|ss) 1.13 ms against 0.37 + 1.10,
+// (ds|ps) 0.79 / 0.14 + 0.73, (dd|ps) 0.36 / 0.13 + 0.60; gradient (dp|ps) 2.87 / 0.41 + 2.49,
+// (dp|ds) 1.62 / 0.34 + 3.28.  Above, the contraction is most of the work: gradient
+// (dp|pp) 3.02 / 0.50 + 1.93, (dd|dp) 1.02 / 0.28 + 0.69; J/K breaks even, (dp|pp) 0.83 /
+// 0.20 + 0.63.  The whole mixed Fock build 12.3 -> 9.8 ms.  A context without such
+// blocks splits its largest class alone (0.1 ms on (pp|pp)), so that no context's
+// mixed form is FP64 only.  largest: components of the context's largest class.
+__host__ __device__ constexpr int default_split(int X, int Y, int largest) {
+  return class_comps(X, Y) > kMaxThreadComp || class_comps(X, Y) == largest ? 1 : 0;
+}
+
 // Cartesian powers, reference order (integrals/cartesian.rs:113-136):
 // x exponent descending, then y exponent descending.
 __host__ __device__ constexpr int cart_pow(int l, int c, int axis) {

@@ -214,10 +214,12 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
   for (int item = next_task(args.next_task, lane); item < args.ntasks * S; item = next_task(args.next_task, lane)) {
   const int warp = item / S;     // the task
   const QuartetTask task = args.tasks[warp];
-  const ShellPair bp = args.pairs[task.bra];
-  if (task_inactive(args.mol_active, bp.mol)) continue;
   const int kper = (task.nket + S - 1) / S, k_lo = (item - warp * S) * kper;
   const int k_hi = task.nket < k_lo + kper ? task.nket : k_lo + kper;
+  const unsigned sel = task_sel(args.mx, warp, task.nket);
+  if (k_lo >= k_hi || ((sel >> k_lo) & ((2u << (k_hi - 1 - k_lo)) - 1u)) == 0) continue;  // no ket of this pass
+  const ShellPair bp = args.pairs[task.bra];
+  if (task_inactive(args.mol_active, bp.mol)) continue;
   // this task's molecule block (bra and ket pairs always share a molecule)
   const int n = args.mol_n[bp.mol];
   const long long mb = args.mol_base[bp.mol];
@@ -228,7 +230,6 @@ __global__ void __launch_bounds__(128, TeamJK<LA, LB, LC, LD>::MINB) jk_team_ker
     Dab[i] = __ldg(D + (bp.oa + i / C::NB) * n + bp.ob + i % C::NB);
 
   int nf32 = 0;
-  const unsigned sel = task_sel(args.mx, warp, task.nket);
   for (int kk = k_lo; kk < k_hi; ++kk) {
     if (!((sel >> kk) & 1u)) continue;  // another pass's ket (the same on every lane)
     const int kpos = task.ket0 + kk;
@@ -554,9 +555,11 @@ grad_team2_kernel(GradArgs args) {
   for (int item = next_task(args.next_task, lane); item < args.ntasks * S; item = next_task(args.next_task, lane)) {
   const int warp = item / S;     // the task
   const QuartetTask task = args.tasks[warp];
-  const ShellPair bp = args.pairs[task.bra];
   const int kper = (task.nket + S - 1) / S, k_lo = (item - warp * S) * kper;
   const int k_hi = task.nket < k_lo + kper ? task.nket : k_lo + kper;
+  const unsigned sel = task_sel(args.mx, warp, task.nket);
+  if (k_lo >= k_hi || ((sel >> k_lo) & ((2u << (k_hi - 1 - k_lo)) - 1u)) == 0) continue;  // no ket of this pass
+  const ShellPair bp = args.pairs[task.bra];
   // this task's molecule block (bra and ket pairs always share a molecule)
   const int n = args.mol_n[bp.mol];
   const long long mb = args.mol_base[bp.mol];
@@ -568,7 +571,6 @@ grad_team2_kernel(GradArgs args) {
   const bool ij_same = bp.sa == bp.sb;
   const double xs = args.xscale;
   int nsel = 0;
-  const unsigned sel = task_sel(args.mx, warp, task.nket);
 
   for (int kk = k_lo; kk < k_hi; ++kk) {
     if (!((sel >> kk) & 1u)) continue;  // another pass's ket (the same on every lane)

@@ -29,6 +29,7 @@ struct TaskRange {
   int mode[2];              // kernel variant for J/K [0] and gradient [1]
   int mode32[2];            // the same for the FP32 share of a mixed call
   int split[2];             // mixed form: 1 = FP64 + FP32 passes, 0 = the whole class in FP64
+  int chosen[2];            // split was set by iqcp_autotune or iqcp_set_kernel_mode
 };
 
 }  // namespace
@@ -306,14 +307,17 @@ int build_tasks(iqcp_ctx* ctx) {
   ctx->n_tasks = h_first[kNumRanges];
   ctx->ranges.clear();
   ctx->n_quartets = 0;
+  int largest = 0;
   for (int X = 0; X < NC; ++X)
     for (int Y = 0; Y <= X; ++Y) {
       const int k = range_of(X, Y);
-      TaskRange r{X, Y, h_first[k], h_first[k + 1] - h_first[k], (long long)work[2 * k + 1], {0, 0}, {0, 0}, {1, 1}};
+      TaskRange r{X, Y, h_first[k], h_first[k + 1] - h_first[k], (long long)work[2 * k + 1], {0, 0}, {0, 0}, {0, 0}, {0, 0}};
       for (int kind = 0; kind < 2; ++kind) r.mode[kind] = r.mode32[kind] = default_mode(X, Y, kind, r.quartets);
+      if (r.count > 0) largest = std::max(largest, class_comps(X, Y));
       ctx->n_quartets += r.quartets;
       ctx->ranges.push_back(r);
     }
+  for (TaskRange& r : ctx->ranges) r.split[0] = r.split[1] = default_split(r.X, r.Y, largest);
   ctx->block[2].want(&ctx->d_tasks, ctx->n_tasks);
   ctx->block[2].want(&ctx->d_mask, ctx->n_tasks);
   ctx->block[2].want(&ctx->d_counters, 4 * (ctx->ranges.size() + 1));
@@ -403,14 +407,22 @@ GradArgs grad_args(const iqcp_ctx* ctx, const TaskRange& r, const double* Ds, do
 }
 
 // Mixed form for density dD (unscaled): per-shell-block density bound, then
-// the FP32 mask of every task (kind 0 J/K, 1 gradient)
-int prepare_mixed(iqcp_ctx* ctx, const double* dD, int kind) {
+// the FP32 mask of every task (kind 0 J/K, 1 gradient) of the classes that run
+// an FP32 share (all: of every class)
+int prepare_mixed(iqcp_ctx* ctx, const double* dD, int kind, bool all = false) {
+  CK(cudaMemsetAsync(ctx->d_fp32, 0, sizeof(unsigned long long), ctx->stream));
+  bool any = all;
+  for (const TaskRange& r : ctx->ranges) any = any || (r.count > 0 && r.split[kind]);
+  if (!any) return IQCP_OK;
   CK(launch_shell_dmax(dD, ctx->pack, ctx->d_bint + 3 * ctx->n_shells, ctx->d_bint, mixed_args(ctx, 0),
                        ctx->dmax_total, ctx->d_dmax, ctx->stream));
-  CK(launch_precision_masks(ctx->d_pairs, ctx->d_ket_list, ctx->d_tasks, ctx->n_tasks, mixed_args(ctx, 1),
-                            kind == 1, ctx->d_mask, ctx->stream));
-  CK(cudaMemsetAsync(ctx->d_fp32, 0, sizeof(unsigned long long), ctx->stream));
-  ctx->launches_total += 2;
+  ctx->launches_total += 1;
+  for (const TaskRange& r : ctx->ranges) {
+    if (r.count == 0 || !(all || r.split[kind])) continue;
+    CK(launch_precision_masks(ctx->d_pairs, ctx->d_ket_list, ctx->d_tasks + r.first, r.count, mixed_args(ctx, 1),
+                              kind == 1, ctx->d_mask + r.first, ctx->stream));
+    ctx->launches_total += 1;
+  }
   return IQCP_OK;
 }
 
@@ -1452,7 +1464,7 @@ int iqcp_autotune(iqcp_ctx* ctx, const double* dD, int reps) {
   };
   for (int kind = 0; kind < 2; ++kind) {
     if (mixed) {
-      rc = prepare_mixed(ctx, dD, kind);
+      rc = prepare_mixed(ctx, dD, kind, true);
       if (rc) return rc;
     }
     for (TaskRange& r : ctx->ranges) {
@@ -1468,6 +1480,7 @@ int iqcp_autotune(iqcp_ctx* ctx, const double* dD, int reps) {
       if ((rc = tune(r, kind, 2, &m2, &t2))) return rc;
       r.mode32[kind] = m2;
       r.split[kind] = (t1 + t2 < t0) ? 1 : 0;
+      r.chosen[kind] = 1;
       if (r.split[kind]) r.mode[kind] = m1;
     }
   }
@@ -1480,11 +1493,12 @@ int iqcp_autotune(iqcp_ctx* ctx, const double* dD, int reps) {
 int iqcp_kernel_modes(const iqcp_ctx* ctx, int* modes) {
   if (!ctx || !modes) return IQCP_ERR_ARG;
   for (int i = 0; i < 4 * kNumPairClasses * kNumPairClasses; ++i) modes[i] = -1;
+  const bool mixed = ctx->opt.precision == IQCP_MIXED;  // in FP64 the default split is not in force
   for (const TaskRange& r : ctx->ranges)
     if (r.count > 0)
       for (int kind = 0; kind < 4; ++kind)
         modes[(kind * kNumPairClasses + r.X) * kNumPairClasses + r.Y] =
-            kind < 2 ? r.mode[kind] : (r.split[kind - 2] ? r.mode32[kind - 2] : kNumModes);
+            kind < 2 ? r.mode[kind] : (r.split[kind - 2] || !(mixed || r.chosen[kind - 2]) ? r.mode32[kind - 2] : kNumModes);
   return IQCP_OK;
 }
 
@@ -1495,11 +1509,10 @@ int iqcp_set_kernel_mode(iqcp_ctx* ctx, int kind, int X, int Y, int mode) {
     if (!((X < 0 || r.X == X) && (Y < 0 || r.Y == Y))) continue;
     if (kind < 2) {
       r.mode[kind] = mode;
-    } else if (mode == kNumModes) {
-      r.split[kind - 2] = 0;
     } else {
-      r.split[kind - 2] = 1;
-      r.mode32[kind - 2] = mode;
+      r.split[kind - 2] = mode < kNumModes;
+      r.chosen[kind - 2] = 1;
+      if (mode < kNumModes) r.mode32[kind - 2] = mode;
     }
   }
   return IQCP_OK;
