@@ -21,7 +21,7 @@
 // 1400 here).  What bounds it now is latency: 12 to 16 resident warps per SM
 // at 128 to 255 registers, FP64 pipe 35-45 %, issue slots 40 %.  40-atom 6-31G*,
 // Rys form -> here: (ps|ss) 3.29 -> 2.70 ms, (ps|ps) 2.69 -> 1.53, (pp|ps) 2.75 -> 1.71,
-// (ds|ps) 2.55 -> 1.72, (dp|ps) 3.41 -> 2.81, (dd|ps) 2.14 -> 1.56.
+// (ds|ps) 2.55 -> 1.72, (dp|ps) 3.41 -> 2.73, (dd|ps) 2.14 -> 1.54.
 //
 // The bra's expansion coefficients depend on the bra primitive only: the warp
 // stages them in shared memory per task, as products over the axes, and its
@@ -237,6 +237,11 @@ struct GradMD {
   // One more costs: (ps|ps) at 4 1.49 against 1.44, (pp|ps) at 3 1.87 against 1.66,
   // (dp|ps) at 3 3.5 against 2.84
   static constexpr int MINB = C::NCOMP > 60 ? 1 : (L == 0 ? 5 : (LC == 1 && L == 2 ? 3 : (L <= 2 ? 4 : (L == 3 && LC == 0 ? 3 : 2))));
+  // LOOPC: the ket components in a loop around branches for the part that differs.
+  // Unrolled three times, the 18 or 36 bra components' code outruns the instruction
+  // cache: (dp|ps) 2.85 -> 2.73 ms, (dd|ps) 1.67 -> 1.54 at 40 atoms in 6-31G*; smaller
+  // bras spill with the loop (300 to 600 bytes against 0 to 270).
+  static constexpr bool LOOPC = LC == 1 && C::NA * C::NB >= 18;
   // shared memory (doubles) beside the gradient accumulator
   static constexpr int FIXED = TAB + WPB * WARP + THREADS * C::NCOMP;
 };
@@ -354,20 +359,11 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
           const double oq = 0.5 * k.inv_p;
           // ket components: s, or p_x, p_y, p_z with E_0 = QC_c and E_{1c} = 1/2q
           // (odd Hermite orders of the ket change sign)
-          static_for<NC>([&](auto cc) {
+          double S[HLOW];  // R contracted with the ket component, |H| <= LA + LB - 1
+          // Lc[h]: the weighted bra expansion of ket component c
+          const auto ket_part = [&](auto cc, const double* Lc) {
             constexpr int c = cc.value;
             const double qc = LC == 0 ? 1.0 : k.P[LC == 0 ? 0 : c] - kp.A[LC == 0 ? 0 : c];
-            double g[NBRA], Lc[HB_];
-#pragma unroll
-            for (int ab = 0; ab < NBRA; ++ab) g[ab] = Wv[(ab * NC + c) * G::THREADS];
-#pragma unroll
-            for (int h = 0; h < HB_; ++h) Lc[h] = 0.0;
-            static_for<NBRA>([&](auto abc) {
-              constexpr int ab = abc.value, ca = ab / C::NB, cb = ab % C::NB;
-              const StagedPtr<HB::Main::TOTAL> Ec = E + ab * HB::Main::LEN;
-              for_coefficients<LA, LB, ca, cb>([&](auto o, auto h) { Lc[h.value] = fma(g[ab], Ec[o.value], Lc[h.value]); });
-            });
-            double S[HLOW];  // R contracted with the ket component, |H| <= LA + LB - 1
             static_for<HB_>([&](auto hc) {
               constexpr int h = hc.value;
               Lm[h] = fma(qc, Lc[h], Lm[h]);
@@ -380,6 +376,19 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
                 S[h] = R[h];
               }
             });
+          };
+          const auto component = [&](int c, auto&& ket) {
+            double g[NBRA], Lc[HB_];
+#pragma unroll
+            for (int ab = 0; ab < NBRA; ++ab) g[ab] = Wv[(ab * NC + c) * G::THREADS];
+#pragma unroll
+            for (int h = 0; h < HB_; ++h) Lc[h] = 0.0;
+            static_for<NBRA>([&](auto abc) {
+              constexpr int ab = abc.value, ca = ab / C::NB, cb = ab % C::NB;
+              const StagedPtr<HB::Main::TOTAL> Ec = E + ab * HB::Main::LEN;
+              for_coefficients<LA, LB, ca, cb>([&](auto o, auto h) { Lc[h.value] = fma(g[ab], Ec[o.value], Lc[h.value]); });
+            });
+            ket(Lc);
             if constexpr (LA > 0) {
               static_for<ncart(LA > 0 ? LA - 1 : 0) * C::NB>([&](auto lc) {
                 constexpr int LL = LA > 0 ? LA - 1 : 0, ca = lc.value / C::NB, cb = lc.value % C::NB;
@@ -404,7 +413,18 @@ __global__ void __launch_bounds__(GradMD<LA, LB, LC>::THREADS, GradMD<LA, LB, LC
                 gRb[2] = fma(double(l + 1) * g[ca * C::NB + cart_index(LB, i, j)], y, gRb[2]);
               });
             }
-          });
+          };
+          if constexpr (G::LOOPC) {
+#pragma unroll 1
+            for (int c = 0; c < NC; ++c)
+              component(c, [&](const double* Lc) {
+                if (c == 0) ket_part(std::integral_constant<int, 0>{}, Lc);
+                else if (c == 1) ket_part(std::integral_constant<int, 1>{}, Lc);
+                else ket_part(std::integral_constant<int, 2>{}, Lc);
+              });
+          } else {
+            static_for<NC>([&](auto cc) { component(cc.value, [&](const double* Lc) { ket_part(cc, Lc); }); });
+          }
           double e = 0.0, dP[3] = {0, 0, 0};
           static_for<HL>([&](auto hc) {
             constexpr int h = hc.value, t = hpow(h, 0), u = hpow(h, 1), v = hpow(h, 2);
