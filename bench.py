@@ -516,7 +516,7 @@ def main():
         step()
     # per-class launch times from a profiled pass before the timed region:
     # with profiling on, the library runs the class launches one after another
-    # (each timed alone), where the timed steps overlap them on four streams
+    # (each timed alone), where the timed steps overlap them on nine streams
     eng.set_profiling(True)
     per_kernel = {}
     for _ in range(max(1, min(args.steps, 3))):
@@ -625,10 +625,8 @@ def main():
         "parity_fp64": {"grad_2e_max_error_vs_oracle_ha_bohr": float(np.abs(g64 - fx["grad_2e"]).max()),
                         "scf_energy_error_vs_oracle_ha": abs(scf.energy - fx["energy"])},
         "kernel_modes": {"jk": modes[0].tolist(), "grad": modes[1].tolist(),
-                         "legend": "rows bra class, cols ket class (ss ps pp ds dp dd); J/K: 0 thread/quartet, "
-                                   "1 warp/quartet, 2 / 3 8 / 32 lanes per quartet; gradient: 0 thread/quartet, "
-                                   "1 warp/quartet, 2 thread/quartet with the D x D weights in shared memory, "
-                                   "3 32 lanes per quartet over (primitive quartet, root) items"},
+                         "legend": "rows bra class, cols ket class (ss ps pp ds dp dd); 0 a group of lanes per "
+                                   "quartet (gradients of ss and ps kets by Hermite expansions), 1 warp/quartet"},
     }
     jk_ms = kind_us[0] * 1e-3 / args.steps
     gr_ms = kind_us[1] * 1e-3 / args.steps

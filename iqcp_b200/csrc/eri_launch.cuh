@@ -1,6 +1,6 @@
 // Launchers for one bra class (LA, LB) against every ket class Y <= X.
 // Classes with many components use the warp-cooperative kernels
-// (eri_team.cuh); the small ones keep one quartet per thread.
+// (eri_team.cuh); the small ones take a group of lanes per quartet.
 #pragma once
 #include <atomic>
 
@@ -83,13 +83,44 @@ inline int persistent_blocks(int per_sm, int sms, int ntasks, int threads) {
   return need < cap ? need : cap;
 }
 
+// Launch with the shared memory of an SM cut to what the resident blocks use, which
+// leaves the rest to L1 for the pair, density and spill loads: the driver's own
+// choice leaves them less.  40 atoms in 6-31G*, J/K (dp|ds) 0.63 -> 0.57 ms, (dd|ps) 0.35 ->
+// 0.31, all 9.76 -> 9.41, gradient 26.8 -> 26.5; with all of it for the blocks J/K 10.38.
+// An SM changes its split only when idle, and short launches run beside each
+// other: those of fewer tasks per resident warp than kFullRounds keep the driver's
+// choice (12 atoms, J/K: 0.465 ms with 8, 0.473 with 2, 0.493 with none; 40 atoms 9.41, 9.34,
+// 9.34; with 32 9.74).  The warp-per-quartet kernels gain nothing.
+constexpr int kFullRounds = 8;
+
+template <typename A>
+cudaError_t launch_split(void (*kernel)(A), int blocks, int threads, size_t smem, int per_sm, bool full, const A& args,
+                         cudaStream_t st) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(blocks);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at = {};
+  if (full) {
+    const size_t need = per_sm * (smem + 1024), all = 228 * 1024;  // 1 KB reserved per block
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = need < all ? unsigned((need * 100 + all - 1) / all) : 100;
+    c.attrs = &at;
+    c.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&c, kernel, args);
+}
+
 #define IQCP_LAUNCH_T(KERNEL, THREADS, SMEM, ARGS, ST)                                           \
   do {                                                                                           \
     static LaunchCache cache_;                                                                   \
     int per_sm_ = 0, sms_ = 0;                                                                   \
     cudaError_t e_ = cache_.resident(KERNEL, SMEM, THREADS, &per_sm_, &sms_);                    \
     if (e_ != cudaSuccess) return e_;                                                            \
-    KERNEL<<<persistent_blocks(per_sm_, sms_, (ARGS).ntasks, THREADS), THREADS, SMEM, ST>>>(ARGS); \
+    e_ = launch_split(KERNEL, persistent_blocks(per_sm_, sms_, (ARGS).ntasks, THREADS), THREADS, SMEM, per_sm_, \
+                      (ARGS).ntasks >= kFullRounds * per_sm_ * sms_ * (THREADS / 32), ARGS, ST);              \
+    if (e_ != cudaSuccess) return e_;                                                            \
   } while (0)
 #define IQCP_LAUNCH(KERNEL, SMEM, ARGS, ST) IQCP_LAUNCH_T(KERNEL, 128, SMEM, ARGS, ST)
 

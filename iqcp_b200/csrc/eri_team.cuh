@@ -2,7 +2,8 @@
 //
 // One warp evaluates one contracted shell quartet at a time (the 32 kets of its
 // task one after another).  Per surviving primitive quartet:
-//   phase A  lanes 0 .. 3*NR-1 each take one (root, axis): the Rys root from
+//   phase A  lanes each take one (root, axis), 3*NR lanes per primitive quartet and
+//            several of them per pass where the tables are small: the root from
 //            the tables, the recurrence coefficients (rys_coefficients.rs:94),
 //            the 2D VRR (vrr_2d.rs:143) and the horizontal transfer to B and D
 //            (htr_4d.rs), written as one 1D table to shared memory;
