@@ -28,10 +28,10 @@ __host__ __device__ constexpr int class_lb(int c) { return c - class_la(c) * (cl
 
 // Largest block (components) of the FP64 thread kernels; above, only the
 // warp-cooperative ones exist.  Measured on 40 atoms in 6-31G*: at 108
-// components ((dp|ds), (dd|ps)) a lane group per quartet takes 0.67 and 0.41 ms
-// against a warp's 1.40 and 0.81 (J/K), 2.37 and 1.56 against 3.02 and 2.06
+// components ((dp|ds), (dd|ps)) a lane group per quartet takes 0.57 and 0.36 ms
+// against a warp's 1.06 and 0.53 (J/K), 1.62 and 1.55 against 2.69 and 1.61
 // (gradient); at 162 ((dp|pp)) the block no longer fits the registers and the
-// warp wins, 1.33 against 1.60 ms (J/K) and 3.33 against 8.2 (gradient).
+// warp wins, 0.86 against 1.60 ms (J/K) and 3.1 against 8.2 (gradient).
 constexpr int kMaxThreadComp = 108;
 constexpr int kMaxThreadComp32 = 324;      // the same for the FP32 share of a mixed call
 
@@ -46,9 +46,9 @@ __host__ __device__ constexpr int kernel_variant(int X, int Y, int mode, bool f3
 // Variant before autotuning.  With fewer quartets than one wave of thread-kernel
 // lanes (148 SMs x 8 warps at 255 registers) the largest blocks leave most of the
 // chip idle behind a few long threads, and a warp per quartet is faster: 12 atoms
-// in 6-31G*, gradient (pp|pp) 0.12 against 0.17 ms, (dp|ds) 0.14 / 0.23, (dd|ps) 0.11 /
-// 0.25, J/K (dd|ps) 0.05 / 0.07; below those sizes of block the thread kernels stay
-// ahead ((ds|pp) gradient 0.12 against 0.19 ms).
+// in 6-31G*, gradient (pp|pp) 0.12 against 0.15 ms, (dp|ds) 0.11 / 0.22, (dd|ps) 0.10 /
+// 0.24, J/K (dp|ds) 0.05 / 0.07, (dd|ps) 0.04 / 0.05; below those sizes of block the
+// thread kernels stay ahead ((ds|pp) J/K 0.06 against 0.04 ms, gradient 0.12 / 0.11).
 __host__ __device__ constexpr int default_mode(int X, int Y, int kind, long long quartets) {
   const int n = class_comps(X, Y);
   if (n > kMaxThreadComp) return 1;
