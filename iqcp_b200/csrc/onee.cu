@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "eri_templates.cuh"
+#include "smem_limit.cuh"
 
 namespace iqcp {
 
@@ -464,14 +465,10 @@ static cudaError_t one_e_blocks(const void* kernel, size_t smem, int units, int*
 
 cudaError_t launch_one_electron_grad(const OneEArgs& a, cudaStream_t st) {
   const size_t smem = a.gsmem ? sizeof(double) * 3 * (a.atom1 - a.atom0) : 0;
-  // beside the static arrays: dynamic shared memory beyond the default limit has to be asked for
-  if (smem > 32 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(one_electron_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = allow_dynamic_smem(one_electron_grad_kernel, smem);
+  if (e != cudaSuccess) return e;
   int blocks = 0;
-  const cudaError_t e = one_e_blocks((const void*)one_electron_grad_kernel, smem, 2 * a.first[kNumPairClasses], &blocks);
+  e = one_e_blocks((const void*)one_electron_grad_kernel, smem, 2 * a.first[kNumPairClasses], &blocks);
   if (e != cudaSuccess) return e;
   one_electron_grad_kernel<<<blocks, 32 * kWarps, smem, st>>>(a);
   return cudaGetLastError();

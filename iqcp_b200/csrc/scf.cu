@@ -38,6 +38,7 @@
 #include "../../include/iqcp.h"
 #include "device_pool.h"
 #include "internal.h"
+#include "smem_limit.cuh"
 
 namespace iqcp {
 namespace {
@@ -518,16 +519,17 @@ __global__ void purify_finish_kernel(const long long* __restrict__ base, const i
     P[o + e] = purify_element(c, in.P[o + e], in.P2[o + e], in.P3[o + e]);
 }
 
-template <int CT>
-cudaError_t launch_purify_step(size_t smem, dim3 grid, const long long* base, const int* nm, const int* active, int step,
-                               PurifyTriple in, PurifyTriple out, const double* prev, const double* prev2, double* part,
-                               cudaStream_t st) {
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(purify_step_kernel<CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+using PurifyStep = void (*)(const long long*, const int*, const int*, int, PurifyTriple, PurifyTriple, const double*,
+                            const double*, double*);
+// The step kernel for molecules of up to nmax functions: a lane takes every 32nd column
+inline PurifyStep purify_step_of(int nmax) {
+  switch ((nmax + 31) / 32) {
+    case 1: return purify_step_kernel<1>;
+    case 2: return purify_step_kernel<2>;
+    case 3: return purify_step_kernel<3>;
+    case 4: return purify_step_kernel<4>;
+    default: return purify_step_kernel<5>;
   }
-  purify_step_kernel<CT><<<grid, 128, smem, st>>>(base, nm, active, step, in, out, prev, prev2, part);
-  return cudaGetLastError();
 }
 
 // 3 I - X per molecule (grid: chunks x molecules)
@@ -628,19 +630,14 @@ struct ScfRun {
     const size_t share = 2 * (size_t)nmol * kStepMaxBlocks;
     const size_t smem = sizeof(double) * ((size_t)nmax * nmax + (size_t)kStepRows * nmax);
     const dim3 grid((nmax + kStepRows - 1) / kStepRows, nmol);
-    cudaError_t e = cudaSuccess;
+    const PurifyStep kernel = purify_step_of(nmax);
+    cudaError_t e = allow_dynamic_smem(kernel, smem);
     for (int s = 0; s < iters && e == cudaSuccess; ++s) {
       // step 0 updates nothing: it reads the start from t[0] as every even step
-      const PurifyTriple in = t[s & 1], out = t[(s + 1) & 1];
       double* now = part + (s % 3) * share;
       const double *p1 = part + ((s + 2) % 3) * share, *p2 = part + ((s + 1) % 3) * share;
-      switch ((nmax + 31) / 32) {
-        case 1: e = launch_purify_step<1>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
-        case 2: e = launch_purify_step<2>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
-        case 3: e = launch_purify_step<3>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
-        case 4: e = launch_purify_step<4>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
-        default: e = launch_purify_step<5>(smem, grid, base, nm, active, s, in, out, p1, p2, now, st); break;
-      }
+      kernel<<<grid, 128, smem, st>>>(base, nm, active, s, t[s & 1], t[(s + 1) & 1], p1, p2, now);
+      e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;
     purify_finish_kernel<<<elem_grid(), 256, 0, st>>>(base, nm, active, t[iters & 1], part + ((iters + 2) % 3) * share, P);
