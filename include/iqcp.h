@@ -89,6 +89,12 @@ int iqcp_basis_build(const char* basis_name, int n_atoms, const int* z, const do
  * (integrals/eri/mod.rs:992-1030, compute_schwarz_bounds :1263).
  */
 int iqcp_create(const iqcp_basis_desc* basis, const iqcp_options* opts, iqcp_ctx** out);
+
+/*
+ * Destroys a context once all work on its device is done, work that its calls
+ * only enqueued and running graphs that captured them included.  Other host
+ * threads may be capturing streams meanwhile; their captures go on.
+ */
 void iqcp_destroy(iqcp_ctx* ctx);
 
 /*

@@ -24,6 +24,22 @@ constexpr unsigned long long kPoolKeep = 64ull << 20, kPoolMax = 16ull << 20;
 cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t stream);
 void pool_free(void* p, cudaStream_t stream);
 
+// A small block from cudaMalloc, whose cudaFree waits for all work on the device
+// (drain).  A context's calls may have left work on any stream it was given, and
+// graphs that captured them may be running: its pooled memory and streams are
+// handed on only behind such a wait.  cudaDeviceSynchronize would end every
+// capture in progress on the device with an error, that of another thread's
+// batched SCF among them.
+cudaError_t drain_block(int device, void** p);
+cudaError_t drain(void* block);
+
+// Allocation calls of this thread are allowed beside captures while one of these lives
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Eight non-blocking streams (a small molecule's class kernels are a block or two
 // each, and their launches the longer the more of them run at once).  Returned sets are handed on to later contexts of
 // the same device, at most kKeepStreams idle sets per device.  A set is returned

@@ -42,6 +42,7 @@ struct iqcp_ctx {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   DeviceBlock block[3];            // tables and work buffers; ket tables; tasks
+  void* drain_block = nullptr;     // freed first, which waits for the device
   int nbf = 0, n_shells = 0, n_atoms = 0;   // totals over the molecules of the context
   // batched contexts: molecule m owns rows/cols [0, mol_nbf[m]) of the block at
   // mol_base[m] in every packed matrix (D, J, K, F, H, S) and atoms
@@ -613,6 +614,7 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->device));
   if (major != 10) return fail(ctx, IQCP_ERR_NODEVICE, "libiqcp_gpu is built for sm_100a only");
   CK(cudaSetDevice(ctx->device));
+  CK(drain_block(ctx->device, &ctx->drain_block));
   CK(streams_take(ctx->device, &ctx->streams));
   ctx->own_stream = ctx->streams.s[0];
   ctx->stream = ctx->own_stream;
@@ -832,10 +834,11 @@ int iqcp_batch_layout(const iqcp_ctx* ctx, long long* mat_offset, int* nbf, int*
 void iqcp_destroy(iqcp_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
-  // calls that only enqueue may have left work on any stream the context was
-  // given: the device is idle before memory and streams are handed on
-  cudaDeviceSynchronize();
-  for (DeviceBlock& b : ctx->block) b.free(ctx->own_stream);
+  RelaxedCapture relaxed;
+  // after a failed wait (the device is lost) pooled memory and streams are not handed on
+  const bool idle = drain(ctx->drain_block) == cudaSuccess;
+  if (idle)
+    for (DeviceBlock& b : ctx->block) b.free(ctx->own_stream);
   cudaFree(ctx->d_multi);
   cudaFree(ctx->d_multi_io);
   cudaFree(ctx->d_cart_info);
@@ -846,7 +849,8 @@ void iqcp_destroy(iqcp_ctx* ctx) {
   if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
   for (int s = 0; s < iqcp_ctx::kSide; ++s)
     if (ctx->join_ev[s]) cudaEventDestroy(ctx->join_ev[s]);
-  streams_give(ctx->device, ctx->streams);
+  if (idle) streams_give(ctx->device, ctx->streams);
+  else cudaGetLastError();
   delete ctx;
 }
 

@@ -925,11 +925,18 @@ done:
   ctx_set_mol_active(ctx, nullptr);
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
-  if (own) cudaStreamSynchronize(own);
   iqcp_set_stream(ctx, caller);
-  buf.free(own);
-  if (own) cudaStreamSynchronize(own);
-  streams_give(ctx_device(ctx), set);
+  if (own) {
+    // a call that failed midway may have left kernels on the context's side
+    // streams, which the wait for this stream does not cover
+    void* all = nullptr;
+    bool idle = cudaStreamSynchronize(own) == cudaSuccess;
+    if (rc) idle = idle && drain_block(ctx_device(ctx), &all) == cudaSuccess && drain(all) == cudaSuccess;
+    if (idle) {
+      buf.free(own);
+      if (cudaStreamSynchronize(own) == cudaSuccess) streams_give(ctx_device(ctx), set);
+    }
+  }
   return rc;
 }
 

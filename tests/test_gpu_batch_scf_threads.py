@@ -1,12 +1,15 @@
 """Batched SCFs and one-electron gradients of several host threads at once, one
 context per thread: molecules whose kernels need different amounts of shared
-memory must not change each other's launches."""
+memory must not change each other's launches, and contexts destroyed beside a
+running SCF must not end its captures, nor be handed on while their own work
+runs."""
 import threading
 
 import numpy as np
 import pytest
 
-from iqcp_b200 import BasisSet, BatchFockEngine
+from conftest import random_density
+from iqcp_b200 import BasisSet, BatchFockEngine, FockEngine
 from iqcp_b200.batch_scf import BatchRHF
 from iqcp_b200.molecules import REFERENCE_MOLECULES
 
@@ -77,3 +80,79 @@ def test_two_one_electron_gradients_of_many_atoms():
                     bad.append(n)
     _in_threads([lambda: run(700), lambda: run(1000)])
     assert not bad
+
+
+def test_contexts_destroyed_beside_a_batched_scf():
+    """A batched SCF captures an iteration; threads that make and destroy contexts
+    meanwhile leave the capture alone (errors of a capture ended by another
+    thread come back as a failed SCF)."""
+    b = BasisSet.build(REFERENCE_MOLECULES["NH3"], "6-31g*")
+    small = BasisSet.build(REFERENCE_MOLECULES["H2"], "sto-3g")
+    scf = BatchRHF([b])
+    e0 = scf.run().energies[0]
+    D = random_density(2, 1)
+    with FockEngine(small) as eng:
+        J0, K0 = eng.build_jk(D)
+    left = [12]
+    bad = []
+
+    def iterate():
+        try:
+            while left[0] > 0:
+                res = scf.run()
+                left[0] -= 1
+                if not res.converged.all() or abs(res.energies[0] - e0) > 1e-9:
+                    bad.append(res.energies[0])
+        finally:
+            left[0] = 0
+
+    def churn():
+        while left[0] > 0:
+            with FockEngine(small) as eng:
+                J, K = eng.build_jk(D)
+            if max(np.abs(J - J0).max(), np.abs(K - K0).max()) > 1e-12:
+                bad.append("J/K")
+    _in_threads([iterate, churn, churn])
+    scf.close()
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_destroy_waits_for_enqueued_work(captured):
+    """A context destroyed right after a call that only enqueues (or the replay of a
+    graph that captured one) on the caller's stream, and the next context in its
+    memory: the first call's results are those of a call waited for (1e-12)."""
+    import torch
+    b = BasisSet.build(REFERENCE_MOLECULES["CH4"], "6-31g*")
+    n = b.n_basis
+    D1, D2 = random_density(n, 1, 0.05), random_density(n, 2, 0.05)
+    with FockEngine(b) as eng:
+        ref = eng.build_jk(D1)
+    stream = torch.cuda.Stream()
+    d = torch.from_numpy(D1).cuda()
+    J, K = torch.zeros_like(d), torch.zeros_like(d)
+    for _ in range(4):
+        eng = FockEngine(b)
+        eng.set_stream(stream.cuda_stream)
+        eng.jk_device_noalloc(d.data_ptr(), J.data_ptr(), K.data_ptr())
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        if captured:
+            with torch.cuda.graph(graph, stream=stream):
+                eng.jk_device_noalloc(d.data_ptr(), J.data_ptr(), K.data_ptr())
+        J.zero_()
+        K.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)
+            if captured:
+                graph.replay()
+            else:
+                eng.jk_device_noalloc(d.data_ptr(), J.data_ptr(), K.data_ptr())
+        eng.close()
+        with FockEngine(b) as other:   # on streams and memory of the first
+            other.build_jk(D2)
+        torch.cuda.synchronize()
+        del graph
+        assert np.abs(J.cpu().numpy() - ref[0]).max() < 1e-12
+        assert np.abs(K.cpu().numpy() - ref[1]).max() < 1e-12
