@@ -21,6 +21,10 @@
  *    the last failure on a context is available from iqcp_last_error().
  *  - Calls on one context are synchronous with respect to the host and not
  *    thread-safe; use one context per host thread.
+ *  - The library keeps up to 64 MB of freed device memory and some idle streams
+ *    per device for its next contexts.  A cudaDeviceReset ends them with the
+ *    contexts of that time, which can then only be destroyed; new contexts
+ *    start afresh.
  */
 #ifndef IQCP_H_
 #define IQCP_H_

@@ -1,6 +1,9 @@
 // Library-wide device memory pool and stream sets (device_pool.h).
 #include "device_pool.h"
 
+#include <cuda.h>
+
+#include <atomic>
 #include <mutex>
 
 namespace iqcp {
@@ -13,6 +16,21 @@ std::vector<StreamSet> g_idle[kMaxDevices];
 // keeps the driver's segment for small blocks mapped: with nothing else from
 // cudaMalloc in the process a 256-byte block costs 608 us, beside one 5 us
 void* g_anchor[kMaxDevices] = {nullptr};
+unsigned long long g_id[kMaxDevices] = {0};  // CUDA context that the above belong to
+std::atomic<unsigned> g_epoch[kMaxDevices];
+
+using CtxGetId = CUresult (*)(CUcontext, unsigned long long*);
+CtxGetId ctx_get_id() {
+  static const CtxGetId fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<CtxGetId>(p);
+  }();
+  return fn;
+}
 
 cudaError_t pool_of(int device, cudaMemPool_t* out) {
   if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
@@ -41,6 +59,27 @@ cudaError_t pool_of(int device, cudaMemPool_t* out) {
 size_t round_up(size_t b) { return (b + 255) / 256 * 256; }
 
 }  // namespace
+
+cudaError_t device_refresh(int device, unsigned long long* id) {
+  *id = 0;
+  if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
+  cudaError_t e = cudaFree(nullptr);  // the primary context, made anew after a reset
+  if (e != cudaSuccess) return e;
+  const CtxGetId get = ctx_get_id();
+  if (!get) return cudaErrorNotSupported;
+  if (get(nullptr, id) != CUDA_SUCCESS) return cudaErrorDeviceUninitialized;
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (g_id[device] != *id) {
+    if (g_id[device]) g_epoch[device].fetch_add(1);
+    g_id[device] = *id;
+    g_pool[device] = nullptr;
+    g_idle[device].clear();
+    g_anchor[device] = nullptr;
+  }
+  return cudaSuccess;
+}
+
+unsigned device_epoch(int device) { return device >= 0 && device < kMaxDevices ? g_epoch[device].load() : 0; }
 
 cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t stream) {
   cudaMemPool_t pool = nullptr;

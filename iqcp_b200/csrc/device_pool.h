@@ -14,6 +14,14 @@
 
 namespace iqcp {
 
+// What the library keeps for the process (pool, idle streams, launch limits) ends
+// with the device's CUDA context: a caller may reset the device between two
+// contexts.  device_refresh, called where a context is made or destroyed with the
+// device current, asks for the CUDA context's id, which no later one shares; on a
+// new id it forgets what belonged to the old one and counts the epoch on.
+cudaError_t device_refresh(int device, unsigned long long* id);
+unsigned device_epoch(int device);
+
 // Memory from the library's pool on `device`, ordered on `stream`.  The pool is
 // the driver's stream-ordered allocator: safe from several threads and streams,
 // and it gives freed memory above kPoolKeep bytes back to the device whenever a

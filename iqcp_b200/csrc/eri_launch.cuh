@@ -4,6 +4,7 @@
 #pragma once
 #include <atomic>
 
+#include "device_pool.h"
 #include "eri_md.cuh"
 #include "eri_team.cuh"
 
@@ -39,10 +40,11 @@ inline size_t max_smem_optin() {
 // Resident blocks of one kernel at one block size and shared-memory size, per
 // device.  The occupancy query and the shared-memory attribute cost as much
 // host time as the launch itself, 21 times per call; a kernel's answer for the
-// size last asked about is kept (a race between threads only asks again).  The
-// attribute is set to the device's limit, the same from every thread.
+// size last asked about is kept (a race between threads only asks again) until
+// the device is reset.  The attribute is set to the device's limit, the same
+// from every thread.
 struct LaunchCache {
-  std::atomic<unsigned long long> slot[64];  // (smem + 1) << 16 | blocks per SM; 0: not asked yet
+  std::atomic<unsigned long long> slot[64];  // epoch << 40 | (smem + 1) << 16 | blocks per SM; 0: not asked yet
 
   template <typename K>
   cudaError_t resident(K kernel, size_t smem, int threads, int* per_sm, int* sms) {
@@ -51,7 +53,7 @@ struct LaunchCache {
     if (e != cudaSuccess) return e;
     const DeviceLimits lim = device_limits(dev);
     *sms = lim.sms;
-    const unsigned long long key = (unsigned long long)(smem + 1) << 16;
+    const unsigned long long key = (unsigned long long)device_epoch(dev) << 40 | (unsigned long long)(smem + 1) << 16;
     if (dev < 64) {
       const unsigned long long v = slot[dev].load(std::memory_order_relaxed);
       if ((v >> 16 << 16) == key) {

@@ -43,6 +43,7 @@ struct iqcp_ctx {
   cudaStream_t stream = nullptr;
   DeviceBlock block[3];            // tables and work buffers; ket tables; tasks
   void* drain_block = nullptr;     // freed first, which waits for the device
+  unsigned long long cuda_id = 0;  // CUDA context of all of these
   int nbf = 0, n_shells = 0, n_atoms = 0;   // totals over the molecules of the context
   // batched contexts: molecule m owns rows/cols [0, mol_nbf[m]) of the block at
   // mol_base[m] in every packed matrix (D, J, K, F, H, S) and atoms
@@ -614,6 +615,7 @@ static int create_batch(int nmol, const iqcp_basis_desc* descs, const iqcp_optio
   CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->device));
   if (major != 10) return fail(ctx, IQCP_ERR_NODEVICE, "libiqcp_gpu is built for sm_100a only");
   CK(cudaSetDevice(ctx->device));
+  CK(device_refresh(ctx->device, &ctx->cuda_id));
   CK(drain_block(ctx->device, &ctx->drain_block));
   CK(streams_take(ctx->device, &ctx->streams));
   ctx->own_stream = ctx->streams.s[0];
@@ -835,6 +837,11 @@ void iqcp_destroy(iqcp_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->device);
   RelaxedCapture relaxed;
+  unsigned long long id = 0;
+  if (device_refresh(ctx->device, &id) == cudaSuccess && id != ctx->cuda_id) {
+    delete ctx;  // its memory, streams and events went with a device reset
+    return;
+  }
   // after a failed wait (the device is lost) pooled memory and streams are not handed on
   const bool idle = drain(ctx->drain_block) == cudaSuccess;
   if (idle)
@@ -917,16 +924,19 @@ int iqcp_fock_device(iqcp_ctx* ctx, const double* dH, const double* dD, double k
 #define IQCP_NOALLOC_MAX_NBF 512
 static __device__ __align__(256) double g_noalloc_scratch[3 * IQCP_NOALLOC_MAX_NBF * IQCP_NOALLOC_MAX_NBF];
 static double* g_noalloc_ptr[64] = {nullptr};
+static unsigned g_noalloc_epoch[64] = {0};  // a device reset loads the array anew
 
 static int noalloc_scratch(iqcp_ctx* ctx, double** out) {
   if (ctx->device < 0 || ctx->device >= 64) return fail(ctx, IQCP_ERR_ARG, "device ordinal out of range");
-  if (!g_noalloc_ptr[ctx->device]) {
+  const unsigned epoch = device_epoch(ctx->device);
+  if (!g_noalloc_ptr[ctx->device] || g_noalloc_epoch[ctx->device] != epoch) {
     void* p = nullptr;
     const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess || !p)
       return fail(ctx, IQCP_ERR_CUDA, std::string("cudaGetSymbolAddress(g_noalloc_scratch): ") +
                                           cudaGetErrorString(e));
     g_noalloc_ptr[ctx->device] = static_cast<double*>(p);
+    g_noalloc_epoch[ctx->device] = epoch;
   }
   *out = g_noalloc_ptr[ctx->device];
   return IQCP_OK;
