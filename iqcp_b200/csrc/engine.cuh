@@ -117,6 +117,16 @@ struct KetTables {
   int n;               // positions
 };
 
+// Field f of a position among n, in geom
+__host__ __device__ constexpr unsigned long long ket_geom_offset(int f, int n) {
+  return (unsigned long long)(unsigned)f * (unsigned)n;
+}
+// Kets of one bucket, so that every offset within it is an int: the kernels' index
+// arithmetic (64-bit products cost the J/K builds of 40 atoms in 6-31G* 1 %).  A
+// longer run of kets with equal primitive counts becomes several buckets (0: not
+// even one ket fits, which context creation refuses).
+constexpr int max_bucket_kets(int np) { return int(0x7fffffffLL / (8LL * (np > 0 ? np : 1))); }
+
 // Unit of work for one warp: one bra pair against up to 32 consecutive ket
 // pairs of a class list.
 struct QuartetTask {

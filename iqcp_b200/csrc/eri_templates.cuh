@@ -185,6 +185,7 @@ __device__ __forceinline__ void prefetch_bra(const PrimPair* __restrict__ pp, co
 struct KetPrims {
   const double* p;
   int m;
+  // offsets within a bucket are ints (max_bucket_kets)
   __device__ __forceinline__ void prefetch(int np, int sub, int stride) const {
     for (int i = sub; i < 8 * np; i += stride) prefetch_l1(p + i * m);
   }
@@ -220,10 +221,10 @@ __device__ __forceinline__ ShellPair load_ket(const KetTables& t, int pos, int m
   k.pstart = 0;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    k.A[d] = __ldg(t.geom + d * t.n + pos);
-    k.B[d] = __ldg(t.geom + (3 + d) * t.n + pos);
+    k.A[d] = __ldg(t.geom + ket_geom_offset(d, t.n) + pos);
+    k.B[d] = __ldg(t.geom + ket_geom_offset(3 + d, t.n) + pos);
   }
-  k.Q = __ldg(t.geom + 6 * t.n + pos);
+  k.Q = __ldg(t.geom + ket_geom_offset(6, t.n) + pos);
   prims->p = t.prim + (unsigned)a.w;
   prims->m = b.w < 0 ? -b.w : b.w;
   return k;

@@ -231,7 +231,10 @@ int build_tasks(iqcp_ctx* ctx) {
     bucket0[s] = (int)bucket.size();
     for (int k0 = seg[s]; k0 < seg[s + 1];) {
       int k1 = k0;
-      while (k1 < seg[s + 1] && keys[k1].np == keys[k0].np) ++k1;
+      const int most = max_bucket_kets(keys[k0].np);
+      if (most < 1) return fail(ctx, IQCP_ERR_NOMEM, "more primitive pairs than the ket tables address");
+      const int end = (int)std::min<long long>(seg[s + 1], (long long)k0 + most);
+      while (k1 < end && keys[k1].np == keys[k0].np) ++k1;
       const int m = k1 - k0;
       bucket.push_back(make_int4(k0, m, keys[k0].np, 0));
       for (int k = k0; k < k1; ++k) {
