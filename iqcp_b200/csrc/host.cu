@@ -256,7 +256,7 @@ int build_tasks(iqcp_ctx* ctx) {
   t.thr = ctx->opt.schwarz_threshold;
   for (int X = 0; X < NC; ++X)
     for (int Y = 0; Y <= X; ++Y) t.entry0[range_of(X, Y) + 1] = t.entry0[range_of(X, Y)] + count[X];
-  const int entries = t.entry0[kNumRanges];
+  const long long entries = t.entry0[kNumRanges];
   // the ket tables stay; the lists only serve the construction
   int4 *i0 = nullptr, *i1 = nullptr;
   double *geom = nullptr, *prim = nullptr;
@@ -275,7 +275,8 @@ int build_tasks(iqcp_ctx* ctx) {
   } release{tmp, ctx->stream};
   int2* d_place = nullptr;
   int *d_pos_seg = nullptr, *d_seg = nullptr, *d_rank = nullptr, *d_bucket0 = nullptr, *offset = nullptr,
-      *part = nullptr, *first = nullptr;
+      *first = nullptr;
+  long long* part = nullptr;
   int4* d_bucket = nullptr;
   unsigned long long* sums = nullptr;
   tmp.upload(&d_place, place.data(), n);

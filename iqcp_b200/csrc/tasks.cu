@@ -39,7 +39,7 @@ __device__ __forceinline__ void for_buckets(const TaskLists& t, int b, F&& f) {
     }
 }
 
-__device__ __forceinline__ int entry_of(const TaskLists& t, int b, int X, int Y) {
+__device__ __forceinline__ long long entry_of(const TaskLists& t, int b, int X, int Y) {
   const int li = t.pos_seg[b];
   return t.entry0[range_of(X, Y)] + t.seg_rank[li] + b - t.seg[li];
 }
@@ -127,34 +127,37 @@ __global__ void __launch_bounds__(128) task_fill_kernel(TaskLists t, PerLane p, 
   });
 }
 
-// Exclusive sums of 1024-element chunks in place; part[chunk] = the chunk's total
-__global__ void __launch_bounds__(1024) scan_chunks_kernel(int n, int* v, int* part) {
-  __shared__ int sh[32];
-  const int i = blockIdx.x * 1024 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = i < n ? v[i] : 0;
-  int s = x;
+// Exclusive sums of 1024-element chunks in place; part[chunk] = the chunk's total,
+// in 64 bits: 1024 bras of a large molecule may have more than 2^31 tasks, and a
+// total that wraps would pass for a small one
+__global__ void __launch_bounds__(1024) scan_chunks_kernel(long long n, int* v, long long* part) {
+  __shared__ long long sh[32];
+  const long long i = blockIdx.x * 1024LL + threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long x = i < n ? v[i] : 0;
+  long long s = x;
   for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, s, o);
+    const long long u = __shfl_up_sync(0xffffffffu, s, o);
     if (lane >= o) s += u;
   }
   if (lane == 31) sh[w] = s;
   __syncthreads();
   if (w == 0) {
-    int u = sh[lane];
+    long long u = sh[lane];
     for (int o = 1; o < 32; o <<= 1) {
-      const int z = __shfl_up_sync(0xffffffffu, u, o);
+      const long long z = __shfl_up_sync(0xffffffffu, u, o);
       if (lane >= o) u += z;
     }
     sh[lane] = u;
   }
   __syncthreads();
   s += w > 0 ? sh[w - 1] : 0;
-  if (i < n) v[i] = s - x;
+  if (i < n) v[i] = int(s - x);
   if (threadIdx.x == 1023) part[blockIdx.x] = s;
 }
 
 // Exclusive sum of the chunk totals (one block; n chunks, total behind them; -1 if it passes 2^31 - 1)
-__global__ void __launch_bounds__(1024) scan_parts_kernel(int n, int* part) {
+__global__ void __launch_bounds__(1024) scan_parts_kernel(int n, long long* part) {
   __shared__ long long sh[32];
   __shared__ long long carry;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -180,18 +183,18 @@ __global__ void __launch_bounds__(1024) scan_parts_kernel(int n, int* part) {
     }
     __syncthreads();
     s += carry + (w > 0 ? sh[w - 1] : 0);
-    if (i < n) part[i] = (int)(s - x);
+    if (i < n) part[i] = s - x;
     __syncthreads();
     if (threadIdx.x == 1023) carry = s;
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[n] = carry > 0x7fffffffLL ? -1 : (int)carry;
+  if (threadIdx.x == 0) part[n] = carry > 0x7fffffffLL ? -1 : carry;
 }
 
-__global__ void __launch_bounds__(1024) scan_add_kernel(int n, int chunks, int* v, const int* part) {
-  const int i = blockIdx.x * 1024 + threadIdx.x;
-  if (i < n) v[i] += part[blockIdx.x];
-  if (i == 0) v[n] = part[chunks];
+__global__ void __launch_bounds__(1024) scan_add_kernel(long long n, int chunks, int* v, const long long* part) {
+  const long long i = blockIdx.x * 1024LL + threadIdx.x;
+  if (i < n) v[i] += int(part[blockIdx.x]);
+  if (i == 0) v[n] = int(part[chunks]);
 }
 
 __global__ void range_first_kernel(TaskLists t, const int* offset, int* first) {
@@ -207,9 +210,10 @@ cudaError_t launch_task_work(const TaskLists& t, unsigned long long* sums, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t launch_task_offsets(const TaskLists& t, const PerLane& p, int* offset, int* part, int* first,
+cudaError_t launch_task_offsets(const TaskLists& t, const PerLane& p, int* offset, long long* part, int* first,
                                 cudaStream_t st) {
-  const int n = t.entry0[kNumRanges], chunks = (n + 1023) / 1024;
+  const long long n = t.entry0[kNumRanges];
+  const int chunks = int((n + 1023) / 1024);
   if (n == 0) return cudaMemsetAsync(first, 0, sizeof(int) * (kNumRanges + 1), st);
   task_count_kernel<<<(t.n + 127) / 128, 128, 0, st>>>(t, p, offset);
   scan_chunks_kernel<<<chunks, 1024, 0, st>>>(n, offset, part);

@@ -23,17 +23,18 @@ struct TaskLists {
   const int4* i0;           // ket tables: .z = np
   const double* Q;          // Schwarz bound by position
   double thr;
-  int entry0[kNumRanges + 1];  // first entry of a range: an entry is (range, bra)
+  long long entry0[kNumRanges + 1];  // first entry of a range: an entry is (range, bra), up to six per position
 };
 
 // Primitive quartets and quartets of every range: sums[2 r], sums[2 r + 1]
 cudaError_t launch_task_work(const TaskLists& t, unsigned long long* sums, cudaStream_t st);
 // Tasks of every entry, then their exclusive sum in place (offset[entries] = total);
-// part: scratch of entries / 1024 + 2 ints.  first[r]: first task of range r, first[kNumRanges] the total.
+// part: scratch of entries / 1024 + 2 words.  first[r]: first task of range r, first[kNumRanges] the total,
+// or -1 where it does not fit an int.
 struct PerLane {
   double v[kNumRanges];  // primitive quartets a lane should serve
 };
-cudaError_t launch_task_offsets(const TaskLists& t, const PerLane& p, int* offset, int* part, int* first,
+cudaError_t launch_task_offsets(const TaskLists& t, const PerLane& p, int* offset, long long* part, int* first,
                                 cudaStream_t st);
 cudaError_t launch_task_fill(const TaskLists& t, const PerLane& p, const int* offset, QuartetTask* tasks,
                              cudaStream_t st);
