@@ -150,7 +150,6 @@ __device__ __forceinline__ void stage_products(int lane, const double* T, double
 // Boys function F_M .. F_0 at T: order M from the staged table below T = 36 and
 // the downward recurrence; above, F_0 = sqrt(pi / T) / 2 (erf(6) is 1 to rounding)
 // and the upward recurrence.
-template <int M>
 __host__ __device__ constexpr int boys_tab_doubles() { return BOYS_TAB_T * BOYS_TAB_PER_UNIT * (BOYS_TAB_NCOEF + 2); }
 
 template <int M>
@@ -225,7 +224,7 @@ template <int LA, int LB, int LC>
 struct GradMD {
   using C = Cls<LA, LB, LC, 0>;
   static constexpr int L = LA + LB + LC, LM = L + 1;
-  static constexpr int TAB = boys_tab_doubles<LM>();
+  static constexpr int TAB = boys_tab_doubles();
   static constexpr int WARP = HermiteBra<LA, LB>::WARP;
   // warps per block: four; six where the weights (110 KB for four warps of
   // (dd|ps)) leave no room for a second block

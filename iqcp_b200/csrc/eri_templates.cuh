@@ -472,7 +472,8 @@ jk_kernel(JKArgs args) {
       double* Km = DO_K ? args.K + mb + s * args.set_stride : nullptr;
       // J~_ab += 2f sum_cd (ab|cd) D_cd  -- same bra on every group: warp sums, up to
       // nine components at a time
-      constexpr int NAB = C::NA * C::NB, NV = NAB <= 9 ? NAB : (NAB % 9 == 0 ? 9 : 6);
+      constexpr int NAB = C::NA * C::NB, NV = NAB <= 9 ? NAB : 9;
+      static_assert(NAB % NV == 0, "blocks of 18 and 36 components");
       const int slot = scatter_slot<NV>(lane);
 #pragma unroll
       for (int ab0 = 0; ab0 < NAB; ab0 += NV) {
@@ -662,9 +663,10 @@ __host__ __device__ constexpr bool grad_stages_rys() {
   return !(WSH && ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) > 60);
 }
 
-// Resident blocks asked of the compiler: 4 for L <= 1 (for (ps|ss) the
-// 128-register cap spills 76 bytes per thread, and is still faster than 3
-// blocks without spill: 4.2 against 4.4 ms on the 40-atom step); 1 above.
+// Resident blocks asked of the compiler: 4 for L <= 1, which only the FP32 share
+// still takes (FP64 blocks with an ss or ps ket go by Hermite expansions), chosen
+// on (ps|ss) when FP64 took it too: 4.2 ms with a 76-byte spill against 4.4 with 3
+// blocks and none; 1 above.
 template <typename R, int LA, int LB, int LC, int LD, bool WSH = false>
 __global__ void __launch_bounds__(128, (LA + LB + LC + LD <= 1) ? 4 : 1) grad_kernel(GradArgs args) {
   using C = Cls<LA, LB, LC, LD>;

@@ -43,7 +43,7 @@ static const int kMaxN = 7;
 // 16-byte pairs) and intervals per unit of T
 static int deg_of(int n) { return n <= 2 ? 9 : 11; }
 static int per_unit(int n) { return n <= 2 ? 2 : 1; }
-static const int kMaxBoys = 9, kBoysT = 36, kBoysDeg = 9, kBoysPerUnit = 2;
+static const int kMaxBoys = 6, kBoysT = 36, kBoysDeg = 9, kBoysPerUnit = 2;
 
 // F_k(T) = int_0^1 t^{2k} e^{-T t^2} dt, k = 0..m, by the series of F_m and
 // downward recurrence (all terms positive, no cancellation).
@@ -237,9 +237,7 @@ int main(int argc, char** argv) {
   fprintf(f, "}\n#define RYS_TAB_PER_UNIT {0");
   for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", per_unit(n));
   fprintf(f, "}\n");
-  fprintf(f, "RYS_TAB_QUAL int kRysTasym[%d] = {0", kMaxN + 1);
-  for (int n = 1; n <= kMaxN; ++n) fprintf(f, ", %d", tasym[n]);
-  fprintf(f, "};\nRYS_TAB_QUAL int kRysOffset[%d] = {0", kMaxN + 2);
+  fprintf(f, "RYS_TAB_QUAL int kRysOffset[%d] = {0", kMaxN + 2);
   for (int n = 1; n <= kMaxN + 1; ++n) fprintf(f, ", %d", offset[n]);
   fprintf(f, "};\n// large-T rule per n (n entries each, n = 1..%d concatenated)\n", kMaxN);
   fprintf(f, "RYS_TAB_QUAL double kRysAsymRoot[%zu] = {\n", asy_y.size());
