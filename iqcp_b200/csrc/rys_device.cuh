@@ -106,14 +106,18 @@ __device__ __forceinline__ int rys_interval(double T, double* x) {
 // remainder one FMA forms exactly, leaves the rounding of the quotient (2^-53).
 // The bare product with 1/T = rsqrt(T)^2 left the roots of the large-T limit off by
 // up to 4.4e-16 instead of 2.9e-16; a division of each root costs the J/K builds 2 to
-// 4 % (40 atoms in 6-31G* 9.47 -> 9.75 ms).
+// 4 % (40 atoms in 6-31G* 9.47 -> 9.75 ms), the step 0.2 to 2.4 % (9.45 -> 9.47; 32 atoms
+// in 6-31G, s and p shells only, 2.40 -> 2.46).
 __device__ __forceinline__ double quotient(double c, double T, double it) {
   const double q = c * it;
   return fma(it, fma(-q, T, c), q);
 }
-// Arguments of the limit are cut here, where its roots no longer matter: an infinite
-// one would make the remainder 0 times infinity.
-constexpr double kRysHuge = 1e300;
+// Arguments of the limit (positive) are cut at 2^996, where its roots no longer
+// matter: an infinite one would make the remainder 0 times infinity.  One integer
+// minimum on the high word; fmin is six instructions.
+__device__ __forceinline__ double rys_cut(double T) {
+  return __hiloint2double(min(__double2hiint(T), 0x7e300000), __double2loint(T));
+}
 
 // The n-point rule at T.  s: the order-N table staged in shared memory, or
 // null to read it through L1.
@@ -122,7 +126,7 @@ __device__ __forceinline__ void rys_rule_tab(double T, const double* s, double* 
                                              double* __restrict__ w) {
   static_assert(N >= 1 && N <= RYS_TAB_MAXN, "unsupported Rys order");
   if (T >= double(rys_tasym(N))) {
-    const double Tc = fmin(T, kRysHuge), is = rsqrt(Tc), it = is * is;
+    const double Tc = rys_cut(T), is = rsqrt(Tc), it = is * is;
     const int base = (N * (N - 1)) / 2;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -151,7 +155,7 @@ __device__ __forceinline__ void rys_rule(double T, double* __restrict__ r, doubl
 template <int N, bool LDG = false>
 __device__ __forceinline__ void rys_rule_one(double T, int r, const double* s, double* t2, double* w) {
   if (T >= double(rys_tasym(N))) {
-    const double Tc = fmin(T, kRysHuge), is = rsqrt(Tc);
+    const double Tc = rys_cut(T), is = rsqrt(Tc);
     const int base = (N * (N - 1)) / 2;
     *t2 = quotient(__ldg(kRysAsymRoot + base + r), Tc, is * is);
     *w = __ldg(kRysAsymWeight + base + r) * is;

@@ -38,3 +38,10 @@ def test_roots_and_weights_of_the_limit(n):
             r, v = mp.mpf(c[base + k]) / t, mp.mpf(w[base + k]) / mp.sqrt(t)
             assert abs(mp.mpf(float(R[i, k])) - r) <= 1.001 * 2.0 ** -53 * r, (n, float(t), k)
             assert abs(mp.mpf(float(W[i, k])) - v) <= 3.001 * 2.0 ** -53 * v, (n, float(t), k)
+
+
+def test_largest_arguments_stay_finite():
+    import iqcp_b200 as iq
+    for n in sorted(TASYM):
+        R, W = iq.rys_roots(n, np.array([1e200, np.finfo(float).max]))
+        assert np.isfinite(R).all() and np.isfinite(W).all() and (R >= 0).all() and R.max() < 1e-197 and W.max() < 1e-99
