@@ -516,7 +516,7 @@ def main():
         step()
     # per-class launch times from a profiled pass before the timed region:
     # with profiling on, the library runs the class launches one after another
-    # (each timed alone), where the timed steps overlap them on nine streams
+    # (each timed alone), where the timed steps overlap them on eight streams
     eng.set_profiling(True)
     per_kernel = {}
     for _ in range(max(1, min(args.steps, 3))):

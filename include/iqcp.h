@@ -126,8 +126,9 @@ int iqcp_nbf(const iqcp_ctx* ctx);
  * digests with; gradients use its square (D x D weights).  Applies to J/K,
  * Fock and ERI-gradient calls, single or batched contexts.  Classes whose FP32
  * share costs as much as the whole class in FP64 (blocks of up to 108
- * components, unless no class of the context is larger) run wholly in FP64 until
- * iqcp_autotune or iqcp_set_kernel_mode says otherwise.
+ * components) run wholly in FP64 until iqcp_autotune or iqcp_set_kernel_mode says
+ * otherwise; where no class of the context has larger blocks, only the largest
+ * runs an FP32 share.
  */
 int iqcp_set_precision(iqcp_ctx* ctx, int precision, double mixed_cutoff);
 
@@ -136,7 +137,7 @@ int iqcp_set_precision(iqcp_ctx* ctx, int precision, double mixed_cutoff);
  * context's own stream, which is created non-blocking (it does not order with
  * the legacy default stream).  A caller working on the legacy default stream
  * passes cudaStreamLegacy, not NULL.  Inside a J/K build or gradient the
- * class kernels also run on eight side streams of the context, forked from
+ * class kernels also run on seven side streams of the context, forked from
  * this stream by an event and joined back to it before the call's last
  * operation, so work queued on this stream before the call precedes all of
  * them and work queued after it follows all of them (in stream capture too).

@@ -91,7 +91,7 @@ struct __align__(16) PrimPair {
   double inv_p;   // 1 / p
 };
 
-// One shell pair (la >= lb after the swap), 64 bytes.
+// One shell pair (la >= lb after the swap), 96 bytes.
 struct __align__(16) ShellPair {
   double A[3];
   double B[3];

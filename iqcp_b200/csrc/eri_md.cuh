@@ -18,10 +18,10 @@
 // the Rys form takes 2 n table functions, n x 3 extended 1D tables and 15 n
 // operations per component (about 2200 and 4100 FP64 instructions per primitive
 // quartet of (pp|ps) and (dp|ps), from the FP64 pipe's activity, against 700 and
-// 1400 here).  What bounds it now is latency: 12 to 16 resident warps per SM
-// at 128 to 255 registers, FP64 pipe 35-45 %, issue slots 40 %.  40-atom 6-31G*,
-// Rys form -> here: (ps|ss) 3.29 -> 2.70 ms, (ps|ps) 2.69 -> 1.53, (pp|ps) 2.75 -> 1.71,
-// (ds|ps) 2.55 -> 1.72, (dp|ps) 3.41 -> 2.73, (dd|ps) 2.14 -> 1.54.
+// 1400 here).  What bounds it now is latency: 6 to 20 resident warps per SM
+// at 96 to 255 registers, FP64 pipe 14-48 %.  40-atom 6-31G*,
+// Rys form -> here: (ps|ss) 3.29 -> 2.11 ms, (ps|ps) 2.69 -> 1.45, (pp|ps) 2.75 -> 1.66,
+// (ds|ps) 2.55 -> 1.68, (dp|ps) 3.41 -> 2.73, (dd|ps) 2.14 -> 1.54.
 //
 // The bra's expansion coefficients depend on the bra primitive only: the warp
 // stages them in shared memory per task, as products over the axes, and its
